@@ -246,7 +246,6 @@ struct sdot_ctx {
     bool has_image = false;
     double img_lo[3] = {0, 0, 0}, img_hi[3] = {1, 1, 1};
     long long img_size[3] = {1, 1, 1};
-    char *img_backup3 = nullptr;  // 3D voxel images: the kernels' per-warp face copies
     int img_ncoeffs = 1;
     std::vector<double> img_data;
     int ball = 0;
@@ -282,10 +281,8 @@ struct sdot_ctx {
     DevStatus *dstat = nullptr, *hstat = nullptr;
     int *ovf_list = nullptr, *ovf_cnt = nullptr;
     int *ovf_list2 = nullptr, *ovf_cnt2 = nullptr;  // 3D: third pass
-    int *ovf_list3 = nullptr, *ovf_cnt3 = nullptr;  // 3D: fourth pass
     unsigned char *hint3 = nullptr;                  // 3D: pass of each cell last time
     bool hint_valid = false;
-    void *scratch3 = nullptr;                        // 3D: third pass faces
     unsigned *err = nullptr;   // &dstat->err
     int *guard = nullptr;      // dstat->guard
     long long item_nv = 0;
@@ -316,7 +313,6 @@ struct sdot_ctx {
         dfree(d_start); dfree(d_img); dfree(d_item_xy); dfree(d_item_nrm); dfree(d_item_coeff); dfree(d_item_off);
         dfree(d_trans);
         dfree(d_planes3);
-        dfree(img_backup3);
         free_eval();
         free_newton();
         free_multi();
@@ -330,7 +326,7 @@ struct sdot_ctx {
         free_rows(rows);
         free_rows(nb);
         dfree(cnt_orig); dfree(offsets); dfree(nb_offsets);
-        dfree(ovf_list); dfree(ovf_list2); dfree(ovf_cnt2); dfree(ovf_list3); dfree(ovf_cnt3); dfree(hint3);
+        dfree(ovf_list); dfree(ovf_list2); dfree(ovf_cnt2); dfree(hint3);
         dfree(dstat);
         dfree(ras_buf);
         dfree(ras_nums);
@@ -342,8 +338,6 @@ struct sdot_ctx {
         stage_cap = 0;
         dfree(dp_off); dfree(dp_col); dfree(dp_val); dfree(dp_v);
         dp_ncap = dp_nnzcap = 0;
-        if (scratch3) cudaFree(scratch3);
-        scratch3 = nullptr;
         if (scratch) cudaFree(scratch);
         if (scan_tmp) cudaFree(scan_tmp);
         scratch = scan_tmp = nullptr;
@@ -390,11 +384,8 @@ struct sdot_ctx {
         if (dim == 3) {
             dalloc(ovf_list2, ecap);
             dalloc(ovf_cnt2, 1);
-            dalloc(ovf_list3, ecap);
-            dalloc(ovf_cnt3, 1);
             dalloc(hint3, ecap);
             hint_valid = false;
-            SDOT_CUDA(cudaMalloc(&scratch3, cells3d_scratch_bytes()));
         }
         SDOT_CUDA(cudaMalloc(&scratch, cells2d_scratch_bytes()));
         SDOT_CUDA(cudaMalloc(&scan_tmp, scan_tmp_size(ecap + 1, sizeof(long long))));
@@ -504,7 +495,6 @@ struct sdot_ctx {
             if (dom_dirty) {
                 dalloc(d_img, img_data.size());
                 SDOT_CUDA(cudaMemcpy(d_img, img_data.data(), img_data.size() * sizeof(double), cudaMemcpyHostToDevice));
-                if (!img_backup3) dalloc(img_backup3, cells3d_image_backup_bytes());
                 dom_dirty = false;
             }
             return;
@@ -598,7 +588,7 @@ struct sdot_ctx {
             a.mass = t_mass;
             a.ctd = t_ctd;
             a.rows = rows_tmp;
-            cells3d_launch(a, scratch3, stream);
+            cells3d_launch(a, stream);
             accum_pass(s_mass, s_mass_c, s_mom, t_mass, t_mass, t_ctd, n, 3, stream);
             rows_append(rows, rows_tmp, n, err, stream);
         }
@@ -624,7 +614,6 @@ struct sdot_ctx {
                 a.img_n[d] = int(img_size[d]);
             }
             a.img = d_img;
-            a.img_backup = img_backup3;
         } else if (k >= 0) {
             for (int d = 0; d < 3; ++d) {
                 a.box_lo[d] = items3[k].lo[d];
@@ -651,8 +640,6 @@ struct sdot_ctx {
         a.ovf_cnt = ovf_cnt;
         a.ovf_list2 = ovf_list2;
         a.ovf_cnt2 = ovf_cnt2;
-        a.ovf_list3 = ovf_list3;
-        a.ovf_cnt3 = ovf_cnt3;
         a.hint = hint3;
         a.use_hint = hint_valid ? 1 : 0;
         a.err = err;
@@ -697,7 +684,7 @@ struct sdot_ctx {
             a.mass = s_mass;
             a.ctd = s_ctd;
             a.rows = rows;
-            cells3d_launch(a, scratch3, stream);
+            cells3d_launch(a, stream);
             hint_valid = true;  // every cell of this tree order now has a pass hint
             // get_centroids' mass is the integral itself in 3D
             SDOT_CUDA(cudaMemcpyAsync(s_mass_c, s_mass, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, stream));
@@ -801,7 +788,7 @@ struct sdot_ctx {
                     a.use_hint = 0;
                 }
                 a.nb = nb;
-                cells3d_launch(a, scratch3, stream);
+                cells3d_launch(a, stream);
             } else {
                 // several shapes: the cut ids of the traversal cell in the
                 // englobing box (the cell the reference's callback receives)

@@ -1,16 +1,23 @@
 // 3D Laguerre-cell kernels (see cell3d.cuh).
 //
-// One warp builds one cell.  The cell is a convex polyhedron held as its
-// faces, one face per lane (2, 4 or 8 in the larger passes): each face is a polygon
-// (vertices counter-clockwise seen from outside, in coordinates relative to
-// the cell's Dirac) whose edge k carries the id of the face across it, plus
-// the face's plane a . u <= b and its cut id (a Dirac index, or a domain
-// face).  A plane cut is then a 2D polygon cut done by every lane on its own
-// face at once, followed by the new face, whose vertices are the points where
-// the cut faces enter the cut: starting from one cut face, the next is the
-// face across its exit edge.  The point where an edge is cut is computed from
-// the edge's inside vertex in both faces that share the edge, so the copies
-// agree bitwise and the new face closes exactly.
+// One warp builds one cell.  The cell is a simple convex polyhedron held by
+// its vertices (every vertex on exactly three faces; a point where more faces
+// meet is several vertices at one place), one vertex per lane and block of 32,
+// in shared memory and in coordinates relative to the cell's Dirac.  A vertex
+// keeps its three faces, counter-clockwise seen from outside, and opposite to
+// each of them the vertex at the other end of its third edge.  Most of the
+// walk asks on which side of a plane, or how near a box, the vertices lie:
+// that is one evaluation per vertex, about 27 of them in 32 lanes, and a
+// ballot.  (Held by its faces, each vertex was stored and tested three times
+// in loops over the faces' polygons, 11.9 of 32 lanes active.)
+//
+// A plane cut marks the vertices outside; every edge from one of them to a
+// vertex that stays gives a new vertex on the cut, found from its inside and
+// outside ends, with the two faces of that edge and the cut as its faces.  Each
+// face that is cut through has one new vertex where the cut enters it and one
+// where it leaves: two tables over the faces link the new vertices.
+// Faces live in numbered slots, a new face in the lowest one free, and the
+// neighbour lists come out in slot order.
 //
 // Reference behaviour restated (ConvexPolyhedron3 and the 3D traversal):
 //  * traversal and eviction test: SpZGrid::for_each_laguerre_cell, as in 2D
@@ -41,232 +48,260 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int STACK3 = 96;  // depth <= 10 levels (10 key bits per axis), <= 7 pending siblings each
+constexpr int MAX_NEW = 128;  // vertices of a new face
 
-// Faces of one warp: vertex v of face slot f at [v * MAXF + f].
-template <int FPL, int MAXV>
-struct Faces {
-    static constexpr int MAXF = 32 * FPL;
-    double *X, *Y, *Z;
-    int *E;
-    __device__ int at(int v, int f) const { return v * MAXF + f; }
+// One warp's cell in shared memory: up to 32 VB vertices and MAXP faces.
+template <int VB, int MAXP>
+struct Cell3 {
+    static constexpr int MAXV = 32 * VB, PW = MAXP / 32;
+    static_assert(MAXV <= 1024 && PW <= 32, "vertex numbers of 10 bits, one word of the face mask per lane");
+    double x[MAXV], y[MAXV], z[MAXV];
+    double plane[MAXP][4];               // face: plane a . u <= b (a, b)
+    int pid[MAXP];                       // face: its cut id
+    unsigned alive[VB];                  // bit v & 31 of word v >> 5: vertex v is in use
+    unsigned live[PW];                   // the same for the faces
+    unsigned short fp[3][MAXV];          // vertex: its faces, counter-clockwise
+    unsigned short nb[3][MAXV];          // vertex: the neighbour opposite to each face
+};
+// What a cut and the walk need beside the cell (not part of its copies).
+template <int VB, int MAXP>
+struct Work3 {
+    unsigned out[VB];                    // the vertices outside a cut
+    unsigned rm[MAXP / 32], hm[MAXP / 32];  // faces of the removed vertices, faces that are cut through
+    int first[MAXP];                     // lowest vertex of each face
+    unsigned short ta[MAXP], tb[MAXP];   // new vertex with this face second, third
+    unsigned short req[MAXP];            // edges to cut: vertex outside | edge << 10
+    unsigned short list[MAXP];           // faces in slot order
+    int stack[STACK3];
 };
 
-template <int FPL, int MAXV>
-constexpr size_t warp_smem_bytes() {
-    return size_t(MAXV) * (32 * FPL) * (3 * sizeof(double) + sizeof(int)) + STACK3 * sizeof(int);
+__device__ inline int next3(int i) { return i == 2 ? 0 : i + 1; }
+
+// Loops over the blocks of vertices are unrolled where a cell has two.
+template <int VB, class F>
+__device__ __forceinline__ void each_block(int nr, F &&f) {
+    if constexpr (VB <= 2) {
+#pragma unroll
+        for (int r = 0; r < VB; ++r)
+            if (r < nr) f(r);
+    } else {
+        for (int r = 0; r < nr; ++r) f(r);
+    }
 }
 
-// One cell's state in a warp: the faces (shared memory) and, per lane and
-// face slot r (face lane + 32 r), the face's plane, id and vertex count.
-template <int FPL, int MAXV>
-struct Cell3 {
-    Faces<FPL, MAXV> F;
-    int *stack;
-    int fid[FPL], nv[FPL];
-    double ax[FPL], ay[FPL], az[FPL], b[FPL];
-};
-
-__device__ inline double shfl(double v, int src) { return __shfl_sync(FULL, v, src); }
-
-// Outcome of a cut: 0 done, 1 a capacity was exceeded, 2 degenerate geometry.
-template <int FPL, int MAXV>
-__device__ __forceinline__ int cut3(Cell3<FPL, MAXV> &C, double qx, double qy, double qz, double qb, int qid) {
+// Cuts the cell by qx x + qy y + qz z <= qb.
+// Outcome: 0 done, 1 a capacity was exceeded, 2 degenerate geometry.
+template <int VB, int MAXP>
+__device__ __forceinline__ int cut3(Cell3<VB, MAXP> &C, Work3<VB, MAXP> &W, int &nr, double qx, double qy, double qz,
+                                    double qb, int qid) {
+    constexpr int PW = MAXP / 32;
+    // the small cells keep the masks of faces in registers, and give the
+    // places of removed vertices to new ones, so that most use one block
+    constexpr bool SMALL = VB <= 2 && PW <= 2;
     const int lane = threadIdx.x & 31;
-    auto &F = C.F;
-    auto outside = [&](int v, int f) {
-        const int i = F.at(v, f);
-        return qb - (qx * F.X[i] + qy * F.Y[i] + qz * F.Z[i]) < 0.0;
-    };
-    // faces of at most 32 vertices keep the classification as a bit mask
-    constexpr bool MASKED = MAXV <= 32;
-    int nouts[FPL];
-    unsigned om[FPL];
-    bool has = false;
-#pragma unroll
-    for (int r = 0; r < FPL; ++r) {
-        const int f = lane + 32 * r;
-        int c = 0;
-        unsigned mk = 0;
-        for (int v = 0; v < C.nv[r]; ++v) {
-            const bool o = outside(v, f);
-            c += o;
-            if (MASKED) mk |= unsigned(o) << v;
-        }
-        nouts[r] = c;
-        om[r] = mk;
-        has |= c != 0;
+    const unsigned below = (1u << lane) - 1u;
+    unsigned any = 0, kept = 0;
+    each_block<VB>(nr, [&](int r) {
+        const unsigned al = C.alive[r];
+        const int v = lane + 32 * r;
+        const bool o = (al >> lane & 1u) && qb - (qx * C.x[v] + qy * C.y[v] + qz * C.z[v]) < 0.0;
+        const unsigned om = __ballot_sync(FULL, o);
+        if (lane == 0) W.out[r] = om;
+        any |= om;
+        kept |= al & ~om;
+    });
+    if (!any) return 0;
+    if (!SMALL && lane < PW) W.rm[lane] = W.hm[lane] = 0;
+    __syncwarp();
+    if (!kept) {  // nothing is left
+        if (lane < PW) C.live[lane] = 0;
+        nr = 0;
+        __syncwarp();
+        return 0;
     }
-    if (!__any_sync(FULL, has)) return 0;
-    // ---- cut every face
-    bool cut[FPL];
-    int exit_nb[FPL];
-    double ex[FPL], ey[FPL], ez[FPL];  // entry point of each cut face
-    bool bad = false, over = false;
+    // ---- the edges that cross the cut, and the faces touched
+    unsigned long long rm = 0, hm = 0;  // SMALL: faces of the removed vertices, faces cut through
+    int m = 0;
+    each_block<VB>(nr, [&](int r) {
+        const unsigned om = W.out[r];
+        if (!om) return;
+        const int v = lane + 32 * r;
+        unsigned hz = 0;
+        int f[3] = {0, 0, 0};
+        if (om >> lane & 1u) {
 #pragma unroll
-    for (int r = 0; r < FPL; ++r) {
-        const int f = lane + 32 * r;
-        cut[r] = false;
-        exit_nb[r] = 0;
-        ex[r] = ey[r] = ez[r] = 0;
-        const int n = C.nv[r];
-        const int nout = nouts[r];
-        if (n == 0 || nout == 0) continue;
-        if (nout == n) {  // the whole face is removed
-            C.nv[r] = 0;
-            continue;
-        }
-        // the outside run: o1 its first vertex (predecessor inside), o2 its
-        // last (successor inside); one run only, else the face is cut twice
-        int o1 = -1, o2 = -1, runs = 0;
-        if (MASKED) {
-            // run starts: outside with the previous vertex inside; ends:
-            // outside with the next vertex inside (cyclic over n bits)
-            const unsigned mk = om[r], valid = n >= 32 ? ~0u : (1u << n) - 1u;
-            const unsigned prevm = ((mk << 1) | (mk >> (n - 1))) & valid;
-            const unsigned nextm = ((mk >> 1) | ((mk & 1u) << (n - 1))) & valid;
-            const unsigned starts = mk & ~prevm, ends = mk & ~nextm;
-            runs = __popc(starts);
-            o1 = __ffs(int(starts)) - 1;
-            o2 = __ffs(int(ends)) - 1;
-        } else {
-            bool prev = outside(n - 1, f);
-            for (int v = 0; v < n; ++v) {
-                const bool o = outside(v, f);
-                if (o && !prev) {
-                    o1 = v;
-                    ++runs;
-                }
-                if (!o && prev) o2 = v == 0 ? n - 1 : v - 1;
-                prev = o;
+            for (int i = 0; i < 3; ++i) {
+                const int u = C.nb[i][v];
+                f[i] = C.fp[i][v];
+                hz |= unsigned(!(W.out[u >> 5] >> (u & 31) & 1u)) << i;
+                if (SMALL)
+                    rm |= 1ull << f[i];
+                else
+                    atomicOr(&W.rm[f[i] >> 5], 1u << (f[i] & 31));
             }
         }
-        if (runs != 1 || o1 < 0 || o2 < 0) {
-            bad = true;
-            continue;
-        }
-        const int il = o1 == 0 ? n - 1 : o1 - 1;  // last inside vertex before the run
-        const int fi = o2 == n - 1 ? 0 : o2 + 1;  // first inside vertex after it
-        const int nn = n - nout + 2;
-        if (nn > MAXV) {
-            over = true;
-            continue;
-        }
-        // the two new points, each from its edge's inside vertex
-        auto interp = [&](int vin, int vout, double &px, double &py, double &pz) {
-            const int a = F.at(vin, f), c = F.at(vout, f);
-            const double din = qb - (qx * F.X[a] + qy * F.Y[a] + qz * F.Z[a]);
-            const double dout = qb - (qx * F.X[c] + qy * F.Y[c] + qz * F.Z[c]);
-            const double t = din / (din - dout);
-            px = F.X[a] + t * (F.X[c] - F.X[a]);
-            py = F.Y[a] + t * (F.Y[c] - F.Y[a]);
-            pz = F.Z[a] + t * (F.Z[c] - F.Z[a]);
-        };
-        double xx, xy, xz, nx, ny, nz;
-        interp(il, o1, xx, xy, xz);  // exit point, on edge il -> o1
-        interp(fi, o2, nx, ny, nz);  // entry point, on edge o2 -> fi
-        const int xnb = F.E[F.at(il, f)], nnb = F.E[F.at(o2, f)];
-        auto move = [&](int dst, int src) {
-            const int a = F.at(dst, f), c = F.at(src, f);
-            F.X[a] = F.X[c];
-            F.Y[a] = F.Y[c];
-            F.Z[a] = F.Z[c];
-            F.E[a] = F.E[c];
-        };
-        int px_at;  // index of the exit point in the new polygon
-        if (o1 <= o2) {
-            // outside run inside the list: [0, o1) X N [o2 + 1, n)
-            const int delta = (o1 + 2) - (o2 + 1);
-            if (delta > 0)
-                for (int k = n - 1; k > o2; --k) move(k + delta, k);
-            else if (delta < 0)
-                for (int k = o2 + 1; k < n; ++k) move(k + delta, k);
-            px_at = o1;
-        } else {
-            // the outside run wraps: inside run [o2 + 1, o1) moves to the front
-            const int m = o1 - o2 - 1;
-            for (int k = 0; k < m; ++k) move(k, o2 + 1 + k);
-            px_at = m;
-        }
-        const int a0 = F.at(px_at, f), a1 = F.at(px_at + 1, f);
-        F.X[a0] = xx;
-        F.Y[a0] = xy;
-        F.Z[a0] = xz;
-        F.E[a0] = qid;
-        F.X[a1] = nx;
-        F.Y[a1] = ny;
-        F.Z[a1] = nz;
-        F.E[a1] = nnb;
-        C.nv[r] = nn;
-        cut[r] = true;
-        exit_nb[r] = xnb;
-        ex[r] = nx;
-        ey[r] = ny;
-        ez[r] = nz;
-    }
-    if (__any_sync(FULL, bad)) return 2;
-    if (__any_sync(FULL, over)) return 1;
-    // ---- the new face: a free slot, vertices chained over the cut faces
-    unsigned cutm[FPL], freem[FPL];
+        const int c = __popc(hz);
+        const unsigned b0 = __ballot_sync(FULL, c & 1), b1 = __ballot_sync(FULL, c & 2);
+        int k = m + __popc(b0 & below) + 2 * __popc(b1 & below);
+        m += __popc(b0) + 2 * __popc(b1);
 #pragma unroll
-    for (int r = 0; r < FPL; ++r) {
-        cutm[r] = __ballot_sync(FULL, cut[r]);
-        freem[r] = __ballot_sync(FULL, C.nv[r] == 0);
-    }
-    int m = 0, slot = -1, start = -1;
-#pragma unroll
-    for (int r = 0; r < FPL; ++r) {
-        m += __popc(cutm[r]);
-        if (slot < 0 && freem[r]) slot = 32 * r + __ffs(freem[r]) - 1;
-        if (start < 0 && cutm[r]) start = 32 * r + __ffs(cutm[r]) - 1;
-    }
-    if (m == 0) return 0;  // only whole faces were removed
+        for (int i = 0; i < 3; ++i)
+            if (hz >> i & 1u) {
+                if (k < MAXP) W.req[k] = (unsigned short)(v | i << 10);
+                const int a = f[i == 2 ? 0 : i + 1];
+                if (SMALL)
+                    hm |= 1ull << a;
+                else
+                    atomicOr(&W.hm[a >> 5], 1u << (a & 31));
+                ++k;
+            }
+    });
     if (m < 3) return 2;
-    if (slot < 0 || m > MAXV) return 1;
-    int cur = start;
-    for (int i = 0; i < m; ++i) {
-        // broadcast the current cut face's entry point, exit neighbour and id
-        const int cl = cur & 31, cr = cur >> 5;
-        double px = 0, py = 0, pz = 0;
-        int nb = 0, id = 0;
-#pragma unroll
-        for (int r = 0; r < FPL; ++r)
-            if (r == cr) {
-                px = shfl(ex[r], cl);
-                py = shfl(ey[r], cl);
-                pz = shfl(ez[r], cl);
-                nb = __shfl_sync(FULL, exit_nb[r], cl);
-                id = __shfl_sync(FULL, C.fid[r], cl);
-            }
-        if (lane == (slot & 31)) {
-            const int a = F.at(i, slot);
-            F.X[a] = px;
-            F.Y[a] = py;
-            F.Z[a] = pz;
-            F.E[a] = id;
+    if (m > MAX_NEW || m > MAXP) return 1;
+    // ---- the new face's slot: the lowest one free once the faces that lost
+    // every vertex (touched, not cut through) are gone
+    int slot;
+    if constexpr (SMALL) {
+        unsigned long long live = C.live[0];
+        if (PW == 2) live |= (unsigned long long)C.live[PW - 1] << 32;
+        const unsigned g0 = __reduce_or_sync(FULL, unsigned(rm)), h0 = __reduce_or_sync(FULL, unsigned(hm));
+        unsigned g1 = 0, h1 = 0;
+        if (PW == 2 && live >> 32) {
+            g1 = __reduce_or_sync(FULL, unsigned(rm >> 32));
+            h1 = __reduce_or_sync(FULL, unsigned(hm >> 32));
         }
-        // next: the cut face whose id is the exit neighbour
-        int next = -1;
-#pragma unroll
-        for (int r = 0; r < FPL; ++r) {
-            const unsigned hit = __ballot_sync(FULL, cut[r] && C.fid[r] == nb);
-            if (next < 0 && hit) next = 32 * r + __ffs(hit) - 1;
-        }
-        if (next < 0) return 2;
-        cur = next;
+        live &= ~(((unsigned long long)g1 << 32 | g0) & ~((unsigned long long)h1 << 32 | h0));
+        slot = __ffsll((long long)~live) - 1;
+        if (slot < 0 || slot >= MAXP) return 1;
+        live |= 1ull << slot;
+        __syncwarp();
+        if (lane < PW) C.live[lane] = unsigned(live >> (32 * lane));
+    } else {
+        __syncwarp();
+        unsigned lw = FULL;
+        if (lane < PW) lw = C.live[lane] & ~(W.rm[lane] & ~W.hm[lane]);
+        const unsigned room = __ballot_sync(FULL, lw != FULL);
+        if (!room) return 1;
+        const int word = __ffs(int(room)) - 1;
+        slot = 32 * word + __ffs(int(~__shfl_sync(FULL, lw, word))) - 1;
+        if (lane == word) lw |= 1u << (slot & 31);
+        if (lane < PW) C.live[lane] = lw;
     }
-    if (cur != start) return 2;
+    // ---- the new vertices
+    struct New {
+        double x, y, z;
+        int a, b, n;
+    };
+    // request q: the edge from a removed vertex t to the kept vertex n
+    auto compute = [&](int q) {
+        New w;
+        const int t = q & 1023, i = q >> 10;
+        const int ia = next3(i), ib = next3(ia);
+        w.a = C.fp[ia][t];
+        w.b = C.fp[ib][t];
+        w.n = C.nb[i][t];
+        const double tx = C.x[t], ty = C.y[t], tz = C.z[t], ux = C.x[w.n], uy = C.y[w.n], uz = C.z[w.n];
+        const double din = qb - (qx * ux + qy * uy + qz * uz), dout = qb - (qx * tx + qy * ty + qz * tz);
+        const double s = din / (din - dout);
+        w.x = ux + s * (tx - ux);
+        w.y = uy + s * (ty - uy);
+        w.z = uz + s * (tz - uz);
+        return w;
+    };
+    auto store = [&](int v, const New &w) {
+        C.x[v] = w.x;
+        C.y[v] = w.y;
+        C.z[v] = w.z;
+        C.fp[0][v] = (unsigned short)slot;
+        C.fp[1][v] = (unsigned short)w.a;
+        C.fp[2][v] = (unsigned short)w.b;
+        C.nb[0][v] = (unsigned short)w.n;
+        W.ta[w.a] = W.tb[w.b] = (unsigned short)v;
 #pragma unroll
-    for (int r = 0; r < FPL; ++r)
-        if (lane + 32 * r == slot) {
-            C.fid[r] = qid;
-            C.nv[r] = m;
-            C.ax[r] = qx;
-            C.ay[r] = qy;
-            C.az[r] = qz;
-            C.b[r] = qb;
+        for (int j = 0; j < 3; ++j) {
+            const int f = C.fp[j][w.n];
+            if (f != w.a && f != w.b) C.nb[j][w.n] = (unsigned short)v;
         }
+    };
+    unsigned mine = 0;  // bit r: this lane's vertex of block r is new
+    int base = 0, top = 0;
+    if constexpr (SMALL) {
+        New w[VB];
+        unsigned now[VB];
+#pragma unroll
+        for (int r = 0; r < VB; ++r) {
+            now[r] = r < nr ? C.alive[r] & ~W.out[r] : 0u;
+            if (base < m) {
+                const int rank = base + __popc(~now[r] & below);
+                if (!(now[r] >> lane & 1u) && rank < m) {
+                    mine |= 1u << r;
+                    w[r] = compute(W.req[rank]);
+                }
+                base += 32 - __popc(now[r]);
+                now[r] |= __ballot_sync(FULL, mine >> r & 1u);
+            }
+            if (now[r]) top = r + 1;
+        }
+        if (base < m) return 1;
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < VB; ++r) {
+            if (mine >> r & 1u) store(lane + 32 * r, w[r]);
+            if (lane == 0) C.alive[r] = now[r];
+        }
+    } else {
+        // in places that were free before the cut: a removed vertex is read
+        // until the last new one is made
+        for (int r = 0; r < VB && (r < nr || base < m); ++r) {
+            const unsigned al = r < nr ? C.alive[r] : 0u;
+            const int rank = base + __popc(~al & below);
+            const bool make = !(al >> lane & 1u) && rank < m;
+            if (make) {
+                store(lane + 32 * r, compute(W.req[rank]));
+                mine |= 1u << r;
+            }
+            base += __popc(~al);
+            const unsigned now = (r < nr ? al & ~W.out[r] : 0u) | __ballot_sync(FULL, make);
+            __syncwarp();
+            if (lane == 0) C.alive[r] = now;
+            if (now) top = r + 1;
+        }
+        if (base < m) return 1;
+    }
+    nr = top;
+    if (lane == 0) {
+        C.pid[slot] = qid;
+        C.plane[slot][0] = qx;
+        C.plane[slot][1] = qy;
+        C.plane[slot][2] = qz;
+        C.plane[slot][3] = qb;
+    }
+    __syncwarp();
+    // ---- link them around the new face: across the edge of the cut and face
+    // b lies the new vertex that has b second, and so on.  Where a face was
+    // entered twice, or entered and not left (the outside vertices are not one
+    // patch), the tables do not agree
+    bool bad = false;
+    each_block<VB>(nr, [&](int r) {
+        if (!(mine >> r & 1u)) return;
+        const int v = lane + 32 * r, a = C.fp[1][v], b = C.fp[2][v];
+        const int p = W.ta[b], q = W.tb[a];
+        bad |= W.ta[a] != v || W.tb[b] != v;
+        bad |= p >= 32 * VB || !(C.alive[p >> 5] >> (p & 31) & 1u) || C.fp[0][p] != slot || C.fp[1][p] != b;
+        bad |= q >= 32 * VB || !(C.alive[q >> 5] >> (q & 31) & 1u) || C.fp[0][q] != slot || C.fp[2][q] != a;
+        C.nb[1][v] = (unsigned short)p;
+        C.nb[2][v] = (unsigned short)q;
+    });
+    if (__any_sync(FULL, bad)) return 2;
     __syncwarp();
     return 0;
+}
+
+// The distance of p from [lo, hi] (the signs read as integers: an FP64
+// minimum and maximum take several times the instructions).
+__device__ __forceinline__ double gap(double lo, double hi, double p) {
+    const double a = lo - p, b = p - hi;
+    return __double2hiint(a) >= 0 ? a : __double2hiint(b) >= 0 ? b : 0.0;
 }
 
 // A multilinear density rewritten about the cell's Dirac c: coefficients of
@@ -316,78 +351,38 @@ struct PolyRel {
     }
 };
 
-// The domain box as six faces (slots 0..5), relative to c0.
-template <int FPL, int MAXV>
-__device__ __forceinline__ void init_box(Cell3<FPL, MAXV> &C, const Cell3DArgs &A, double c0x, double c0y, double c0z) {
+// The domain box as six faces (slots 0..5: x-lo, x-hi, y-lo, ...) and eight
+// vertices (vertex v at corner bits x, y, z = 0, 1, 2 of v: 0 lo, 1 hi).
+template <int VB, int MAXP>
+__device__ __forceinline__ void init_box(Cell3<VB, MAXP> &C, int &nr, const Cell3DArgs &A, double c0x, double c0y,
+                                         double c0z) {
     const int lane = threadIdx.x & 31;
-    const double lo[3] = {A.box_lo[0] - c0x, A.box_lo[1] - c0y, A.box_lo[2] - c0z};
-    const double hi[3] = {A.box_hi[0] - c0x, A.box_hi[1] - c0y, A.box_hi[2] - c0z};
-    // corners: bit 0 -> x, bit 1 -> y, bit 2 -> z (0: lo, 1: hi)
-    // per face: 4 corners counter-clockwise seen from outside, and the face
-    // across each edge (faces: 0 x-lo, 1 x-hi, 2 y-lo, 3 y-hi, 4 z-lo, 5 z-hi)
-    constexpr int corner[6][4] = {{0, 4, 6, 2}, {1, 3, 7, 5}, {0, 1, 5, 4}, {2, 6, 7, 3}, {0, 2, 3, 1}, {4, 5, 7, 6}};
-    constexpr int across[6][4] = {{2, 5, 3, 4}, {4, 3, 5, 2}, {4, 1, 5, 0}, {0, 5, 1, 4}, {0, 3, 1, 2}, {2, 1, 3, 0}};
-#pragma unroll
-    for (int r = 0; r < FPL; ++r) {
-        const int f = lane + 32 * r;
-        C.nv[r] = 0;
-        C.fid[r] = 0;
-        C.ax[r] = C.ay[r] = C.az[r] = C.b[r] = 0;
-        if (f < 6) {
-            const int ax = f >> 1, side = f & 1;
-            C.nv[r] = 4;
-            C.fid[r] = domain_id(f);
-            double nrm[3] = {0, 0, 0};
-            nrm[ax] = side ? 1.0 : -1.0;
-            C.ax[r] = nrm[0];
-            C.ay[r] = nrm[1];
-            C.az[r] = nrm[2];
-            C.b[r] = side ? hi[ax] : -lo[ax];
-            for (int v = 0; v < 4; ++v) {
-                const int c = corner[f][v];
-                const int a = C.F.at(v, f);
-                C.F.X[a] = (c & 1) ? hi[0] : lo[0];
-                C.F.Y[a] = (c & 2) ? hi[1] : lo[1];
-                C.F.Z[a] = (c & 4) ? hi[2] : lo[2];
-                C.F.E[a] = domain_id(across[f][v]);
-            }
-        }
+    if (lane < 8) {
+        const int bx = lane & 1, by = lane >> 1 & 1, bz = lane >> 2 & 1;
+        C.x[lane] = (bx ? A.box_hi[0] : A.box_lo[0]) - c0x;
+        C.y[lane] = (by ? A.box_hi[1] : A.box_lo[1]) - c0y;
+        C.z[lane] = (bz ? A.box_hi[2] : A.box_lo[2]) - c0z;
+        // faces x, y, z run counter-clockwise at the corner (hi, hi, hi), and
+        // the other way round where an odd number of coordinates is lo
+        const bool odd = !((bx + by + bz) & 1);
+        C.fp[0][lane] = (unsigned short)bx;
+        C.nb[0][lane] = (unsigned short)(lane ^ 1);
+        C.fp[odd ? 2 : 1][lane] = (unsigned short)(2 + by);
+        C.nb[odd ? 2 : 1][lane] = (unsigned short)(lane ^ 2);
+        C.fp[odd ? 1 : 2][lane] = (unsigned short)(4 + bz);
+        C.nb[odd ? 1 : 2][lane] = (unsigned short)(lane ^ 4);
     }
+    if (lane < 6) {
+        const int ax = lane >> 1, side = lane & 1;
+        const double c = ax == 0 ? c0x : ax == 1 ? c0y : c0z;
+        for (int d = 0; d < 3; ++d) C.plane[lane][d] = d == ax ? (side ? 1.0 : -1.0) : 0.0;
+        C.plane[lane][3] = side ? A.box_hi[ax] - c : -(A.box_lo[ax] - c);
+        C.pid[lane] = domain_id(lane);
+    }
+    for (int r = lane; r < VB; r += 32) C.alive[r] = r == 0 ? 0xffu : 0u;
+    if (lane < MAXP / 32) C.live[lane] = lane == 0 ? 0x3fu : 0u;
+    nr = 1;
     __syncwarp();
-}
-
-// Writes a row of `cnt` entries: the lanes' neighbour faces (slot r of a
-// lane writes entry pos[r] when mine[r]), then the diagonal from lane 0 when
-// with_diag, into the ELL slots or, for a long row, the side buffer.
-template <int FPL>
-__device__ __forceinline__ bool write_row(const Rows &R, long long s, int cnt, const int *pos, const bool *mine, const int *col,
-                          const double *val, bool with_diag, int diag_col, double diag_val) {
-    const int lane = threadIdx.x & 31;
-    long long off = 0;
-    const bool side = cnt > R.cap;
-    if (side) {
-        unsigned long long o = 0;
-        if (lane == 0) o = atomicAdd(R.side_used, (unsigned long long)cnt);
-        o = __shfl_sync(FULL, o, 0);
-        if ((long long)(o + cnt) > R.side_cap) return false;
-        off = (long long)o;
-        if (lane == 0) R.side[s] = off;
-    }
-    auto put = [&](int k, int c, double v) {
-        if (side) {
-            R.side_col[off + k] = c;
-            if (R.side_val) R.side_val[off + k] = v;
-        } else {
-            R.col[k * R.stride + s] = c;
-            if (R.val) R.val[k * R.stride + s] = v;
-        }
-    };
-#pragma unroll
-    for (int r = 0; r < FPL; ++r)
-        if (mine[r]) put(pos[r], col[r], val[r]);
-    if (with_diag && lane == 0) put(cnt - 1, diag_col, diag_val);
-    if (lane == 0) R.cnt[s] = cnt;
-    return true;
 }
 
 // First failed guard of a 3D cell (the 2D kernels' guard_fail).
@@ -399,95 +394,166 @@ __device__ void guard_fail3(const Cell3DArgs &A, int code, long long s, long lon
     flag_error(A.err, DE_GUARD);
 }
 
-// Volume, first moments (relative to c0) and per face slot the area of the
-// faces of C, the pyramids of apex c0 over the faces (this lane's slots only;
-// the caller sums over the warp).  Constant density.
-template <int FPL, int MAXV>
-__device__ __forceinline__ void face_volumes(const Cell3<FPL, MAXV> &C, double &vol, double &mx, double &my, double &mz,
-                             double *area_r) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int r = 0; r < FPL; ++r) {
-        const int f = lane + 32 * r;
-        const int n = C.nv[r];
-        area_r[r] = 0;
-        if (n < 3) continue;
-        const double na = sqrt(C.ax[r] * C.ax[r] + C.ay[r] * C.ay[r] + C.az[r] * C.az[r]);
-        const double ux = C.ax[r] / na, uy = C.ay[r] / na, uz = C.az[r] / na;
-        const int i0 = C.F.at(0, f);
-        const double x0 = C.F.X[i0], y0 = C.F.Y[i0], z0 = C.F.Z[i0];
-        double area = 0, fx = 0, fy = 0, fz = 0;
-        for (int k = 1; k + 1 < n; ++k) {
-            const int i1 = C.F.at(k, f), i2 = C.F.at(k + 1, f);
-            const double e1x = C.F.X[i1] - x0, e1y = C.F.Y[i1] - y0, e1z = C.F.Z[i1] - z0;
-            const double e2x = C.F.X[i2] - x0, e2y = C.F.Y[i2] - y0, e2z = C.F.Z[i2] - z0;
-            const double ta =
-                0.5 * ((e1y * e2z - e1z * e2y) * ux + (e1z * e2x - e1x * e2z) * uy + (e1x * e2y - e1y * e2x) * uz);
-            area += ta;
-            fx += ta * (3 * x0 + e1x + e2x);
-            fy += ta * (3 * y0 + e1y + e2y);
-            fz += ta * (3 * z0 + e1z + e2z);
-        }
-        const double h = C.b[r] / na;
-        const double v = h * area / 3;
-        vol += v;
-        if (area != 0) {
-            const double k = v * 0.75 / (3 * area);
-            mx += k * fx;
-            my += k * fy;
-            mz += k * fz;
-        }
-        area_r[r] = area;
+// Destination of one row of cnt entries: its ELL slots, or a place in the side
+// buffer for a long row (called by the whole warp; ok: false when the side
+// buffer is full).  Rows that are not wanted (R.cnt null) are skipped.
+struct RowPut {
+    const Rows &R;
+    long long s, off = 0;
+    int cnt;
+    bool side, ok = true;
+    __device__ RowPut(const Rows &r, long long s_, int c) : R(r), s(s_), cnt(c), side(r.cnt && c > r.cap) {
+        if (!side) return;
+        unsigned long long o = 0;
+        if ((threadIdx.x & 31) == 0) o = atomicAdd(R.side_used, (unsigned long long)cnt);
+        o = __shfl_sync(FULL, o, 0);
+        off = (long long)o;
+        ok = off + cnt <= R.side_cap;
     }
+    __device__ void put(int k, int c, double v) const {
+        if (!R.cnt || !ok) return;
+        if (side) {
+            R.side_col[off + k] = c;
+            if (R.side_val) R.side_val[off + k] = v;
+        } else {
+            R.col[k * R.stride + s] = c;
+            if (R.val) R.val[k * R.stride + s] = v;
+        }
+    }
+    __device__ void finish() const {  // one lane
+        if (!R.cnt) return;
+        if (side) R.side[s] = off;
+        R.cnt[s] = cnt;
+    }
+};
+
+// The outputs of a cell that could not be built.
+__device__ void fail_cell(const Cell3DArgs &A, long long s) {
+    if (A.mass) A.mass[s] = nan("");
+    if (A.ctd) A.ctd[3 * s] = A.ctd[3 * s + 1] = A.ctd[3 * s + 2] = nan("");
+    if (A.rows.cnt) {
+        A.rows.cnt[s] = 1;
+        A.rows.col[s] = int(s);
+        A.rows.val[s] = 0.0;
+    }
+    if (A.nb.cnt) A.nb.cnt[s] = 0;
+}
+
+// The faces of the cell in slot order into W.list, and the lowest vertex of
+// each into W.first; returns their number, or -1 where the numbers of faces
+// and vertices are not those of a polyhedron (V = 2 F - 4).
+template <int VB, int MAXP>
+__device__ __forceinline__ int list_faces(const Cell3<VB, MAXP> &C, Work3<VB, MAXP> &W, int nr) {
+    const int lane = threadIdx.x & 31;
+    int nf = 0, nv = 0;
+#pragma unroll
+    for (int w = 0; w < MAXP / 32; ++w) {
+        const unsigned lw = C.live[w];
+        W.first[32 * w + lane] = 32 * VB;
+        if (lw >> lane & 1u) W.list[nf + __popc(lw & ((1u << lane) - 1u))] = (unsigned short)(32 * w + lane);
+        nf += __popc(lw);
+    }
+    __syncwarp();
+    for (int r = 0; r < nr; ++r) {
+        const unsigned al = C.alive[r];
+        nv += __popc(al);
+        if (al >> lane & 1u)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) atomicMin(&W.first[C.fp[i][lane + 32 * r]], lane + 32 * r);
+    }
+    __syncwarp();
+    return nv == (nf ? 2 * nf - 4 : 0) ? nf : -1;
+}
+
+// Walks the polygon of face f counter-clockwise and calls tri(x0, y0, z0, e1,
+// e2) for the triangles of its fan from the lowest vertex (e1, e2 from that
+// vertex).  At most 32 VB steps; false where the walk does not close.
+template <int VB, int MAXP, class F>
+__device__ __forceinline__ bool walk_face(const Cell3<VB, MAXP> &C, const Work3<VB, MAXP> &W, int f, F &&tri) {
+    const int v0 = W.first[f];
+    if (v0 >= 32 * VB) return false;
+    const double x0 = C.x[v0], y0 = C.y[v0], z0 = C.z[v0];
+    auto step = [&](int v) { return int(C.fp[0][v] == f ? C.nb[1][v] : C.fp[1][v] == f ? C.nb[2][v] : C.nb[0][v]); };
+    int v = step(v0);
+    double ax = C.x[v] - x0, ay = C.y[v] - y0, az = C.z[v] - z0;
+    for (int k = 0; k < 32 * VB; ++k) {
+        v = step(v);
+        if (v == v0) return true;
+        const double bx = C.x[v] - x0, by = C.y[v] - y0, bz = C.z[v] - z0;
+        tri(x0, y0, z0, ax, ay, az, bx, by, bz);
+        ax = bx;
+        ay = by;
+        az = bz;
+    }
+    return false;
+}
+
+// Integrals of one face at constant density: its area and the sum over its
+// fan of (triangle area) x 3 (triangle centroid).
+template <int VB, int MAXP>
+__device__ __forceinline__ bool face_area(const Cell3<VB, MAXP> &C, const Work3<VB, MAXP> &W, int f, double ux, double uy,
+                                          double uz, double &area, double &fx, double &fy, double &fz) {
+    return walk_face(C, W, f, [&](double x0, double y0, double z0, double e1x, double e1y, double e1z, double e2x,
+                                  double e2y, double e2z) {
+        const double ta =
+            0.5 * ((e1y * e2z - e1z * e2y) * ux + (e1z * e2x - e1x * e2z) * uy + (e1x * e2y - e1y * e2x) * uz);
+        area += ta;
+        fx += ta * (3 * x0 + e1x + e2x);
+        fy += ta * (3 * y0 + e1y + e2y);
+        fz += ta * (3 * z0 + e1z + e2z);
+    });
+}
+
+// Adds a face's pyramid of apex c0 (area, moments as face_area gives them, h
+// the signed distance of its plane from c0): the centroid of a pyramid lies 3/4
+// of the way from the apex to that of the face.
+__device__ __forceinline__ void add_pyramid(double h, double area, double fx, double fy, double fz, double &vol,
+                                            double &mx, double &my, double &mz) {
+    const double v = h * area / 3;
+    vol += v;
+    if (area != 0) {
+        const double k = v * 0.75 / (3 * area);
+        mx += k * fx;
+        my += k * fy;
+        mz += k * fz;
+    }
+}
+
+template <class T>
+__device__ __forceinline__ void copy_cell(T &dst, const T &src) {
+    static_assert(sizeof(T) % 8 == 0, "copied by 8 bytes");
+    const double *s = reinterpret_cast<const double *>(&src);
+    double *d = reinterpret_cast<double *>(&dst);
+    for (int i = threadIdx.x & 31; i < int(sizeof(T) / 8); i += 32) d[i] = s[i];
+    __syncwarp();
 }
 
 // The cell integrated voxel by voxel (ScaledImage::for_each_intersection,
 // ScaledImage.tcc:98-149: each voxel box intersected with the cell and
-// integrated with the voxel's value): the faces are saved to the warp's
-// backup, and for every voxel that the cell's bounding box meets the faces
-// are restored and cut by the voxel's six planes, then integrated.  Sums
-// (this lane's slots) into vol, m*, and per slot the value-weighted area of
-// the Dirac faces.  Returns 0, or 1 / 2 as cut3 (capacity, degenerate).
-template <int FPL, int MAXV>
-__device__ __forceinline__ int voxel_integrals(const Cell3DArgs &A, Cell3<FPL, MAXV> &C, char *backup, double c0x, double c0y,
-                               double c0z, double &vol, double &mx, double &my, double &mz, double *wa_r) {
+// integrated with the voxel's value): for every voxel that the cell's bounding
+// box meets a copy of the cell is cut by the voxel's six planes and
+// integrated.  Sums (this lane's faces) into vol, m*, and per face slot of the
+// cell the value-weighted area into wa.  Leaves the cell in C.  Returns 0, or
+// 1 / 2 as cut3 (capacity, degenerate).
+template <int VB, int MAXP>
+__device__ int voxel_integrals(const Cell3DArgs &A, Cell3<VB, MAXP> &C, Work3<VB, MAXP> &W, Cell3<VB, MAXP> &B, double *wa,
+                               int &nr, double c0x, double c0y, double c0z, double &vol, double &mx, double &my,
+                               double &mz) {
     const int lane = threadIdx.x & 31;
-    Faces<FPL, MAXV> B;
-    constexpr int MAXF = 32 * FPL;
-    B.X = reinterpret_cast<double *>(backup);
-    B.Y = B.X + MAXV * MAXF;
-    B.Z = B.Y + MAXV * MAXF;
-    B.E = reinterpret_cast<int *>(B.Z + MAXV * MAXF);
-    int fid0[FPL], nv0[FPL];
-    double ax0[FPL], ay0[FPL], az0[FPL], b0[FPL];
+    for (int f = lane; f < MAXP; f += 32) wa[f] = 0;
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-#pragma unroll
-    for (int r = 0; r < FPL; ++r) {
-        const int f = lane + 32 * r;
-        fid0[r] = C.fid[r];
-        nv0[r] = C.nv[r];
-        ax0[r] = C.ax[r];
-        ay0[r] = C.ay[r];
-        az0[r] = C.az[r];
-        b0[r] = C.b[r];
-        wa_r[r] = 0;
-        for (int v = 0; v < C.nv[r]; ++v) {
-            const int i = C.F.at(v, f);
-            B.X[i] = C.F.X[i];
-            B.Y[i] = C.F.Y[i];
-            B.Z[i] = C.F.Z[i];
-            B.E[i] = C.F.E[i];
-            lo[0] = fmin(lo[0], C.F.X[i]); hi[0] = fmax(hi[0], C.F.X[i]);
-            lo[1] = fmin(lo[1], C.F.Y[i]); hi[1] = fmax(hi[1], C.F.Y[i]);
-            lo[2] = fmin(lo[2], C.F.Z[i]); hi[2] = fmax(hi[2], C.F.Z[i]);
+    for (int r = 0; r < nr; ++r)
+        if (C.alive[r] >> lane & 1u) {
+            const int v = lane + 32 * r;
+            lo[0] = fmin(lo[0], C.x[v]); hi[0] = fmax(hi[0], C.x[v]);
+            lo[1] = fmin(lo[1], C.y[v]); hi[1] = fmax(hi[1], C.y[v]);
+            lo[2] = fmin(lo[2], C.z[v]); hi[2] = fmax(hi[2], C.z[v]);
         }
-    }
     for (int d = 0; d < 3; ++d)
         for (int o = 16; o > 0; o >>= 1) {
             lo[d] = fmin(lo[d], __shfl_xor_sync(FULL, lo[d], o));
             hi[d] = fmax(hi[d], __shfl_xor_sync(FULL, hi[d], o));
         }
-    __syncwarp();
     if (!(lo[0] <= hi[0])) return 0;  // an empty cell
     const double c0[3] = {c0x, c0y, c0z};
     int i0[3], i1[3];
@@ -497,29 +563,15 @@ __device__ __forceinline__ int voxel_integrals(const Cell3DArgs &A, Cell3<FPL, M
         i0[d] = max(0, int(floor((lo[d] + c0[d] - A.img_lo[d]) / ps[d])));
         i1[d] = min(A.img_n[d] - 1, int(floor((hi[d] + c0[d] - A.img_lo[d]) / ps[d])));
     }
+    const int nr0 = nr;
+    __syncwarp();
+    copy_cell(B, C);
     for (int iz = i0[2]; iz <= i1[2]; ++iz)
         for (int iy = i0[1]; iy <= i1[1]; ++iy)
             for (int ix = i0[0]; ix <= i1[0]; ++ix) {
                 const double val = A.img[((long long)iz * A.img_n[1] + iy) * A.img_n[0] + ix];
-                // restore the cell
-#pragma unroll
-                for (int r = 0; r < FPL; ++r) {
-                    const int f = lane + 32 * r;
-                    C.fid[r] = fid0[r];
-                    C.nv[r] = nv0[r];
-                    C.ax[r] = ax0[r];
-                    C.ay[r] = ay0[r];
-                    C.az[r] = az0[r];
-                    C.b[r] = b0[r];
-                    for (int v = 0; v < nv0[r]; ++v) {
-                        const int i = C.F.at(v, f);
-                        C.F.X[i] = B.X[i];
-                        C.F.Y[i] = B.Y[i];
-                        C.F.Z[i] = B.Z[i];
-                        C.F.E[i] = B.E[i];
-                    }
-                }
-                __syncwarp();
+                copy_cell(C, B);
+                nr = nr0;
                 // the voxel's six planes, relative to c0
                 const int ii[3] = {ix, iy, iz};
                 for (int d = 0; d < 3; ++d) {
@@ -527,52 +579,48 @@ __device__ __forceinline__ int voxel_integrals(const Cell3DArgs &A, Cell3<FPL, M
                     const double vhi = A.img_lo[d] + ps[d] * (ii[d] + 1) - c0[d];
                     double a[3] = {0, 0, 0};
                     a[d] = -1.0;
-                    int st = cut3(C, a[0], a[1], a[2], -vlo, domain_id(200 + 2 * d));
+                    int st = cut3(C, W, nr, a[0], a[1], a[2], -vlo, domain_id(200 + 2 * d));
                     if (st) return st;
                     a[d] = 1.0;
-                    st = cut3(C, a[0], a[1], a[2], vhi, domain_id(201 + 2 * d));
+                    st = cut3(C, W, nr, a[0], a[1], a[2], vhi, domain_id(201 + 2 * d));
                     if (st) return st;
                 }
-                double v = 0, px = 0, py = 0, pz = 0, ar[FPL];
-                face_volumes(C, v, px, py, pz, ar);
-                vol += val * v;
-                mx += val * px;
-                my += val * py;
-                mz += val * pz;
-#pragma unroll
-                for (int r = 0; r < FPL; ++r)
-                    if (C.fid[r] >= 0 && C.nv[r] >= 3) wa_r[r] += val * ar[r];
+                const int nf = list_faces(C, W, nr);
+                if (nf < 0) return 2;
+                bool closed = true;
+                for (int k = lane; k < nf; k += 32) {
+                    const int f = W.list[k];
+                    const double *q = C.plane[f];
+                    const double na = sqrt(q[0] * q[0] + q[1] * q[1] + q[2] * q[2]);
+                    double area = 0, fx = 0, fy = 0, fz = 0, v = 0, px = 0, py = 0, pz = 0;
+                    closed &= face_area(C, W, f, q[0] / na, q[1] / na, q[2] / na, area, fx, fy, fz);
+                    add_pyramid(q[3] / na, area, fx, fy, fz, v, px, py, pz);
+                    vol += val * v;
+                    mx += val * px;
+                    my += val * py;
+                    mz += val * pz;
+                    // a face of the cell keeps its slot while it lives
+                    if (C.pid[f] >= 0) wa[f] += val * area;
+                }
+                if (!__all_sync(FULL, closed)) return 2;
+                __syncwarp();
             }
-    // restore the cell for the outputs that follow (its faces' ids and planes)
-#pragma unroll
-    for (int r = 0; r < FPL; ++r) {
-        const int f = lane + 32 * r;
-        C.fid[r] = fid0[r];
-        C.nv[r] = nv0[r];
-        C.ax[r] = ax0[r];
-        C.ay[r] = ay0[r];
-        C.az[r] = az0[r];
-        C.b[r] = b0[r];
-        for (int v = 0; v < nv0[r]; ++v) {
-            const int i = C.F.at(v, f);
-            C.F.X[i] = B.X[i];
-            C.F.Y[i] = B.Y[i];
-            C.F.Z[i] = B.Z[i];
-            C.F.E[i] = B.E[i];
-        }
-    }
-    __syncwarp();
+    copy_cell(C, B);
+    nr = nr0;
     return 0;
 }
 
 // Builds and integrates the cell of sorted Dirac s.  Returns 0 (outputs
-// written), 1 (a capacity was exceeded: retry in the large pass), 2 (failed:
+// written), 1 (a capacity was exceeded: retry in the next pass), 2 (failed:
 // outputs written as NaN / empty row, error flagged).
-template <int FPL, int MAXV>
-__device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<FPL, MAXV> &C, char *backup) {
+enum Density3 : int { D_CONST = 0, D_POLY = 1, D_IMAGE = 2 };
+template <int VB, int MAXP, int DENS, int PASS>
+__device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<VB, MAXP> &C, Work3<VB, MAXP> &W,
+                                      Cell3<VB, MAXP> *B, double *wa) {
     const int lane = threadIdx.x & 31;
     const double c0x = A.pos[3 * s], c0y = A.pos[3 * s + 1], c0z = A.pos[3 * s + 2], w0 = A.w[s];
-    init_box(C, A, c0x, c0y, c0z);
+    int nr;
+    init_box(C, nr, A, c0x, c0y, c0z);
     int status = 0;
     // a convex shape: its half-spaces cut the box first (relative to c0:
     // a . u <= b - a . c0), as ConvexPolyhedronAssembly::add_convex_polyhedron
@@ -580,10 +628,9 @@ __device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<FP
     for (int k = 0; k < A.nplanes && status == 0; ++k) {
         const double ax = A.planes[4 * k], ay = A.planes[4 * k + 1], az = A.planes[4 * k + 2];
         const double b = A.planes[4 * k + 3] - (ax * c0x + ay * c0y + az * c0z);
-        const int r = cut3(C, ax, ay, az, b, domain_id(6 + k));
-        if (r) status = r;
+        status = cut3(C, W, nr, ax, ay, az, b, domain_id(6 + k));
     }
-    if (lane == 0) C.stack[0] = 0;
+    if (lane == 0) W.stack[0] = 0;
     __syncwarp();
     int sp = 1;
     for (int visits = 0; sp > 0 && status == 0; ++visits) {
@@ -592,27 +639,27 @@ __device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<FP
             status = 2;
             break;
         }
-        const int node = C.stack[--sp];
+        const int node = W.stack[--sp];
         __syncwarp();
         const TreeNode<3> nd = A.nodes[node];
-        // eviction test (SpZGrid.tcc:475-480) on every vertex of every face
+        // eviction test (SpZGrid.tcc:475-480) on every vertex
         const double lo0 = nd.lo[0] - c0x, lo1 = nd.lo[1] - c0y, lo2 = nd.lo[2] - c0z;
         const double hi0 = nd.hi[0] - c0x, hi1 = nd.hi[1] - c0y, hi2 = nd.hi[2] - c0z;
-        bool fail = false;
-#pragma unroll
-        for (int r = 0; r < FPL; ++r) {
-            const int f = lane + 32 * r;
-            for (int v = 0; v < C.nv[r] && !fail; ++v) {
-                const int i = C.F.at(v, f);
-                const double px = C.F.X[i], py = C.F.Y[i], pz = C.F.Z[i];
-                const double qx = fmin(hi0, fmax(lo0, px)) - px, qy = fmin(hi1, fmax(lo1, py)) - py,
-                             qz = fmin(hi2, fmax(lo2, pz)) - pz;
+        bool need = false;
+        each_block<VB>(nr, [&](int r) {
+            if (need) return;
+            bool fail = false;
+            if (C.alive[r] >> lane & 1u) {
+                const int v = lane + 32 * r;
+                const double px = C.x[v], py = C.y[v], pz = C.z[v];
+                const double qx = gap(lo0, hi0, px), qy = gap(lo1, hi1, py), qz = gap(lo2, hi2, pz);
                 const double lhs = px * px + py * py + pz * pz - w0;
                 const double rhs = qx * qx + qy * qy + qz * qz - nd.maxw;
                 fail = !(lhs <= rhs);
             }
-        }
-        if (!__any_sync(FULL, fail)) continue;
+            need = __any_sync(FULL, fail);
+        });
+        if (!need) continue;
         if (nd.b < 0) {
             const int first = nd.a, nch = -nd.b;
             if (nch < 2 || nch > 8 || first < 1 || first + nch > A.max_nodes) {
@@ -641,7 +688,7 @@ __device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<FP
                 const float kc = __shfl_sync(FULL, key, c);
                 rank += c < nch && (kc > key || (kc == key && c < lane));
             }
-            if (lane < nch) C.stack[sp + rank] = first + lane;
+            if (lane < nch) W.stack[sp + rank] = first + lane;
             __syncwarp();
             sp += nch;
         } else {
@@ -655,90 +702,72 @@ __device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<FP
                 // weighted bisector, relative to c0: V . u <= 1/2 |V|^2 + 1/2 (w0 - w1)
                 const double vx = A.pos[3 * j] - c0x, vy = A.pos[3 * j + 1] - c0y, vz = A.pos[3 * j + 2] - c0z;
                 const double qb = 0.5 * (vx * vx + vy * vy + vz * vz) + 0.5 * (w0 - A.w[j]);
-                const int r = cut3(C, vx, vy, vz, qb, j);
-                if (r) status = r;
+                status = cut3(C, W, nr, vx, vy, vz, qb, j);
             }
         }
     }
     if (status == 1) return 1;
     // ---- integrals over the faces (pyramids with apex c0)
     double vol = 0, mx = 0, my = 0, mz = 0, der0 = 0;
-    int nrow = 0, nnb = 0;
-    int rpos[FPL], npos[FPL];
-    double rval[FPL];
-    bool rmine[FPL], nmine[FPL];
-    double img_area[FPL];  // voxel image: the value-weighted area of each Dirac face
-    if (status == 0 && A.img) {
-        status = voxel_integrals(A, C, backup, c0x, c0y, c0z, vol, mx, my, mz, img_area);
+    if (DENS == D_IMAGE && status == 0) {
+        status = voxel_integrals(A, C, W, *B, wa, nr, c0x, c0y, c0z, vol, mx, my, mz);
         if (status == 1) return 1;
     }
+    int nf = 0, nrow = 0;
     if (status == 0) {
-        const bool poly = A.has_poly;
-        const PolyRel pr(A.poly, c0x, c0y, c0z);
-#pragma unroll
-        for (int r = 0; r < FPL; ++r) {
-            const int f = lane + 32 * r;
-            const int n = C.nv[r];
-            rmine[r] = false;
-            nmine[r] = n > 0;
-            rval[r] = 0;
-            if (n < 3) continue;
-            const double na = sqrt(C.ax[r] * C.ax[r] + C.ay[r] * C.ay[r] + C.az[r] * C.az[r]);
-            if (A.img) {
-                // integrated voxel by voxel above
-                if (C.fid[r] >= 0) {
-                    const double bd = 0.5 * A.coeff * img_area[r] / na;
-                    rmine[r] = true;
-                    rval[r] = -bd;
+        nf = list_faces(C, W, nr);
+        if (nf < 0) status = 2;
+    }
+    bool ok = true;  // the rows fit the side buffer
+    if (status == 0) {
+        for (int k0 = 0; k0 < nf; k0 += 32)
+            nrow += __popc(__ballot_sync(FULL, k0 + lane < nf && C.pid[W.list[min(k0 + lane, nf - 1)]] >= 0));
+        RowPut row(A.rows, s, nrow + 1), nbr(A.nb, s, nf);
+        ok = row.ok && nbr.ok;
+        bool closed = true;
+        int at = 0;
+        for (int k0 = 0; k0 < nf; k0 += 32) {
+            const int k = k0 + lane;
+            const bool has = k < nf;
+            const int f = has ? W.list[k] : 0;
+            const int id = has ? C.pid[f] : -1;
+            const unsigned rm = __ballot_sync(FULL, id >= 0);
+            if (has) {
+                const double qa = C.plane[f][0], qc = C.plane[f][1], qd = C.plane[f][2];
+                const double na = sqrt(qa * qa + qc * qc + qd * qd);
+                const double ux = qa / na, uy = qc / na, uz = qd / na;
+                const double h = C.plane[f][3] / na;  // signed distance of the face plane from c0
+                double area = 0;
+                if (DENS == D_IMAGE) {
+                    area = wa[f];  // integrated voxel by voxel above
+                } else if (DENS == D_POLY) {
+                    const PolyRel pr(A.poly, c0x, c0y, c0z);
+                    double pm = 0, pdx = 0, pdy = 0, pdz = 0;  // density-weighted
+                    closed &= walk_face(C, W, f, [&](double x0, double y0, double z0, double e1x, double e1y, double e1z,
+                                                     double e2x, double e2y, double e2z) {
+                        const double ta = 0.5 * ((e1y * e2z - e1z * e2y) * ux + (e1z * e2x - e1x * e2z) * uy +
+                                                 (e1x * e2y - e1y * e2x) * uz);
+                        pr.triangle(x0, y0, z0, e1x, e1y, e1z, e2x, e2y, e2z, ta, pm, pdx, pdy, pdz, area);
+                    });
+                    vol += h * pm;
+                    mx += h * pdx;
+                    my += h * pdy;
+                    mz += h * pdz;
+                } else {
+                    double fx = 0, fy = 0, fz = 0;
+                    closed &= face_area(C, W, f, ux, uy, uz, area, fx, fy, fz);
+                    add_pyramid(h, area, fx, fy, fz, vol, mx, my, mz);
+                }
+                if (id >= 0) {
+                    const double bd = 0.5 * A.coeff * area / na;  // |x_i - x_j| = |a|
+                    row.put(at + __popc(rm & ((1u << lane) - 1u)), id, -bd);
                     der0 += bd;
                 }
-                continue;
+                nbr.put(k, id, 0.0);
             }
-            const double ux = C.ax[r] / na, uy = C.ay[r] / na, uz = C.az[r] / na;
-            const int i0 = C.F.at(0, f);
-            const double x0 = C.F.X[i0], y0 = C.F.Y[i0], z0 = C.F.Z[i0];
-            double area = 0, fx = 0, fy = 0, fz = 0;
-            double pm = 0, pdx = 0, pdy = 0, pdz = 0, pf = 0;  // density-weighted (poly)
-            for (int k = 1; k + 1 < n; ++k) {
-                const int i1 = C.F.at(k, f), i2 = C.F.at(k + 1, f);
-                const double e1x = C.F.X[i1] - x0, e1y = C.F.Y[i1] - y0, e1z = C.F.Z[i1] - z0;
-                const double e2x = C.F.X[i2] - x0, e2y = C.F.Y[i2] - y0, e2z = C.F.Z[i2] - z0;
-                const double ta = 0.5 * ((e1y * e2z - e1z * e2y) * ux + (e1z * e2x - e1x * e2z) * uy +
-                                         (e1x * e2y - e1y * e2x) * uz);
-                if (poly) {
-                    pr.triangle(x0, y0, z0, e1x, e1y, e1z, e2x, e2y, e2z, ta, pm, pdx, pdy, pdz, pf);
-                } else {
-                    area += ta;
-                    fx += ta * (3 * x0 + e1x + e2x);
-                    fy += ta * (3 * y0 + e1y + e2y);
-                    fz += ta * (3 * z0 + e1z + e2z);
-                }
-            }
-            const double h = C.b[r] / na;  // signed distance of the face plane from c0
-            if (poly) {
-                vol += h * pm;
-                mx += h * pdx;
-                my += h * pdy;
-                mz += h * pdz;
-                area = pf;  // the face's density integral
-            } else {
-                const double v = h * area / 3;
-                vol += v;
-                // pyramid centroid: 3/4 of the way from the apex to the face centroid
-                if (area != 0) {
-                    const double k = v * 0.75 / (3 * area);
-                    mx += k * fx;
-                    my += k * fy;
-                    mz += k * fz;
-                }
-            }
-            if (C.fid[r] >= 0) {
-                const double bd = 0.5 * A.coeff * area / na;  // |x_i - x_j| = |a|
-                rmine[r] = true;
-                rval[r] = -bd;
-                der0 += bd;
-            }
+            at += __popc(rm);
         }
+        if (!__all_sync(FULL, closed)) status = 2;
         for (int o = 16; o > 0; o >>= 1) {
             vol += __shfl_xor_sync(FULL, vol, o);
             mx += __shfl_xor_sync(FULL, mx, o);
@@ -746,184 +775,147 @@ __device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<FP
             mz += __shfl_xor_sync(FULL, mz, o);
             der0 += __shfl_xor_sync(FULL, der0, o);
         }
-        // positions of the row and neighbour entries: slot order
-        const unsigned below = (1u << lane) - 1u;
-#pragma unroll
-        for (int r = 0; r < FPL; ++r) {
-            const unsigned rm = __ballot_sync(FULL, rmine[r]), nm = __ballot_sync(FULL, nmine[r]);
-            rpos[r] = nrow + __popc(rm & below);
-            npos[r] = nnb + __popc(nm & below);
-            nrow += __popc(rm);
-            nnb += __popc(nm);
-        }
-    }
-    bool ok = true;  // the rows fit the side buffer
-    if (status == 0 && A.hint) {
-        // the smallest pass that holds this polyhedron (faces, vertices per face)
-        int faces = 0, maxv = 0;
-#pragma unroll
-        for (int r = 0; r < FPL; ++r) {
-            faces += __popc(__ballot_sync(FULL, C.nv[r] > 0));
-            maxv = max(maxv, C.nv[r]);
-        }
-        for (int o = 16; o > 0; o >>= 1) maxv = max(maxv, __shfl_xor_sync(FULL, maxv, o));
-        const int level = (faces <= 32 && maxv <= 16) ? 0 : (faces <= 64 && maxv <= 32) ? 1
-                          : (faces <= 128 && maxv <= 64) ? 2 : 3;
-        // polyhedra grow larger during the build than at its end, so the
-        // hint is the pass that held this build, lowered by one level at most
-        // when the final polyhedron is smaller (a cell that then overflows
-        // simply moves on to the next pass again)
-        constexpr int pass = FPL == 1 ? 0 : FPL == 2 ? 1 : FPL == 4 ? 2 : 3;
-        const int hint = level >= pass ? pass : pass - 1;
-        if (lane == 0) A.hint[s] = (unsigned char)hint;
-    }
-    if (status == 0) {
-        const double mass = A.coeff * vol;
-        if (lane == 0) {
-            if (A.mass) A.mass[s] = mass;
+        if (status == 0 && ok && lane == 0) {
+            row.put(nrow, int(s), der0);
+            row.finish();
+            nbr.finish();
+            if (A.mass) A.mass[s] = A.coeff * vol;
             if (A.ctd) {
                 const bool empty = vol == 0;
                 A.ctd[3 * s] = empty ? 0.0 : c0x + mx / vol;
                 A.ctd[3 * s + 1] = empty ? 0.0 : c0y + my / vol;
                 A.ctd[3 * s + 2] = empty ? 0.0 : c0z + mz / vol;
             }
+            if (A.hint) {
+                // polyhedra grow larger during the build than at its end, so
+                // the hint is the pass that held this build, lowered by one
+                // level at most when the final polyhedron is much smaller (a
+                // cell that then overflows moves on to the next pass again)
+                const int level = 2 * nf - 4 <= 40 ? 0 : 2 * nf - 4 <= 128 ? 1 : 2;
+                A.hint[s] = (unsigned char)(level >= PASS ? PASS : PASS - 1);
+            }
         }
-        if (A.rows.cnt) ok &= write_row<FPL>(A.rows, s, nrow + 1, rpos, rmine, C.fid, rval, true, int(s), der0);
-        if (A.nb.cnt) ok &= write_row<FPL>(A.nb, s, nnb, npos, nmine, C.fid, rval, false, 0, 0.0);
-        ok = __all_sync(FULL, ok);
     }
     if (status == 2 || !ok) {
         if (lane == 0) {
             flag_error(A.err, status == 2 ? DE_DEGEN : DE_SIDE);
-            if (A.mass) A.mass[s] = nan("");
-            if (A.ctd) A.ctd[3 * s] = A.ctd[3 * s + 1] = A.ctd[3 * s + 2] = nan("");
-            if (A.rows.cnt) {
-                A.rows.cnt[s] = 1;
-                A.rows.col[s] = int(s);
-                A.rows.val[s] = 0.0;
-            }
-            if (A.nb.cnt) A.nb.cnt[s] = 0;
+            fail_cell(A, s);
         }
         return 2;
     }
     return 0;
 }
 
-// The faces of a warp live in shared memory, or, for the largest capacity,
-// in global scratch (gscratch != null: WB bytes per warp).
-// Launch shapes of the passes: the first runs two warps per block (seven
-// blocks per SM, bounded by shared memory), the others one warp per block
-// (three per SM for the second pass, eight for the global-scratch passes);
-// the bounds let the compiler use every register those counts leave (128 in
-// the first pass, up to 255 in the others, which then spill little or not at
-// all: 8.7% faster on the 200k 3D mix, 3% on the largest serving request,
-// than the compiler's own choice under a bound of 64 threads alone).
-constexpr int k3_threads(int fpl) { return fpl == 1 ? 64 : 32; }
-constexpr int k3_min_blocks(int fpl) { return fpl == 1 ? 7 : fpl == 2 ? 3 : 8; }
+// Shared memory of one warp of a pass: the cell, its working space and, for
+// voxel images, the copy of the cell and the weighted areas.
+template <int VB, int MAXP, int DENS>
+constexpr size_t warp_smem_bytes() {
+    const size_t b = sizeof(Cell3<VB, MAXP>) + sizeof(Work3<VB, MAXP>) +
+                     (DENS == D_IMAGE ? sizeof(Cell3<VB, MAXP>) + MAXP * sizeof(double) : 0);
+    return (b + 15) / 16 * 16;
+}
 
-template <int FPL, int MAXV>
-__global__ void __launch_bounds__(k3_threads(FPL), k3_min_blocks(FPL)) k_cells3d(const Cell3DArgs A, const int *list, const int *list_cnt,
-                                                int *next_list, int *next_cnt, int nwarps, char *gscratch) {
+// The passes.  The first takes every cell, with room for 64 vertices (a
+// uniform cell has 27, and about 36 at most while it is built).  Cells that
+// outgrow it run again with 192 vertices and 128 faces, then with 640 vertices
+// and 256 faces (508 vertices): every pass in shared memory.
+//
+// Bound by instruction issue (62% of the cycles, 22 of 32 lanes active; 28
+// effective cuts, 50 others and 98 box tests per uniform cell) and by the
+// latency of FP64 and shared memory between them, so the first pass takes the
+// occupancy of 80 registers (12 blocks; 8, 10, 14, 16 blocks of the
+// multilinear kernel: 14.9, 11.6, 10.0, 9.9 ms at 96 registers and more spills
+// for the last two; 10 to 16 are within 5% at constant density).  Measured
+// against the faces held as polygons, four passes, the last two in global
+// memory: 200,000 Diracs of the 3D mix 30.9 -> 10.2 ms, 20,000 clustered ones
+// 13.1 -> 2.8 ms, whole evaluations 31.7 -> 11.0 and 13.9 -> 3.5 ms.
+struct Pass0 { static constexpr int VB = 2, MAXP = 64, WARPS = 2, BLOCKS = 12, POLY_BLOCKS = 16; };
+struct Pass1 { static constexpr int VB = 6, MAXP = 128, WARPS = 1, BLOCKS = 14, POLY_BLOCKS = 10; };
+struct Pass2 { static constexpr int VB = 20, MAXP = 256, WARPS = 1, BLOCKS = 5, POLY_BLOCKS = 5; };
+
+template <class P, int PASS, int DENS>
+__global__ void __launch_bounds__(32 * P::WARPS, DENS == D_IMAGE ? 1 : DENS == D_POLY ? P::POLY_BLOCKS : P::BLOCKS)
+    k_cells3d(const Cell3DArgs A, const int *list, const int *list_cnt, int *next_list, int *next_cnt) {
     extern __shared__ double smem3[];
-    constexpr int MAXF = 32 * FPL;
-    constexpr size_t WB = warp_smem_bytes<FPL, MAXV>();
+    constexpr int VB = P::VB, MAXP = P::MAXP;
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gw = blockIdx.x * (blockDim.x >> 5) + wib;
-    char *base = gscratch ? gscratch + WB * size_t(gw) : reinterpret_cast<char *>(smem3) + WB * wib;
-    Cell3<FPL, MAXV> C;
-    C.F.X = reinterpret_cast<double *>(base);
-    C.F.Y = C.F.X + MAXV * MAXF;
-    C.F.Z = C.F.Y + MAXV * MAXF;
-    C.F.E = reinterpret_cast<int *>(C.F.Z + MAXV * MAXF);
-    C.stack = C.F.E + MAXV * MAXF;
+    const int gw = blockIdx.x * P::WARPS + wib;
+    char *base = reinterpret_cast<char *>(smem3) + warp_smem_bytes<VB, MAXP, DENS>() * wib;
+    using C3 = Cell3<VB, MAXP>;
+    using W3 = Work3<VB, MAXP>;
+    C3 &C = *reinterpret_cast<C3 *>(base);
+    W3 &W = *reinterpret_cast<W3 *>(base + sizeof(C3));
+    C3 *B = reinterpret_cast<C3 *>(base + sizeof(C3) + sizeof(W3));
+    double *wa = reinterpret_cast<double *>(base + 2 * sizeof(C3) + sizeof(W3));
     const long long cnt = list ? *list_cnt : A.n;
+    const int nwarps = gridDim.x * P::WARPS;
     for (long long i = gw; i < cnt; i += nwarps) {
         const long long s = list ? list[i] : i;
-        if (!list && A.use_hint && A.hint) {
+        if (PASS == 0 && A.use_hint && A.hint) {
             // a cell that needed a larger pass last time goes straight there
             const int h = A.hint[s];
-            int *to = h == 1 ? next_list : h == 2 ? A.ovf_list2 : h == 3 ? A.ovf_list3 : nullptr;
-            int *tc = h == 1 ? next_cnt : h == 2 ? A.ovf_cnt2 : h == 3 ? A.ovf_cnt3 : nullptr;
-            if (to && tc) {
-                if (lane == 0) to[atomicAdd(tc, 1)] = int(s);
-                __syncwarp();
+            if (h == 1 || h == 2) {
+                if (lane == 0) {
+                    if (h == 1)
+                        next_list[atomicAdd(next_cnt, 1)] = int(s);
+                    else
+                        A.ovf_list2[atomicAdd(A.ovf_cnt2, 1)] = int(s);
+                }
                 continue;
             }
         }
-        const int r = cell3d<FPL, MAXV>(A, s, C, A.img_backup ? A.img_backup + WB * size_t(gw) : nullptr);
-        if (r == 1) {
+        const int r = cell3d<VB, MAXP, DENS, PASS>(A, s, C, W, B, wa);
+        if (r == 1 && lane == 0) {
             if (next_list) {
-                if (lane == 0) next_list[atomicAdd(next_cnt, 1)] = int(s);
-            } else if (lane == 0) {
+                next_list[atomicAdd(next_cnt, 1)] = int(s);
+            } else {
                 flag_error(A.err, DE_CAPACITY);
-                if (A.mass) A.mass[s] = nan("");
-                if (A.ctd) A.ctd[3 * s] = A.ctd[3 * s + 1] = A.ctd[3 * s + 2] = nan("");
-                if (A.rows.cnt) {
-                    A.rows.cnt[s] = 1;
-                    A.rows.col[s] = int(s);
-                    A.rows.val[s] = 0.0;
-                }
-                if (A.nb.cnt) A.nb.cnt[s] = 0;
+                fail_cell(A, s);
             }
         }
         __syncwarp();
     }
 }
 
-template <int FPL, int MAXV, int WPB>
-void launch3(const Cell3DArgs &a, const int *list, const int *list_cnt, int *next_list, int *next_cnt, long long ncells,
-             char *gscratch, long long max_blocks, cudaStream_t st) {
-    const size_t smem = gscratch ? 0 : warp_smem_bytes<FPL, MAXV>() * WPB;
+template <class P, int PASS, int DENS>
+void launch3(const Cell3DArgs &a, const int *list, const int *list_cnt, int *next_list, int *next_cnt, long long blocks,
+             cudaStream_t st) {
+    const size_t smem = warp_smem_bytes<P::VB, P::MAXP, DENS>() * P::WARPS;
     static PerDevice<int> attr;
-    if (!gscratch)
-        attr.once([&] {
-            SDOT_CUDA(cudaFuncSetAttribute(k_cells3d<FPL, MAXV>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        });
-    long long blocks = (ncells + WPB - 1) / WPB;
-    if (blocks > max_blocks) blocks = max_blocks;
-    if (blocks < 1) blocks = 1;
-    k_cells3d<FPL, MAXV><<<int(blocks), 32 * WPB, smem, st>>>(a, list, list_cnt, next_list, next_cnt,
-                                                               int(blocks) * WPB, gscratch);
+    attr.once([&] {
+        SDOT_CUDA(cudaFuncSetAttribute(k_cells3d<P, PASS, DENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    });
+    k_cells3d<P, PASS, DENS><<<int(blocks), 32 * P::WARPS, smem, st>>>(a, list, list_cnt, next_list, next_cnt);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
 }
 
-// warps of the third and fourth passes (faces in global memory, 230 KB and
-// 918 KB per warp; the two passes share the scratch, 1.09 GB): 8 per SM,
-// the most that the fourth pass's registers let an SM hold
-constexpr long long G3_WARPS = 148 * 8;
+template <int DENS>
+void launch_passes(const Cell3DArgs &a, cudaStream_t st) {
+    // one block per two cells: the hardware hands them out as blocks end
+    launch3<Pass0, 0, DENS>(a, nullptr, nullptr, a.ovf_list, a.ovf_cnt, (a.n + Pass0::WARPS - 1) / Pass0::WARPS, st);
+    // the larger passes take the overflow lists (their lengths are on the
+    // device): as many blocks as fit the device, or one per cell
+    launch3<Pass1, 1, DENS>(a, a.ovf_list, a.ovf_cnt, a.ovf_list2, a.ovf_cnt2,
+                            std::min<long long>(a.n, 148LL * Pass1::BLOCKS), st);
+    launch3<Pass2, 2, DENS>(a, a.ovf_list2, a.ovf_cnt2, nullptr, nullptr, std::min<long long>(a.n, 148LL * Pass2::BLOCKS),
+                            st);
+}
 
 }  // namespace
 
-constexpr long long G4_WARPS = 148 * 8;
-size_t cells3d_scratch_bytes() {
-    const size_t a = warp_smem_bytes<4, 64>() * G3_WARPS, b = warp_smem_bytes<8, 128>() * G4_WARPS;
-    return (a > b ? a : b) + 256;
-}
-
-size_t cells3d_image_backup_bytes() {
-    // the most warps of any pass times its face storage
-    const size_t p1 = warp_smem_bytes<1, 16>() * 148 * 7 * 2, p2 = warp_smem_bytes<2, 32>() * 148 * 3;
-    const size_t p3 = warp_smem_bytes<4, 64>() * G3_WARPS, p4 = warp_smem_bytes<8, 128>() * G4_WARPS;
-    return std::max(std::max(p1, p2), std::max(p3, p4)) + 256;
-}
-
-void cells3d_launch(const Cell3DArgs &a, void *scratch, cudaStream_t st) {
+void cells3d_launch(const Cell3DArgs &a, cudaStream_t st) {
     if (a.n == 0) return;
     SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt, 0, sizeof(int), st));
     SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt2, 0, sizeof(int), st));
-    SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt3, 0, sizeof(int), st));
     if (a.rows.side_used) SDOT_CUDA(cudaMemsetAsync(a.rows.side_used, 0, sizeof(unsigned long long), st));
     if (a.nb.side_used) SDOT_CUDA(cudaMemsetAsync(a.nb.side_used, 0, sizeof(unsigned long long), st));
-    launch3<1, 16, 2>(a, nullptr, nullptr, a.ovf_list, a.ovf_cnt, a.n, nullptr, 148LL * 7, st);
-    // the larger passes take the overflow lists (their lengths are on the
-    // device: every warp of the launch reads them)
-    launch3<2, 32, 1>(a, a.ovf_list, a.ovf_cnt, a.ovf_list2, a.ovf_cnt2, 148LL * 3, nullptr, 148LL * 3, st);
-    // passes 3 and 4 share the scratch, one after the other
-    launch3<4, 64, 1>(a, a.ovf_list2, a.ovf_cnt2, a.ovf_list3, a.ovf_cnt3, G3_WARPS, static_cast<char *>(scratch),
-                      G3_WARPS, st);
-    launch3<8, 128, 1>(a, a.ovf_list3, a.ovf_cnt3, nullptr, nullptr, G4_WARPS, static_cast<char *>(scratch), G4_WARPS,
-                       st);
+    if (a.img)
+        launch_passes<D_IMAGE>(a, st);
+    else if (a.has_poly)
+        launch_passes<D_POLY>(a, st);
+    else
+        launch_passes<D_CONST>(a, st);
 }
 
 }  // namespace sdot

@@ -28,11 +28,9 @@ struct Cell3DArgs {
     // piecewise-constant voxel image (ScaledImage, nb_coeffs = 1): nx x ny x nz
     // values, x fastest, over [img_lo, img_hi]; each cell is integrated voxel
     // by voxel (the density of a piece is the voxel's value times coeff).
-    // img_backup: per warp a copy of the faces (img_backup_bytes per warp).
     const double *img = nullptr;
     int img_n[3] = {0, 0, 0};
     double img_lo[3] = {0, 0, 0}, img_hi[3] = {1, 1, 1};
-    char *img_backup = nullptr;
     // optional multilinear density factor (has_poly): coeff * (p0 + p1 x +
     // p2 y + p3 z + p4 xy + p5 xz + p6 yz + p7 xyz), absolute coordinates
     int has_poly = 0;
@@ -45,9 +43,7 @@ struct Cell3DArgs {
     int *ovf_cnt = nullptr;
     int *ovf_list2 = nullptr;  // cells handed to the third pass
     int *ovf_cnt2 = nullptr;
-    int *ovf_list3 = nullptr;  // cells handed to the fourth pass
-    int *ovf_cnt3 = nullptr;
-    // per cell (sorted order): the pass (0..3) its last build needed; with
+    // per cell (sorted order): the pass (0..2) its last build needed; with
     // use_hint the first pass sends each cell straight to that pass (the
     // positions, hence the tree order, must not have changed)
     unsigned char *hint = nullptr;
@@ -56,13 +52,9 @@ struct Cell3DArgs {
     int *guard = nullptr;
 };
 
-// First pass over every cell (up to 32 faces of 16 vertices, shared memory),
-// then the cells that overflowed it (64 faces of 32 vertices, shared memory),
-// then those that overflowed again (128 faces of 64 vertices, then 256 faces
-// of 128 vertices, both in `scratch` of cells3d_scratch_bytes() bytes).
-size_t cells3d_scratch_bytes();
-// Bytes of the per-warp face copies of the voxel-image mode (all passes).
-size_t cells3d_image_backup_bytes();
-void cells3d_launch(const Cell3DArgs &a, void *scratch, cudaStream_t st);
+// First pass over every cell (up to 64 vertices), then the cells that
+// overflowed it (192 vertices, 128 faces), then those that overflowed again
+// (640 vertices, 256 faces); the cells live in shared memory.
+void cells3d_launch(const Cell3DArgs &a, cudaStream_t st);
 
 }  // namespace sdot
