@@ -45,8 +45,8 @@ struct Request {
 
 // Device memory a request needs beyond its worker's fixed buffers: Diracs,
 // tree, cell outputs, Hessian rows (ELL) and solver vectors, per Dirac.
-int64_t request_bytes(int dim, int64_t n) { return n * (dim == 3 ? 1400 : 800) + (1 << 20); }
-constexpr int64_t HIGH_PRIORITY_BYTES = int64_t(64) << 20;  // 3D from ~47k Diracs, 2D from ~83k
+int64_t request_bytes(int dim, int64_t n) { return n * (dim == 3 ? 1650 : 950) + (1 << 20); }
+constexpr int64_t HIGH_PRIORITY_BYTES = int64_t(75) << 20;  // 3D from ~47k Diracs, 2D from ~83k
 
 }  // namespace
 

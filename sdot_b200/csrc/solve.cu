@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace sdot {
 
@@ -15,6 +16,7 @@ namespace {
 
 constexpr int TB = 256;
 enum { S_RZ = 0, S_RR = 1, S_RR0 = 2, S_PQ = 3, S_ALPHA = 4, S_BETA = 5, S_GDIAG = 6, S_BAD = 7, S_NSCAL = 8 };
+constexpr int S_ITER = S_PQ;  // the multilevel solve keeps p . q in registers and its iteration count here
 
 __device__ double block_sum(double v, double *sh) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -28,6 +30,44 @@ __device__ double block_sum(double v, double *sh) {
     }
     __syncthreads();
     return r;  // valid in thread 0
+}
+
+// sum_k val_k f(col_k) over an ELL row, in order.  U entries are read at once,
+// so that their latencies overlap (entry by entry a row is a chain of m loads
+// of the column and then of the vector); the first U slots (the row has at
+// least U, used or not) without waiting for the row's length.
+template <int U, class V, class F>
+__device__ __forceinline__ double ell_sum(const V *val, const int *col, long long stride, long long s, const int *cnt,
+                                          int m, const F &f) {
+    double acc = 0;
+    int c[U];
+    V v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (cnt || u < m) {
+            c[u] = col[u * stride + s];
+            v[u] = val[u * stride + s];
+        }
+    if (cnt) m = cnt[s];
+#pragma unroll 1
+    for (int k0 = 0; k0 < m; k0 += U) {
+        if (k0 > 0) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k0 + u < m) {
+                    c[u] = col[(k0 + u) * stride + s];
+                    v[u] = val[(k0 + u) * stride + s];
+                }
+        }
+        double x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k0 + u < m) x[u] = f(c[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k0 + u < m) acc += double(v[u]) * x[u];
+    }
+    return acc;
 }
 
 // Matrix views for the PCG kernels: row s times x, and the diagonal entry
@@ -66,14 +106,9 @@ struct RowsMatT {
     template <class F>
     __device__ double row_sum(long long s, const F &f) const {
         const int m = R.cnt[s];
-        double acc = 0;
-        if (m <= R.cap) {
-            for (int k = 0; k < m; ++k) acc += double(val[k * R.stride + s]) * f(R.col[k * R.stride + s]);
-        } else {
-            const long long o = R.side[s];
-            for (int k = 0; k < m; ++k) acc += double(side_val[o + k]) * f(R.side_col[o + k]);
-        }
-        return acc;
+        if (m <= R.cap) return ell_sum<4>(val, R.col, R.stride, s, R.cnt, m, f);
+        const long long o = R.side[s];
+        return ell_sum<2>(side_val + o, R.side_col + o, 1, 0, nullptr, m, f);
     }
 };
 using RowsMat = RowsMatT<double>;
@@ -145,17 +180,30 @@ struct CsrView {
 };
 
 // ---- multilevel preconditioner (one V-cycle per application) ------------
-// Aggregates: MG_B consecutive rows (the rows are in Morton order, so an
-// aggregate is a compact patch of cells).  Coarse matrices P^T A P with P
-// piecewise constant on the aggregates, stored as ELL (width MG_CAP);
-// damped-Jacobi smoothing (MG_OMEGA) before and after the coarse
-// correction; the coarsest level (<= MG_COARSE rows) is applied as its dense
-// inverse.  Same smoother on both sides and an exact coarsest solve: the
-// cycle is a symmetric positive operator, a valid CG preconditioner.
-constexpr int MG_B = 8;
+// Aggregates: consecutive rows (the rows are in Morton order, so an aggregate
+// is a compact patch of cells), 4 of the finest level, MG_B of the others.
+// Coarse matrices P^T A P / MG_SCALE with P piecewise constant on the
+// aggregates, stored as ELL (width mg_cap); damped-Jacobi smoothing (MG_OMEGA)
+// before and after the coarse correction; the coarsest level (<= MG_COARSE
+// rows) is applied as its dense inverse.  Same smoother on both sides and
+// symmetric coarse operators: the cycle is a symmetric positive operator (the
+// smoother converges for MG_OMEGA < 1, the matrices being weighted graph
+// Laplacians plus a diagonal), a valid CG preconditioner.
+//
+// Piecewise constant P makes the coarse matrices too stiff for smooth errors
+// (over-correction: D. Braess, "Towards algebraic multigrid for elliptic
+// problems of second order", Computing 55, 1995); 1.4 is the best of 1 to 2.2
+// with 0.8 of 0.67 to 0.9.  CG iterations to 1e-12 on Voronoi Laplacians,
+// 10,000 uniform / 30,000 clustered / 8,000 3D points: aggregates of 8, omega
+// 0.67, no scaling 135 / 195 / 59; omega 0.8 and 1.4: 113 / 149 / 51; 4 at the
+// finest level: 99 / 136 / 45; 4 at every level: 87 / 110 / 41, but twice the
+// levels, each with two barriers of the grid.
+constexpr int MG_BF = 4;         // rows of an aggregate of the finest level
+constexpr int MG_B = 8;          // and of the coarse levels
 constexpr int MG_CAP_MAX = 128;  // coarse ELL width: w.mg_cap (64 in 2D, 128 in 3D)
 constexpr int MG_COARSE = 48;  // dense coarsest level: two 48 x 49 doubles in shared memory
-constexpr double MG_OMEGA = 0.67;
+constexpr double MG_OMEGA = 0.8;
+constexpr double MG_SCALE = 1.4;
 
 template <class V>
 struct EllViewT {
@@ -168,9 +216,7 @@ struct EllViewT {
     __device__ double valk(long long s, int k) const { return double(val[k * stride + s]); }
     template <class F>
     __device__ double row_sum(long long s, const F &f) const {
-        double acc = 0;
-        for (int k = 0, m = cnt[s]; k < m; ++k) acc += double(val[k * stride + s]) * f(col[k * stride + s]);
-        return acc;
+        return ell_sum<4>(val, col, stride, s, cnt, 0, f);
     }
 };
 
@@ -348,12 +394,12 @@ __global__ void k_gather_sorted(const double *t, const int *idx, double *out, lo
         out[s] = t[idx[s]];
 }
 
-// One warp per coarse row c: the entries of fine rows c*MG_B .. c*MG_B+7, in
+// One warp per coarse row c: the entries of fine rows c*B .. c*B+B-1, in
 // row order then stored order, are merged by coarse column into a table of
 // 32 SLOTS entries (SLOTS per lane), so the sums have a fixed order.  The
 // gauge term of the fine level joins the coarse diagonal.  A row with more
 // than 32 SLOTS coarse columns sets *flag (the solve falls back to Jacobi).
-template <class M, int SLOTS, class T>
+template <class M, int SLOTS, int B, class T>
 __global__ void k_mg_coarsen(M A, long long nf, long long gauge, const double *scal, MgLevelT<T> out, int *flag) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -393,11 +439,11 @@ __global__ void k_mg_coarsen(M A, long long nf, long long gauge, const double *s
                 over = true;
             }
         };
-        for (int r = 0; r < MG_B; ++r) {
-            const long long s = c * MG_B + r;
+        for (int r = 0; r < B; ++r) {
+            const long long s = c * B + r;
             if (s >= nf) break;
             const int len = A.len(s);
-            for (int k = 0; k < len; ++k) insert(int(A.colk(s, k) / MG_B), A.valk(s, k));
+            for (int k = 0; k < len; ++k) insert(int(A.colk(s, k) / B), A.valk(s, k));
             if (s == gauge) insert(int(c), scal[S_GDIAG]);
         }
         double diag = 0;
@@ -405,6 +451,7 @@ __global__ void k_mg_coarsen(M A, long long nf, long long gauge, const double *s
         for (int q = 0; q < SLOTS; ++q)
             if (lane + 32 * q < count) {
                 out.col[(lane + 32 * q) * out.n + c] = key[q];
+                v[q] *= 1.0 / MG_SCALE;
                 out.val[(lane + 32 * q) * out.n + c] = T(v[q]);
                 if (key[q] == c) diag = v[q];
             }
@@ -413,116 +460,6 @@ __global__ void k_mg_coarsen(M A, long long nf, long long gauge, const double *s
             out.cnt[c] = count;
             out.dinv[c] = T(diag > 0 ? 1.0 / diag : 0.0);
             if (over) atomicExch(flag, 1);
-        }
-    }
-}
-
-// Pre-smoothing and restriction of one level: z = w D^-1 r, and
-// rc[aggregate] = sum over its rows of (r - A z).  Rows are taken a block at a
-// time so that the MG_B rows of an aggregate sit in consecutive lanes.
-template <class M, class T, class TC>
-__global__ void k_mg_pre(M A, long long n, long long gauge, const double *scal, const T *dinv, const T *r, T *z,
-                         TC *rc) {
-    const unsigned FULL = 0xffffffffu;
-    for (long long i0 = blockIdx.x * (long long)blockDim.x; i0 < n; i0 += (long long)gridDim.x * blockDim.x) {
-        const long long i = i0 + threadIdx.x;
-        double t = 0;
-        if (i < n) {
-            const double ri = double(r[i]);
-            const double zi = MG_OMEGA * double(dinv[i]) * ri;
-            z[i] = T(zi);
-            double acc = A.row_sum(i, [&](long long j) { return MG_OMEGA * double(dinv[j]) * double(r[j]); });
-            if (i == gauge) acc += scal[S_GDIAG] * zi;
-            t = ri - acc;
-        }
-        for (int o = MG_B / 2; o > 0; o >>= 1) t += __shfl_down_sync(FULL, t, o, MG_B);
-        if ((threadIdx.x & (MG_B - 1)) == 0 && i < n) rc[i / MG_B] = TC(t);
-    }
-}
-
-// Coarse correction and post-smoothing: z' = z + P zc, zo = z' + w D^-1 (r - A z').
-// On the finest level (FINE) it also sums r . zo per block into partial[]
-// and, when p is given, writes p = zo (the first CG direction).
-template <class M, bool FINE, class T, class TC>
-__global__ void k_mg_post(M A, long long n, long long gauge, const double *scal, const T *dinv, const T *r, const T *z,
-                          const TC *zc, T *zo, double *partial, T *p) {
-    __shared__ double sh[32];
-    double rz = 0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        auto zp = [&](long long j) { return double(z[j]) + double(zc[j / MG_B]); };
-        const double zi = zp(i);
-        double acc = A.row_sum(i, zp);
-        if (i == gauge) acc += scal[S_GDIAG] * zi;
-        const T v = T(zi + MG_OMEGA * double(dinv[i]) * (double(r[i]) - acc));
-        zo[i] = v;
-        if (FINE) {
-            rz += double(r[i]) * double(v);
-            if (p) p[i] = v;
-        }
-    }
-    if (FINE) {
-        rz = block_sum(rz, sh);
-        if (threadIdx.x == 0) partial[blockIdx.x] = rz;
-    }
-}
-
-// The same two steps on a coarse level, four lanes per row (a warp holds the
-// eight rows of one aggregate): the coarse rows are up to MG_CAP_MAX entries
-// wide and the levels small, so one thread per row left each kernel bound by
-// the latency of a long chain of dependent loads.  Each lane sums every
-// fourth entry of its row; the partial sums are combined in a fixed order.
-constexpr int CL = 4;  // lanes per coarse row
-__global__ void k_mg_pre_coarse(EllViewT<double> A, long long n, const double *dinv, const double *r, double *z,
-                                double *rc) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, sub = lane & (CL - 1);
-    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    const long long nagg = (n + MG_B - 1) / MG_B;
-    for (long long g = warp; g < nagg; g += nw) {
-        const long long i = g * MG_B + (lane >> 2);
-        // z = w D^-1 r; t = r - A z (A z from the smoothed values w D^-1 r)
-        double acc = 0, ri = 0;
-        if (i < n) {
-            ri = r[i];
-            if (sub == 0) z[i] = MG_OMEGA * dinv[i] * ri;
-            const int m = A.cnt[i];
-            for (int k = sub; k < m; k += CL) {
-                const long long c = A.col[k * A.stride + i];
-                acc += A.val[k * A.stride + i] * (MG_OMEGA * dinv[c] * r[c]);
-            }
-        }
-        acc += __shfl_xor_sync(FULL, acc, 1);
-        acc += __shfl_xor_sync(FULL, acc, 2);
-        double t = i < n && sub == 0 ? ri - acc : 0.0;
-        // the aggregate's residual: the rows in order (lanes 0, 4, ..., 28)
-        for (int o = 4; o < 32; o <<= 1) t += __shfl_xor_sync(FULL, t, o);
-        if (lane == 0) rc[g] = t;
-    }
-}
-
-__global__ void k_mg_post_coarse(EllViewT<double> A, long long n, const double *dinv, const double *r, const double *z,
-                                 const double *zc, double *zo) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, sub = lane & (CL - 1);
-    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    const long long nrow = (n + 7) / 8 * 8;
-    for (long long i0 = warp * 8; i0 < nrow; i0 += nw * 8) {
-        const long long i = i0 + (lane >> 2);
-        double acc = 0;
-        if (i < n) {
-            const int m = A.cnt[i];
-            for (int k = sub; k < m; k += CL) {
-                const long long c = A.col[k * A.stride + i];
-                acc += A.val[k * A.stride + i] * (z[c] + zc[c / MG_B]);
-            }
-        }
-        acc += __shfl_xor_sync(FULL, acc, 1);
-        acc += __shfl_xor_sync(FULL, acc, 2);
-        if (i < n && sub == 0) {
-            const double zi = z[i] + zc[i / MG_B];
-            zo[i] = zi + MG_OMEGA * dinv[i] * (r[i] - acc);
         }
     }
 }
@@ -575,45 +512,16 @@ __global__ void k_mg_coarsest_setup(EllViewT<V> A, int nc, double *cinv) {
         for (int c = 0; c < nc; ++c) cinv[t * nc + c] = I[t][c];
 }
 
+// CG start for the multilevel preconditioner: x = 0, r = b, s = omega D^-1 r;
+// the vectors of a previous iteration are zero.
 template <class T>
-__global__ void k_mg_coarsest_apply(const double *cinv, int nc, const T *r, T *zo) {
-    const int t = threadIdx.x;
-    if (t < nc) {
-        double acc = 0;
-        for (int c = 0; c < nc; ++c) acc += cinv[t * nc + c] * double(r[c]);
-        zo[t] = T(acc);
+__global__ void k_init_mg(const T *b, T *x, T *r, T *s, const T *dinv, T *p, T *q, T *qs, T *z, long long n) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const T rv = b[i];
+        x[i] = p[i] = q[i] = qs[i] = z[i] = 0;
+        r[i] = rv;
+        s[i] = T(MG_OMEGA * double(dinv[i]) * double(rv));
     }
-}
-
-// CG start and update for the multilevel preconditioner: z, p and r . z come
-// from the V-cycle (k_mg_post on the finest level).
-template <class T>
-__global__ void k_init_mg(const T *b, T *x, T *r, double *partial, long long n) {
-    __shared__ double sh[32];
-    double rr = 0;
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < n; s += (long long)gridDim.x * blockDim.x) {
-        const T rv = b[s];
-        x[s] = 0;
-        r[s] = rv;
-        rr += double(rv) * double(rv);
-    }
-    rr = block_sum(rr, sh);
-    if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = rr;
-}
-
-template <class T>
-__global__ void k_update_mg(T *x, T *r, const T *p, const T *q, const double *scal, double *partial, long long n) {
-    __shared__ double sh[32];
-    const T alpha = T(scal[S_ALPHA]);
-    double rr = 0;
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < n; s += (long long)gridDim.x * blockDim.x) {
-        x[s] += alpha * p[s];
-        const T rv = r[s] - alpha * q[s];
-        r[s] = rv;
-        rr += double(rv) * double(rv);
-    }
-    rr = block_sum(rr, sh);
-    if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = rr;
 }
 
 int grid_of(long long n) {
@@ -635,6 +543,8 @@ struct MgPlan {
     MgLevelT<double> lev[MG_MAX_LEV + 1];  // lev[0]: the fine level (n only); coarse levels in FP64
     double *cinv = nullptr;           // coarsest dense inverse
     int *flag = nullptr;              // coarse-row overflow
+    unsigned *sync = nullptr;         // the solve's grid barrier: arrivals, given up
+    T *s0 = nullptr, *s1 = nullptr, *qs = nullptr, *p1 = nullptr;  // vectors beside PcgWorkT's
 };
 
 // Carves the levels of an n-row solve out of `base` (null: sizes only);
@@ -654,13 +564,13 @@ size_t mg_plan(long long n, int cap, double *base, MgPlan<T> &pl) {
     pl.lev[0].n = n;
     long long m = n;
     while (m > MG_COARSE && pl.L < MG_MAX_LEV) {
-        m = (m + MG_B - 1) / MG_B;
+        const int ag = pl.L == 0 ? MG_BF : MG_B;
+        m = (m + ag - 1) / ag;
         MgLevelT<double> &v = pl.lev[++pl.L];
         v.n = m;
         v.val = take(size_t(cap) * m, (double *)nullptr);
         v.dinv = take(m, (double *)nullptr);
         v.r = take(m, (double *)nullptr);
-        v.z = take(m, (double *)nullptr);
         v.zo = take(m, (double *)nullptr);
         v.cnt = take(m, (int *)nullptr);
         v.col = take(size_t(cap) * m, (int *)nullptr);
@@ -668,6 +578,11 @@ size_t mg_plan(long long n, int cap, double *base, MgPlan<T> &pl) {
     if (pl.L > 0) {
         pl.cinv = take(size_t(MG_COARSE) * MG_COARSE, (double *)nullptr);
         pl.flag = take(1, (int *)nullptr);
+        pl.sync = take(2, (unsigned *)nullptr);
+        pl.s0 = take(n, (T *)nullptr);
+        pl.s1 = take(n, (T *)nullptr);
+        pl.qs = take(n, (T *)nullptr);
+        pl.p1 = take(n, (T *)nullptr);
     }
     return used;
 }
@@ -685,9 +600,9 @@ void mg_coarsen_all(const M &A, long long gauge, const double *scal, const MgPla
     for (int l = 1; l <= pl.L; ++l) {
         const int g = coarse_grid(32 * pl.lev[l].n);  // one warp per coarse row
         if (l == 1)
-            k_mg_coarsen<M, SLOTS, double><<<g, TB, 0, st>>>(A, pl.lev[0].n, gauge, scal, pl.lev[1], pl.flag);
+            k_mg_coarsen<M, SLOTS, MG_BF, double><<<g, TB, 0, st>>>(A, pl.lev[0].n, gauge, scal, pl.lev[1], pl.flag);
         else
-            k_mg_coarsen<EllViewT<double>, SLOTS, double><<<g, TB, 0, st>>>(ell(pl.lev[l - 1]), pl.lev[l - 1].n, -1, scal,
+            k_mg_coarsen<EllViewT<double>, SLOTS, MG_B, double><<<g, TB, 0, st>>>(ell(pl.lev[l - 1]), pl.lev[l - 1].n, -1, scal,
                                                                   pl.lev[l], pl.flag);
         note_launch();
     }
@@ -708,29 +623,6 @@ bool mg_setup(const M &A, long long gauge, const double *scal, const MgPlan<T> &
     SDOT_CUDA(cudaStreamSynchronize(st));
     return flag == 0;
 }
-
-// z0 = V-cycle(r0) on the finest level (pre-smoothed values in zpre0), with
-// r0 . z0 per block into partial[0 .. g) and, when p0 is given, p0 = z0.
-template <class M, class T>
-void mg_vcycle(const M &A, long long gauge, const double *scal, const T *dinv0, const MgPlan<T> &pl, const T *r0,
-               T *zpre0, T *z0, double *partial, T *p0, int g, cudaStream_t st) {
-    const long long n = pl.lev[0].n;
-    k_mg_pre<M, T, double><<<g, TB, 0, st>>>(A, n, gauge, scal, dinv0, r0, zpre0, pl.lev[1].r);
-    for (int l = 1; l < pl.L; ++l) {
-        const MgLevelT<double> &v = pl.lev[l];
-        k_mg_pre_coarse<<<coarse_grid(4 * v.n), TB, 0, st>>>(ell(v), v.n, v.dinv, v.r, v.z, pl.lev[l + 1].r);
-    }
-    const MgLevelT<double> &c = pl.lev[pl.L];
-    k_mg_coarsest_apply<double><<<1, MG_COARSE, 0, st>>>(pl.cinv, int(c.n), c.r, c.zo);
-    for (int l = pl.L - 1; l >= 1; --l) {
-        const MgLevelT<double> &v = pl.lev[l];
-        k_mg_post_coarse<<<coarse_grid(4 * v.n), TB, 0, st>>>(ell(v), v.n, v.dinv, v.r, v.z, pl.lev[l + 1].zo, v.zo);
-    }
-    k_mg_post<M, true, T, double><<<g, TB, 0, st>>>(A, n, gauge, scal, dinv0, r0, zpre0, pl.lev[1].zo, z0, partial, p0);
-}
-
-template <class T>
-int mg_launches(const MgPlan<T> &pl) { return 2 * pl.L + 1; }
 
 }  // namespace
 
@@ -756,6 +648,384 @@ template void pcg_bind<float>(PcgWorkT<float> &, double *, long long);
 
 namespace {
 
+// ---- the whole solve in one kernel -----------------------------------------
+// As launches, an iteration of multilevel CG is 13 to 16 kernels of 3 to 20 us
+// at 10,000 to 60,000 rows, most of it their latency.  Here the blocks
+// stay for up to `iters` iterations (a cooperative launch: every block is
+// resident) and meet at grid barriers:
+//   A  p = z + beta p_old; q = A p, qs = omega D^-1 q; p . q       | barrier
+//   B  x += alpha p; r -= alpha q; s = s_old - alpha qs (= omega D^-1 r);
+//      |r|^2; coarse right-hand side sum (r - A s)                 | barrier
+//   C  coarse levels above SOLO rows: one barrier a level and direction; the
+//      rest by one block, its vectors in shared memory             | barrier
+//   D  z' = s + P zc, z = z' + omega D^-1 (r - A z'); r . z        | barrier
+// The vector updates are folded into the passes over the matrix: what a row
+// needs of its neighbours' new values it computes from the old ones (hence two
+// copies of p and s).  Sums go by block partials that every block adds in one
+// order, so that all blocks take the same decisions and a solve repeats bit
+// for bit.  The barrier gives up after a bounded wait (the solve then ends as
+// not converged).
+//
+// One thread per row.  Measured per iteration (launches of the phases in a CUDA
+// graph -> this kernel): 10,000 rows 45 -> 29 us, 60,000 70 -> 45, 20,000 3D
+// rows 80 -> 51; about 2 us of each are a barrier, 1 to 4 us a phase (two
+// dependent reads of the L2 and the block's sum).  Blocks of 128, 256, 512
+// threads: 32 / 29 / 35 us and 59 / 45 / 52 us.  A hardware cluster of 16
+// blocks has a barrier of 0.7 us, but its 16 SMs take 8 us for a phase of 10,000
+// rows.  Two blocks per SM pay from several 100,000 rows on, where the passes
+// are bound by the loads in flight (Newton at 1M rows 1.79 -> 1.56 s, at
+// 200,000 0.247 -> 0.262 s).
+constexpr int MGT = 256;
+constexpr int MANY_PER_SM = 2;
+constexpr long long MANY_ROWS = 400000;
+constexpr int SOLO = 512;       // rows of the largest level one block does alone
+constexpr int SOLO_ALL = 640;   // rows of all such levels together (512 + 64 + 8, and a margin)
+
+template <class M, class T>
+struct PcgArgs {
+    M A;
+    long long n, gauge;
+    MgPlan<T> pl;
+    const T *dinv;
+    T *x, *r, *s[2], *q, *qs, *p[2], *z;
+    double *scal, *partial;
+    double rel2;  // square of the relative tolerance
+    int iters;
+    int first;    // 1: starts a solve; 0: goes on from scal
+};
+
+// Sum of the blocks' partials, the same in every thread of every block.
+__device__ double grid_sum(const double *partial, double *sh) {
+    double a = 0;
+    for (int i = threadIdx.x; i < int(gridDim.x); i += blockDim.x) a += partial[i];
+    a = block_sum(a, sh);
+    if (threadIdx.x == 0) sh[0] = a;
+    __syncthreads();
+    a = sh[0];
+    __syncthreads();
+    return a;
+}
+
+// Waits for every block of the grid; false when the wait was given up (by any
+// block).  target counts the arrivals expected so far.  The release and the
+// acquire, with the block's own barriers around them, order the plain reads and
+// writes of all threads (and drop what the L1 cache holds of other blocks').
+__device__ bool grid_barrier(unsigned *sync, unsigned &target) {
+    __shared__ int ok;
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sync[0]) : "memory");
+        ok = 0;
+        for (unsigned k = 0; k < (1u << 24); ++k) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&sync[0]) : "memory");
+            if (int(v - target) >= 0) {
+                ok = 1;
+                break;
+            }
+            if ((k & 1023u) == 1023u && *(volatile unsigned *)&sync[1]) break;
+        }
+        if (!ok) atomicExch(&sync[1], 1u);
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// r - A z of row i with z_j = f(j); the aggregate's sum of it to rc (whole
+// warps call this: rows past n give 0)
+template <int B>
+__device__ void restrict_row(double t, long long i, long long n, double *rc) {
+    for (int o = B / 2; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o, B);
+    if ((threadIdx.x & (B - 1)) == 0 && i < n) rc[i / B] = t;
+}
+
+// The phases.  Each is a function of its own: in one body the compiler keeps
+// the addresses of all of them in registers and spills inside the loops (1.6 KB
+// a thread; the barriers empty the L1 cache that would hold them).
+template <class M, class T>
+__device__ __noinline__ double phase_a(const PcgArgs<M, T> &a, const T *pold, T *pnew, double beta, double gd) {
+    const long long step = (long long)gridDim.x * MGT;
+    auto pv = [&](long long j) { return double(T(double(a.z[j]) + beta * double(pold[j]))); };
+    double pq = 0;
+    for (long long i = blockIdx.x * (long long)MGT + threadIdx.x; i < a.n; i += step) {
+        const double pi = pv(i);
+        double v = a.A.row_sum(i, pv);
+        if (i == a.gauge) v += gd * pi;
+        const T qv = T(v);
+        pnew[i] = T(pi);
+        a.q[i] = qv;
+        a.qs[i] = T(MG_OMEGA * double(a.dinv[i]) * double(qv));
+        pq += pi * double(qv);
+    }
+    return pq;
+}
+
+template <class M, class T>
+__device__ __noinline__ double phase_b(const PcgArgs<M, T> &a, const T *p, const T *sold, T *snew, double alpha,
+                                       double gd, bool update) {
+    const long long step = (long long)gridDim.x * MGT;
+    auto sv = [&](long long j) { return double(T(double(sold[j]) - alpha * double(a.qs[j]))); };
+    double rs = 0;
+    for (long long i0 = blockIdx.x * (long long)MGT; i0 < a.n; i0 += step) {
+        const long long i = i0 + threadIdx.x;
+        double t = 0;
+        if (i < a.n) {
+            T rv = a.r[i];
+            if (update) {
+                a.x[i] += T(alpha) * p[i];
+                rv = T(double(rv) - alpha * double(a.q[i]));
+                a.r[i] = rv;
+            }
+            const double si = sv(i);
+            snew[i] = T(si);
+            double v = a.A.row_sum(i, sv);
+            if (i == a.gauge) v += gd * si;
+            t = double(rv) - v;
+            rs += double(rv) * double(rv);
+        }
+        restrict_row<MG_BF>(t, i, a.n, a.pl.lev[1].r);
+    }
+    return rs;
+}
+
+template <class M, class T>
+__device__ __noinline__ double phase_d(const PcgArgs<M, T> &a, const T *s, double gd) {
+    const long long step = (long long)gridDim.x * MGT;
+    const double *zc = a.pl.lev[1].zo;
+    auto zv = [&](long long j) { return double(s[j]) + zc[j / MG_BF]; };
+    double rs = 0;
+    for (long long i = blockIdx.x * (long long)MGT + threadIdx.x; i < a.n; i += step) {
+        const double zi = zv(i), ri = double(a.r[i]);
+        double v = a.A.row_sum(i, zv);
+        if (i == a.gauge) v += gd * zi;
+        const T zo = T(zi + MG_OMEGA * double(a.dinv[i]) * (ri - v));
+        a.z[i] = zo;
+        rs += ri * double(zo);
+    }
+    return rs;
+}
+
+// Smoothing and restriction of a coarse level (right-hand side r, the sums to
+// rc), rows i0 + threadIdx.x of every step-th block of rows from i0
+__device__ __noinline__ void coarse_down(const EllViewT<double> A, int n, const double *dinv, const double *r, double *rc,
+                                         int i0, int step) {
+    for (; i0 < n; i0 += step) {
+        const int i = i0 + threadIdx.x;
+        double t = 0;
+        if (i < n) t = r[i] - A.row_sum(i, [&](long long j) { return MG_OMEGA * dinv[j] * r[j]; });
+        restrict_row<MG_B>(t, i, n, rc);
+    }
+}
+
+// Coarse correction zc and smoothing of a coarse level, into zo
+__device__ __noinline__ void coarse_up(const EllViewT<double> A, int n, const double *dinv, const double *r,
+                                       const double *zc, double *zo, int i0, int step) {
+    auto zv = [&](long long j) { return MG_OMEGA * dinv[j] * r[j] + zc[j / MG_B]; };
+    for (int i = i0 + threadIdx.x; i < n; i += step)
+        zo[i] = zv(i) + MG_OMEGA * dinv[i] * (r[i] - A.row_sum(i, zv));
+}
+
+// Levels [solo, L] by one block, their vectors in shared memory.
+struct SoloMem {
+    double r[SOLO_ALL], z[SOLO_ALL], dinv[SOLO_ALL];
+    double cinv[MG_COARSE * MG_COARSE];
+};
+template <class T>
+__device__ __noinline__ void coarse_solo(const MgPlan<T> &pl, int solo, SoloMem &S) {
+    double *sr = S.r, *sz = S.z;
+    const int tid = threadIdx.x, L = pl.L;
+    const int n0 = int(pl.lev[solo].n);
+    for (int i = tid; i < n0; i += MGT) sr[i] = pl.lev[solo].r[i];
+    __syncthreads();
+    int at = 0;
+    for (int l = solo; l < L; ++l) {
+        const MgLevelT<double> &v = pl.lev[l];
+        const double *r = sr + at, *dinv = S.dinv + at;
+        const int nl = int(v.n);
+        const EllViewT<double> A{v.cnt, v.col, v.val, v.n};
+        at += nl;
+        for (int i0 = 0; i0 < nl; i0 += MGT) {
+            const int i = i0 + tid;
+            double t = 0;
+            if (i < nl) t = r[i] - A.row_sum(i, [&](long long j) { return MG_OMEGA * dinv[j] * r[j]; });
+            restrict_row<MG_B>(t, i, nl, sr + at);
+        }
+        __syncthreads();
+    }
+    const int nc = int(pl.lev[L].n);
+    if (tid < nc) {
+        double acc = 0;
+        for (int c = 0; c < nc; ++c) acc += S.cinv[c * nc + tid] * sr[at + c];
+        sz[at + tid] = acc;
+    }
+    __syncthreads();
+    for (int l = L - 1; l >= solo; --l) {
+        const MgLevelT<double> &v = pl.lev[l];
+        const int nl = int(v.n);
+        const double *zc = sz + at;
+        at -= nl;
+        const double *r = sr + at, *dinv = S.dinv + at;
+        const EllViewT<double> A{v.cnt, v.col, v.val, v.n};
+        auto zv = [&](long long j) { return MG_OMEGA * dinv[j] * r[j] + zc[j / MG_B]; };
+        for (int i = tid; i < nl; i += MGT) sz[at + i] = zv(i) + MG_OMEGA * dinv[i] * (r[i] - A.row_sum(i, zv));
+        __syncthreads();
+    }
+    for (int i = tid; i < n0; i += MGT) pl.lev[solo].zo[i] = sz[i];
+}
+
+template <class M, class T, int PER_SM>
+__global__ void __launch_bounds__(MGT, PER_SM) k_pcg_mg(const __grid_constant__ PcgArgs<M, T> param) {
+    __shared__ double sh[33];
+    __shared__ SoloMem solo_mem;
+    // the arguments in shared memory: read through the L1 cache, which the
+    // barriers empty, each use of a pointer would wait for the L2 first
+    using Args = PcgArgs<M, T>;
+    static_assert(sizeof(Args) % 8 == 0, "copied by 8 bytes");
+    __shared__ double arg_mem[sizeof(Args) / 8];
+    for (int i = threadIdx.x; i < int(sizeof(Args) / 8); i += MGT)
+        arg_mem[i] = reinterpret_cast<const double *>(&param)[i];
+    const Args &a = *reinterpret_cast<const Args *>(arg_mem);
+    __syncthreads();
+    const int tid = threadIdx.x, L = a.pl.L, t0 = blockIdx.x * MGT, step = gridDim.x * MGT;
+    const double gd = a.gauge >= 0 ? a.scal[S_GDIAG] : 0.0;
+    double *p_pq = a.partial, *p_rr = a.partial + gridDim.x, *p_rz = a.partial + 2 * gridDim.x;
+    // the levels [solo, L] are one block's
+    int solo = L;
+    while (solo > 1 && a.pl.lev[solo - 1].n <= SOLO) --solo;
+    if (blockIdx.x == 0) {
+        const int nc = int(a.pl.lev[L].n);
+        for (int i = tid; i < nc * nc; i += MGT) solo_mem.cinv[i] = a.pl.cinv[i];
+        int at = 0;
+        for (int l = solo; l < L; at += int(a.pl.lev[l].n), ++l)
+            for (int i = tid; i < int(a.pl.lev[l].n); i += MGT) solo_mem.dinv[at + i] = a.pl.lev[l].dinv[i];
+        __syncthreads();
+    }
+    unsigned target = 0;
+    bool first = a.first != 0, bad = false;
+    double rz = first ? 0 : a.scal[S_RZ], beta = first ? 0 : a.scal[S_BETA], rr0 = first ? 0 : a.scal[S_RR0];
+    double rr = 0, alpha = 0;
+    int done = first ? 0 : int(a.scal[S_ITER]);
+    const int last = done + a.iters;
+    int cur = first ? 0 : (done + 1) & 1;  // the copy of s that holds the current one (and of p, the last one)
+    // the block's share of a sum to every block's total; false: waits given up
+    auto total = [&](double &v, double *partial) {
+        v = block_sum(v, sh);
+        if (tid == 0) partial[blockIdx.x] = v;
+        if (!grid_barrier(a.pl.sync, target)) return false;
+        v = grid_sum(partial, sh);
+        return true;
+    };
+    while (true) {
+        bad = true;
+        if (!first) {
+            if (done >= last) {
+                bad = false;
+                break;
+            }
+            double pq = phase_a(a, a.p[cur], a.p[cur ^ 1], beta, gd);
+            if (!total(pq, p_pq)) break;
+            alpha = rz / pq;
+            if (!(pq > 0) || !isfinite(alpha)) break;
+        }
+        rr = phase_b(a, a.p[cur ^ 1], a.s[cur], a.s[cur ^ 1], alpha, gd, !first);
+        if (!total(rr, p_rr)) break;
+        cur ^= 1;
+        if (first)
+            rr0 = rr;
+        else
+            ++done;
+        if (!(rr > a.rel2 * rr0)) {  // reached, or not a number
+            bad = false;
+            break;
+        }
+        bool lost = false;
+        for (int l = 1; l < solo && !lost; ++l) {
+            const MgLevelT<double> &v = a.pl.lev[l];
+            coarse_down(EllViewT<double>{v.cnt, v.col, v.val, v.n}, int(v.n), v.dinv, v.r, a.pl.lev[l + 1].r, t0, step);
+            lost = !grid_barrier(a.pl.sync, target);
+        }
+        if (lost) break;
+        if (blockIdx.x == 0) coarse_solo(a.pl, solo, solo_mem);
+        lost = !grid_barrier(a.pl.sync, target);
+        for (int l = solo - 1; l >= 1 && !lost; --l) {
+            const MgLevelT<double> &v = a.pl.lev[l];
+            coarse_up(EllViewT<double>{v.cnt, v.col, v.val, v.n}, int(v.n), v.dinv, v.r, a.pl.lev[l + 1].zo, v.zo, t0, step);
+            lost = !grid_barrier(a.pl.sync, target);
+        }
+        if (lost) break;
+        double rzn = phase_d(a, a.s[cur], gd);
+        if (!total(rzn, p_rz)) break;
+        beta = first ? 0.0 : rzn / rz;
+        if (!isfinite(beta)) beta = 0;
+        rz = rzn;
+        first = false;
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        a.scal[S_RZ] = rz;
+        a.scal[S_BETA] = beta;
+        a.scal[S_RR] = rr;
+        a.scal[S_RR0] = rr0;
+        a.scal[S_ITER] = done;
+        a.scal[S_BAD] = bad ? 1.0 : 0.0;
+    }
+}
+
+template <class M, class T>
+PcgResult pcg_run_mg(const M &A, long long n, long long gauge_row, const T *b, T *x, double rel_tol, int max_iter,
+                     const PcgWorkT<T> &w, const MgPlan<T> &pl, cudaStream_t st, int check, int stall_checks) {
+    PcgResult res;
+    res.levels = pl.L;
+    int sms = 0, dev = 0;
+    SDOT_CUDA(cudaGetDevice(&dev));
+    SDOT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const bool many = n > MANY_ROWS;
+    void (*const kernel)(PcgArgs<M, T>) = many ? k_pcg_mg<M, T, MANY_PER_SM> : k_pcg_mg<M, T, 1>;
+    // all blocks are resident: the kernels are compiled for these numbers per SM
+    const int g = int(std::min<long long>((n + MGT - 1) / MGT, std::min(many ? MANY_PER_SM * sms : sms, 2 * PCG_BLOCKS)));
+    k_init_mg<T><<<grid_of(n), TB, 0, st>>>(b, x, w.r, pl.s0, w.dinv, pl.p1, w.q, pl.qs, w.z, n);
+    note_launch();
+    SDOT_CUDA(cudaGetLastError());
+    PcgArgs<M, T> a{A, n, gauge_row, pl, w.dinv, x, w.r, {pl.s0, pl.s1}, w.q, pl.qs, {w.p, pl.p1}, w.z, w.scal, w.partial,
+                    rel_tol * rel_tol, 0, 1};
+    double hs[S_NSCAL] = {0}, hist[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int nchecks = 0;
+    // a launch runs until the tolerance is met or for this many iterations, so
+    // that no kernel holds the device for long
+    const int chunk = stall_checks > 0 ? check : 256;
+    for (int it = 0;;) {
+        a.iters = std::min(chunk, max_iter - it);
+        SDOT_CUDA(cudaMemsetAsync(pl.sync, 0, 2 * sizeof(unsigned), st));
+        void *args[] = {&a};
+        SDOT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(kernel), dim3(g), dim3(MGT), args, 0, st));
+        note_launch();
+        SDOT_CUDA(cudaMemcpyAsync(hs, w.scal, sizeof(hs), cudaMemcpyDeviceToHost, st));
+        SDOT_CUDA(cudaStreamSynchronize(st));
+        a.first = 0;
+        it = int(hs[S_ITER]);
+        if (hs[S_BAD] != 0 || !(hs[S_RR] == hs[S_RR])) break;
+        if (hs[S_RR] <= a.rel2 * hs[S_RR0]) {
+            res.converged = true;
+            break;
+        }
+        if (it >= max_iter) break;
+        if (stall_checks > 0) {
+            const int k = stall_checks < 8 ? stall_checks : 8;
+            if (nchecks >= k && !(hs[S_RR] <= 0.5 * hist[(nchecks - k) % 8])) break;
+            hist[nchecks % 8] = hs[S_RR];
+            ++nchecks;
+        }
+    }
+    res.iterations = int(hs[S_ITER]);
+    if (hs[S_RR0] == 0) {
+        res.converged = true;
+        return res;
+    }
+    res.rel_residual = std::sqrt(hs[S_RR] / hs[S_RR0]);
+    if (res.rel_residual <= rel_tol) res.converged = true;
+    return res;
+}
+
 // stall_checks > 0: also stop once |r|^2 has not halved over the last
 // stall_checks checks (the inner FP32 solves, whose attainable accuracy ends
 // above the tolerance on ill-conditioned systems).
@@ -773,20 +1043,15 @@ PcgResult pcg_run(const M &A, long long n, long long gauge_row, const T *b, T *x
     note_launch();
     MgPlan<T> pl;
     const int cap = w.mg_cap > 64 ? MG_CAP_MAX : 64;
-    bool mg = multilevel && n > MG_COARSE && w.mg && mg_plan(n, cap, nullptr, pl) <= w.mg_doubles;
+    const bool mg = multilevel && n > MG_COARSE && w.mg && mg_plan(n, cap, nullptr, pl) <= w.mg_doubles;
     if (mg) {
         mg_plan(n, cap, w.mg, pl);
-        mg = mg_setup(A, gauge_row, w.scal, pl, cap, st);
+        if constexpr (!std::is_same_v<M, CsrView>)  // CSR solves are Jacobi's
+            if (mg_setup(A, gauge_row, w.scal, pl, cap, st))
+                return pcg_run_mg(A, n, gauge_row, b, x, rel_tol, max_iter, w, pl, st, check, stall_checks);
     }
-    if (mg) {
-        k_init_mg<T><<<g, TB, 0, st>>>(b, x, w.r, w.partial, n);
-        mg_vcycle(A, gauge_row, w.scal, w.dinv, pl, w.r, w.q, w.z, w.partial, w.p, g, st);
-        for (int c = 0; c < 1 + mg_launches(pl); ++c) note_launch();
-        res.levels = pl.L;
-    } else {
-        k_init<T><<<g, TB, 0, st>>>(b, x, w.r, w.z, w.p, w.dinv, w.partial, n);
-        note_launch();
-    }
+    k_init<T><<<g, TB, 0, st>>>(b, x, w.r, w.z, w.p, w.dinv, w.partial, n);
+    note_launch();
     k_final<<<1, TB, 0, st>>>(w.partial, g, w.scal, 0);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
@@ -803,18 +1068,12 @@ PcgResult pcg_run(const M &A, long long n, long long gauge_row, const T *b, T *x
         for (int c = 0; c < chunk; ++c) {
             k_spmv<M, T><<<g, TB, 0, st>>>(A, n, gauge_row, w.p, w.q, w.scal, w.partial);
             k_final<<<1, TB, 0, st>>>(w.partial, g, w.scal, 1);
-            if (mg) {
-                // q is free once r is updated: it holds the pre-smoothed values
-                k_update_mg<T><<<g, TB, 0, st>>>(x, w.r, w.p, w.q, w.scal, w.partial, n);
-                mg_vcycle(A, gauge_row, w.scal, w.dinv, pl, w.r, w.q, w.z, w.partial, (T *)nullptr, g, st);
-            } else {
-                k_update<T><<<g, TB, 0, st>>>(x, w.r, w.z, w.p, w.q, w.dinv, w.scal, w.partial, n);
-            }
+            k_update<T><<<g, TB, 0, st>>>(x, w.r, w.z, w.p, w.q, w.dinv, w.scal, w.partial, n);
             k_final<<<1, TB, 0, st>>>(w.partial, g, w.scal, 2);
             k_pupdate<T><<<g, TB, 0, st>>>(w.z, w.p, w.scal, n);
         }
     };
-    const int per_iter = 5 + (mg ? mg_launches(pl) : 0);
+    const int per_iter = 5;
     // With `graph`, a full chunk of iterations is captured once as a CUDA
     // graph and replayed: one launch instead of 5 * check.
     cudaGraphExec_t exec = nullptr;

@@ -32,7 +32,7 @@ struct MgLevelT {
     long long n = 0;
     int *cnt = nullptr, *col = nullptr;  // ELL rows (width PcgWork::mg_cap)
     T *val = nullptr, *dinv = nullptr;
-    T *r = nullptr, *z = nullptr, *zo = nullptr;  // right-hand side, smoothed, output
+    T *r = nullptr, *zo = nullptr;  // right-hand side, output
 };
 
 // Doubles of multilevel storage a solve over n rows needs (coarse rows of
@@ -58,7 +58,8 @@ struct PcgResult {
 // |r| <= rel_tol |b| or after max_iter iterations (checked every `check`
 // iterations, the only host synchronisations).
 // graph: replay full chunks of `check` iterations from one captured CUDA
-// graph (st must be a created stream).
+// graph (st must be a created stream); Jacobi only, the multilevel solve runs
+// in one kernel.
 // multilevel: precondition with one V-cycle over Morton aggregates (needs
 // w.mg); Jacobi when n is small, when w.mg is too small, or when a coarse row
 // outgrows its ELL width.

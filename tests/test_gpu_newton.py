@@ -275,3 +275,27 @@ def test_refined_newton_3d(gpu_lib):
         g.solve_weights(c["target"], rel_mass_tol=1e-10, linear_solver=ls)
         out[ls] = g.get_weights()
     assert np.abs(out["fp64"] - out["fp32_refined"]).max() <= 1e-8 * np.abs(out["fp64"]).max()
+
+
+@pytest.mark.parametrize("dim,n", [(2, 49), (2, 192), (2, 193), (2, 1025), (2, 2048), (2, 16390), (2, 38000), (3, 50),
+                                   (3, 777), (3, 4100)])
+def test_multilevel_solve_sizes(gpu_lib, dim, n):
+    # the one-kernel multilevel solve where its levels and blocks change: the
+    # smallest size it takes (49 rows), one and two levels, levels around the
+    # largest that one block does alone, one row more or less than full blocks
+    # and aggregates, more rows than one per thread of the grid.  The Newton
+    # solution does not depend on the preconditioner: the bound of
+    # test_multilevel_and_jacobi_give_the_same_weights
+    from sdot_b200.power_diagram import PowerDiagram
+
+    p = np.random.default_rng(5300 + n).random((n, dim))
+    w = {}
+    for pc, ls in (("jacobi", "fp64"), ("multilevel", "fp64"), ("multilevel", "fp32_refined")):
+        g = PowerDiagram(p, np.zeros(n))
+        g.add_box_shape(np.zeros(dim), np.ones(dim))
+        rep = g.solve_weights(np.full(n, 1.0 / n), rel_mass_tol=1e-11, preconditioner=pc, linear_solver=ls)
+        assert (rep["pcg_levels"] > 0) == (pc == "multilevel")
+        w[pc, ls] = g.get_weights()
+    ref = w["jacobi", "fp64"]
+    for x in w.values():
+        assert np.abs(x - ref).max() <= 1e-9 * np.abs(ref).max()
