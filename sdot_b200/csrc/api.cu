@@ -467,7 +467,6 @@ struct sdot_ctx {
         a.start_xy = d_start;
         a.coeff = coeff;
         a.mode = mode;
-        a.mixed = precision == SDOT_MIXED;
         a.ball = ball;
         a.img_lo[0] = img_lo[0]; a.img_lo[1] = img_lo[1];
         a.img_hi[0] = img_hi[0]; a.img_hi[1] = img_hi[1];
@@ -843,7 +842,6 @@ struct sdot_ctx {
             SDOT_CUDA(cudaMemsetAsync(ras_buf, 0, size_t(3 * np) * sizeof(double), stream));
         SDOT_CUDA(cudaMemsetAsync(dstat, 0, sizeof(DevStatus), stream));
         Cell2DArgs a = args();
-        a.mixed = 0;
         a.ras = nums ? nullptr : ras_buf;
         a.ras_nums = nums ? ras_nums : nullptr;
         a.perm = perm();

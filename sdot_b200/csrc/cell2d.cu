@@ -2,10 +2,10 @@
 //
 // One thread builds one cell.  Threads take Diracs in Morton (sorted) order so
 // a warp works on 32 neighbouring cells and walks nearly the same tree nodes.
-// The fast tier keeps the cell polygon in shared memory (SoA, one column per
-// thread); cells that outgrow it are rebuilt by the big and huge tiers whose
-// polygons live in global scratch (one column per thread, coalesced).  The
-// traversal stack lives in local memory.
+// The fast tier keeps the cell polygon in shared memory (one column per thread,
+// coordinates relative to the Dirac, the order of the vertices in a register);
+// cells that outgrow it are rebuilt by the warp tier, whose polygons live in
+// global scratch.  The traversal stack lives in local memory.
 //
 // Reference behaviour restated here:
 //  * traversal, eviction test and bisector cuts: SpZGrid::for_each_laguerre_cell
@@ -45,7 +45,6 @@ static __device__ unsigned long long sdot_work[8];
 
 namespace {
 
-constexpr int T2D_MAX = 128;  // largest block of the fast kernels (their block size is tuned, see launch_all)
 constexpr int STACK = 64;   // traversal stack (depth <= 17 levels, <= 3 pending siblings each)
 constexpr int WTIER_WARPS = 148 * 4;  // warps of the warp-per-cell tier (4 per SM; 8 or 16 measured no faster)
 
@@ -404,37 +403,128 @@ SDOT_HDI void order_children(const Cell2DArgs &A, int first, int nch, double c0x
     cx(1, 2);
 }
 
-// Builds the Laguerre cell of sorted Dirac s (before any disc clipping) as a
-// machine of uniform steps, so that the 32 cells of a warp advance together.
-// The walk is SpZGrid::for_each_laguerre_cell's (SpZGrid.tcc:494-719): boxes
-// popped nearest-first (children pushed farthest-first, keyed on the float
-// squared distance from c0 to the box centre as the reference's queue),
-// skipped when the eviction test holds for every vertex (SpZGrid.tcc:475-480),
-// a leaf's Diracs cut in index order (bisector SpZGrid.tcc:506-522).
-// Every step -- a node test or one cut -- is the same pass over the vertices:
-// a cut classifies each vertex by its side of the bisector, a node test asks
-// whether some vertex fails the eviction test; both quantities are computed
-// for every vertex and the step's one is kept, so lanes on different kinds of
-// steps run the same instructions.  Only the application of an effective cut
-// and the handling of a needed node branch.
-// Returns the vertex count, -1 on capacity (or stack / visit cap) overflow,
-// -2 on a failed guard.
+// The polygon of one thread's cell in the fast tier: up to CAP vertices in
+// shared memory (slot k of thread t at [k * BS + t]) in coordinates relative to
+// the cell's Dirac, and the order of the slots in a register: nibble k of
+// `order` is the slot of vertex k, the nibbles past the last vertex are the free
+// slots.  A cut then moves no vertex: it writes the two new ones and rearranges
+// nibbles (the copy loops it takes the place of ran as long as the longest of
+// the warp).
+template <int CAP, int BS>
+struct Ring {
+    static_assert(CAP <= 16, "slots of four bits in a 64-bit word");
+    static constexpr unsigned long long ALL = CAP == 16 ? ~0ull : (1ull << (4 * CAP)) - 1;
+    double *x, *y;
+    int *id;
+    unsigned long long order = 0xfedcba9876543210ull & ALL;
+    double c0x, c0y;
+    int cap = CAP;  // bound of the debug checks
+
+    __device__ int slot(int k) const { return int(order >> (4 * SDOT_CHECK_IDX(k, CAP, 1))) & 15; }
+    __device__ double &ux(int k) const { return x[slot(k) * BS]; }
+    __device__ double &uy(int k) const { return y[slot(k) * BS]; }
+    __device__ int &I(int k) const { return id[slot(k) * BS]; }
+    // absolute coordinates, for the streaming stages
+    __device__ double X(int k) const { return c0x + ux(k); }
+    __device__ double Y(int k) const { return c0y + uy(k); }
+
+    // Cuts the polygon (n vertices) by nx ux + ny uy <= b; bit k of mask:
+    // vertex k is outside.  Same new vertices at the same places as
+    // plane_cut_apply: with i1 the first and i2 the last vertex removed, A on
+    // the edge into i1 takes the cut's id, B on the edge out of i2 keeps that
+    // edge's.  Returns the new count, or -1 past CAP.
+    __device__ int cut(int n, unsigned mask, double nx, double ny, double b, int cut_id) {
+        const CutFacts f = cut_facts(mask, n);
+        if (f.nb_out == n) return 0;
+        const int nb_in = n - f.nb_out;
+        if (f.nb_out == 1 && n + 1 > CAP) return -1;
+        const bool wrap = f.out_last && f.first_out == 0;
+        const int i3 = wrap ? f.first_in : f.first_out + f.nb_out;  // may be n: vertex 0
+        const int i1 = wrap ? f.first_in + nb_in : f.first_out;
+        const int s1 = slot(i1), s0 = slot(i1 == 0 ? n - 1 : i1 - 1);
+        const int s2 = slot(i3 == 0 ? n - 1 : i3 - 1), s3 = slot(i3 == n ? 0 : i3);
+        const double p0x = x[s0 * BS], p0y = y[s0 * BS], p1x = x[s1 * BS], p1y = y[s1 * BS];
+        const double p2x = x[s2 * BS], p2y = y[s2 * BS], p3x = x[s3 * BS], p3y = y[s3 * BS];
+        const double d0 = b - (p0x * nx + p0y * ny), d1 = b - (p1x * nx + p1y * ny);
+        const double d2 = b - (p2x * nx + p2y * ny), d3 = b - (p3x * nx + p3y * ny);
+        // the two edge ratios d0 / (d1 - d0) and d3 / (d2 - d3) by one division
+        const double u = d1 - d0, v = d2 - d3, r = 1.0 / (u * v);
+        const double m1 = d0 * v * r, m2 = d3 * u * r;
+        const int id2 = id[s2 * BS];
+        int sa, sb;  // slots of A and B
+        if (wrap) {
+            // [B, kept run, A]: B takes the place before the kept run, A the
+            // one after it, and the order is turned to start at B
+            sa = s1;
+            sb = s2;
+            const int t = 4 * (i3 - 1);
+            order = ((order >> t) | (order << (4 * CAP - t))) & ALL;
+        } else if (f.nb_out == 1) {
+            // A in the removed place, B in a free slot after it
+            sa = s1;
+            sb = slot(n);
+            const unsigned long long low = (1ull << (4 * (i1 + 1))) - 1;
+            const unsigned long long used = n + 1 == 16 ? ~0ull : (1ull << (4 * (n + 1))) - 1;
+            order = (order & (low | ~used)) | ((unsigned long long)sb << (4 * (i1 + 1))) |
+                    (((order & ~low) << 4) & used & ~((1ull << (4 * (i1 + 2))) - 1));
+        } else {
+            // A and B in the first two removed places, the other removed ones
+            // to the end
+            sa = s1;
+            sb = slot(i1 + 1);
+            if (f.nb_out > 2) {
+                const int keep = 4 * (i1 + 2), gone = 4 * (f.nb_out - 2);
+                const unsigned long long low = (1ull << keep) - 1;
+                const unsigned long long run = (order >> keep) & ((1ull << gone) - 1);
+                order = (order & low) | (((order >> gone) & ~low) & ALL) | (run << (4 * CAP - gone));
+            }
+        }
+        x[sa * BS] = p0x - m1 * (p1x - p0x);
+        y[sa * BS] = p0y - m1 * (p1y - p0y);
+        id[sa * BS] = cut_id;
+        x[sb * BS] = p3x - m2 * (p2x - p3x);
+        y[sb * BS] = p3y - m2 * (p2y - p3y);
+        id[sb * BS] = id2;
+        return nb_in + 2;
+    }
+};
+
+// Builds the Laguerre cells of the warp's 32 sorted Diracs, one per lane
+// (before any disc clipping).  The walk of each is
+// SpZGrid::for_each_laguerre_cell's (SpZGrid.tcc:494-719): boxes popped
+// nearest-first (children pushed farthest-first, keyed on the float squared
+// distance from c0 to the box centre as the reference's queue), skipped when
+// the eviction test holds for every vertex (SpZGrid.tcc:475-480), a leaf's
+// Diracs cut in index order (bisector SpZGrid.tcc:506-522).
+// The lanes run node tests together and cuts together: node steps go on until
+// at most WAIT lanes still look for a leaf while others hold one, then the
+// leaves are cut out of every cell that holds one.  (With one loop in which
+// each lane took whichever step its walk was at, every turn ran the node test,
+// the ordering of children, the cut test and the cut for some of the lanes:
+// 6.2 of 32 lanes active.)
+// Returns per lane the vertex count, -1 on capacity (or stack / visit cap)
+// overflow, -2 on a failed guard; every lane of the warp calls it (live: it has
+// a cell).
 // PER (periodic domains): after the tree, the walk visits it again once per
 // translation t, as the tree of the Diracs x_j + t (SpZGrid.tcc:558-561:
 // every translation's root enters the front; boxes and Diracs are shifted by
 // t, :396-397 and :608-611); a cut by the image of Dirac j under translation
 // k carries the id j + (k + 1) n, and the Dirac's own images cut it too.
-template <bool PER = false>
-SDOT_KFN int build_cell(const Cell2DArgs &A, long long s, const PolyView<double> &cell, int cap, double c0x, double c0y,
-                        double w0) {
-    int n = A.start_n;
+// WAIT 4 / 8 / 12 / 16 / 22: 3.47 / 3.29 / 3.26 / 3.26 / 3.30 ms at 1M Diracs,
+// 0.75 / 0.69 / 0.66 / 0.65 / 0.67 ms at 147,000.
+constexpr int WAIT = 12;
+
+template <bool PER, int CAP, int BS>
+__device__ int build_cell(const Cell2DArgs &A, long long s, bool live, Ring<CAP, BS> &cell, double w0) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const double c0x = cell.c0x, c0y = cell.c0y;
+    int n = live ? A.start_n : 0;
     for (int k = 0; k < n; ++k) {
-        cell.X(k) = A.start_xy[2 * k];
-        cell.Y(k) = A.start_xy[2 * k + 1];
+        cell.ux(k) = A.start_xy[2 * k] - c0x;
+        cell.uy(k) = A.start_xy[2 * k + 1] - c0y;
         cell.I(k) = domain_id(k);
     }
-    // The walk's memory reads are issued a step before their use, so that
-    // their latency overlaps the vertex pass of the step before: the node
+    // The walk's memory reads are issued a step before their use: the node
     // popped next is kept in a register (the stack holds the others), and the
     // position and weight of the next Dirac of a leaf are loaded while the
     // current one cuts.
@@ -442,6 +532,7 @@ SDOT_KFN int build_cell(const Cell2DArgs &A, long long s, const PolyView<double>
     int sp = 0;                 // stack entries below `top`
     int top = 0;                // the node the next node step pops
     bool has_top = true;
+    bool done = !live;
     int j = 0, je = 0;          // Diracs of the current leaf still to cut by
     double cjx = 0, cjy = 0, cjw = 0;  // Dirac j
     int visits = 0;
@@ -451,398 +542,140 @@ SDOT_KFN int build_cell(const Cell2DArgs &A, long long s, const PolyView<double>
     // shifted by the current translation (PER only: adding a zero would not
     // be free, it turns -0 into +0)
     auto tr = [&](double v, double t) { return PER ? v + t : v; };
+    auto load = [&](int k) {
+        (void)SDOT_CHECK_IDX(k, A.n, 6);
+        const double2 p = reinterpret_cast<const double2 *>(A.pos)[k];
+        cjx = tr(p.x, tx);
+        cjy = tr(p.y, ty);
+        cjw = A.w[k];
+    };
+    auto stop = [&](int result) {
+        n = result;
+        done = true;
+        j = je = 0;
+    };
     while (true) {
-        // ---- the step: one cut (j < je) or one node test
-        if (PER && j >= je && !has_top && sym + 1 < A.ntrans) {
-            // the next translation's walk starts from the root again
-            ++sym;
-            tx = A.trans[2 * sym];
-            ty = A.trans[2 * sym + 1];
-            top = 0;
-            has_top = true;
-        }
-        const bool is_cut = j < je;
-        double ox = 0, oy = 0, nx = 0, ny = 0;
-        double lo0 = 0, lo1 = 0, hi0 = 0, hi1 = 0, maxw = 0;
-        int node = -1, nd_a = 0, nd_b = 0;
-        int jn = 0;
-        double njx = 0, njy = 0, njw = 0;
-        if (is_cut) {
-            bisector(c0x, c0y, w0, cjx, cjy, cjw, ox, oy, nx, ny);
-            jn = skip_self(j + 1);
-            if (jn < je) {
-                (void)SDOT_CHECK_IDX(jn, A.n, 6);
-                njx = tr(A.pos[2 * jn], tx);
-                njy = tr(A.pos[2 * jn + 1], ty);
-                njw = A.w[jn];
+        // ---- node steps
+        while (true) {
+            const bool want = !done && j >= je;
+            const unsigned wm = __ballot_sync(FULL, want), hm = __ballot_sync(FULL, j < je);
+            if (!wm || (hm && __popc(wm) <= WAIT)) break;
+            if (!want) continue;
+            if (!has_top) {
+                if (!PER || sym + 1 >= A.ntrans) {
+                    done = true;
+                    continue;
+                }
+                // the next translation's walk starts from the root again
+                ++sym;
+                tx = A.trans[2 * sym];
+                ty = A.trans[2 * sym + 1];
+                top = 0;
+                has_top = true;
             }
-        } else {
-            if (!has_top) break;
             if (++visits > (PER ? (A.ntrans + 1) * A.max_nodes : A.max_nodes)) {  // each tree walk visits a node once
                 flag_error(A.err, DE_ITER);
-                return -1;
+                stop(-1);
+                continue;
             }
-            node = top;
+            const int node = top;
             if (sp > 0)
                 top = stack[--sp];
             else
                 has_top = false;
-            const TreeNode<2> &nd = A.nodes[SDOT_CHECK_IDX(node, A.max_nodes, 4)];
-            lo0 = tr(nd.lo[0], tx);
-            lo1 = tr(nd.lo[1], ty);
-            hi0 = tr(nd.hi[0], tx);
-            hi1 = tr(nd.hi[1], ty);
-            maxw = nd.maxw;
-            nd_a = nd.a;
-            nd_b = nd.b;
-        }
-        // ---- the pass over the vertices: a cut classifies each vertex by
-        // its side of the bisector (bit k: vertex k outside); a node test
-        // stops at the first vertex that fails the eviction test, as the
-        // reference's all_pos does (mask 1: the box is needed)
-        unsigned mask = 0;
-        int tested = n;
-        if (is_cut) {
-            for (int k = 0; k < n; ++k) {
-                const double d = (ox - cell.X(k)) * nx + (oy - cell.Y(k)) * ny;
-                mask |= unsigned(d < 0.0) << k;
+            const TreeNode<2> nd = A.nodes[SDOT_CHECK_IDX(node, A.max_nodes, 4)];
+            const double lo0 = tr(nd.lo[0], tx) - c0x, lo1 = tr(nd.lo[1], ty) - c0y;
+            const double hi0 = tr(nd.hi[0], tx) - c0x, hi1 = tr(nd.hi[1], ty) - c0y;
+            // the eviction test, left at the first vertices that fail it, as
+            // the reference's all_pos does
+            bool need = false;
+            for (int k = 0; k < n && !need; k += 2) {
+                const int a = cell.slot(k), b = cell.slot(k + 1 < n ? k + 1 : k);
+                const double ax = cell.x[a * BS], ay = cell.y[a * BS], bx = cell.x[b * BS], by = cell.y[b * BS];
+                const double gx = gap(lo0, hi0, ax), gy = gap(lo1, hi1, ay);
+                const double hx = gap(lo0, hi0, bx), hy = gap(lo1, hi1, by);
+                need = !(ax * ax + ay * ay - w0 <= gx * gx + gy * gy - nd.maxw) ||
+                       !(bx * bx + by * by - w0 <= hx * hx + hy * hy - nd.maxw);
+                SDOT_WORK_ADD(3, k + 1 < n ? 2 : 1);
             }
-        } else {
-            for (int k = 0; k < n; ++k) {
-                const double px = cell.X(k), py = cell.Y(k);
-                const double qx = fmin(hi0, fmax(lo0, px)), qy = fmin(hi1, fmax(lo1, py));
-                const double lhs = (c0x - px) * (c0x - px) + (c0y - py) * (c0y - py) - w0;
-                const double rhs = (qx - px) * (qx - px) + (qy - py) * (qy - py) - maxw;
-                if (!(lhs <= rhs)) {  // this vertex fails: the box is needed
-                    mask = 1u;
-                    tested = k + 1;
-                    break;
+            SDOT_WORK_ADD(2, 1);
+            if (!need) continue;  // every vertex passes: the box is evicted
+            if (nd.b < 0) {
+                const int first = nd.a, nch = -nd.b;
+                if (nch < 2 || nch > 4 || first < 1 || first + nch > A.max_nodes) {
+                    guard_fail(A, 1, s, node);
+                    stop(-2);
+                    continue;
                 }
-            }
-        }
-        (void)tested;
-        const CutFacts f = cut_facts(mask, n);
-        SDOT_WORK_ADD(is_cut ? 0 : 2, 1);
-        SDOT_WORK_ADD(is_cut ? 1 : 3, tested);
-        if (is_cut) {
-            if (f.nb_out) {
-                SDOT_WORK_ADD(4, 1);
-                n = plane_cut_apply(cell, n, cap, ox, oy, nx, ny, PER ? j + (sym + 1) * int(A.n) : j, f);
-                if (n <= 0) return n;
-            }
-            j = jn;
-            cjx = njx;
-            cjy = njy;
-            cjw = njw;
-            continue;
-        }
-        if (f.nb_out == 0) continue;  // every vertex passes: the box is evicted
-        if (nd_b < 0) {
-            const int first = nd_a, nch = -nd_b;
-            if (nch < 2 || nch > 4 || first < 1 || first + nch > A.max_nodes) {
-                guard_fail(A, 1, s, node);
-                return -2;
-            }
-            if (sp + nch > STACK) {
-                flag_error(A.err, DE_STACK);
-                return -1;
-            }
-            int ch[4];
-            order_children<PER>(A, first, nch, c0x, c0y, tx, ty, ch);
+                if (sp + nch > STACK) {
+                    flag_error(A.err, DE_STACK);
+                    stop(-1);
+                    continue;
+                }
+                int ch[4];
+                order_children<PER>(A, first, nch, c0x, c0y, tx, ty, ch);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                if (c < nch) {
-                    if (has_top) stack[sp++] = top;
-                    top = ch[c];
-                    has_top = true;
+                for (int c = 0; c < 4; ++c) {
+                    if (c < nch) {
+                        if (has_top) stack[sp++] = top;
+                        top = ch[c];
+                        has_top = true;
+                    }
+                }
+            } else {
+                if (nd.a < 0 || nd.b > A.n) {
+                    guard_fail(A, 2, s, node);
+                    stop(-2);
+                    continue;
+                }
+                j = skip_self(nd.a);
+                je = nd.b;
+                if (j < je) load(j);
+            }
+        }
+        if (!__any_sync(FULL, j < je)) break;  // no leaf, and no walk goes on
+        // ---- cuts
+        while (__any_sync(FULL, j < je)) {
+            if (!(j < je)) continue;
+            // the bisector (SpZGrid.tcc:506-522) relative to c0: n . u <= b.
+            // One position twice has none (the reference's is not a number)
+            const double nx = cjx - c0x, ny = cjy - c0y;
+            const double b = 0.5 * (nx * nx + ny * ny) + 0.5 * (w0 - cjw);
+            const int jc = j;
+            j = skip_self(j + 1);
+            if (j < je) load(j);
+            unsigned mask = 0;
+            for (int k0 = 0; k0 < n; k0 += 4) {
+                const unsigned h = unsigned(cell.order >> (4 * k0));
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int a = int(h >> (4 * k)) & 15;
+                    const double d = b - (cell.x[a * BS] * nx + cell.y[a * BS] * ny);
+                    mask |= unsigned(d < 0.0) << (k0 + k);
                 }
             }
-        } else {
-            if (nd_a < 0 || nd_b > A.n) {
-                guard_fail(A, 2, s, node);
-                return -2;
-            }
-            j = skip_self(nd_a);
-            je = nd_b;
-            if (j < je) {
-                cjx = tr(A.pos[2 * j], tx);
-                cjy = tr(A.pos[2 * j + 1], ty);
-                cjw = A.w[j];
+            mask &= (1u << n) - 1u;
+            SDOT_WORK_ADD(0, 1);
+            SDOT_WORK_ADD(1, n);
+            if (mask && (nx != 0 || ny != 0)) {
+                SDOT_WORK_ADD(4, 1);
+                n = cell.cut(n, mask, nx, ny, b, PER ? jc + (sym + 1) * int(A.n) : jc);
+                if (n <= 0) stop(n);
             }
         }
     }
     return n;
 }
 
-// ---------------------------------------------------------------- mixed FP32
-// FP32 build of the cell of Dirac s for the mixed-precision path, in
-// coordinates relative to c0 (vertex u = p - c0), so that the float error is
-// relative to the size of the cell rather than of the domain.  Same walk and
-// same steps as build_cell; the decisions are made safe this way:
-//  * a box is evicted only when every vertex passes the eviction test by more
-//    than the float rounding of its two sides (a wrong eviction could drop a
-//    neighbour; an extra visit only costs time);
-//  * a cut that classifies some vertex within the float rounding of the
-//    bisector stops the build with -3: the caller rebuilds the cell in FP64.
-// The polygon's edge ids then give the topology that the FP64 re-clip
-// (ReclipView) turns into exact vertices.  Returns like build_cell, or -3.
-constexpr float F32_MARGIN = 16.0f * 5.96e-8f;  // 16 float ulps, relative
-
-SDOT_KFN int build_cell_f32(const Cell2DArgs &A, long long s, const PolyView<float> &cell, int cap, double c0x,
-                            double c0y, double w0, bool local) {
-    const float w0f = float(w0);
-    int n = 0;
-    float span = 0;  // size of the starting polygon: the scale of the vertices' rounding
-    if (local) {
-        // Start from a local square of half-size R around c0 cut by the
-        // domain's edges, not from the domain itself: float vertices
-        // interpolated along domain-sized edges would carry errors at the
-        // domain's scale.  R is 3 times the farthest of the 12 Morton-order
-        // neighbours.  The square is exact for the cell when none of its
-        // edges survives (the eviction tests on the truncated polygon are
-        // then valid for the whole cell); otherwise the cell is rebuilt in
-        // FP64, or, when it only emptied within the square, walked again from
-        // the whole domain (-4).
-        double r2 = 0;
-        for (long long q = s - 6; q <= s + 6; ++q) {
-            if (q == s || q < 0 || q >= A.n) continue;
-            const double dx = A.pos[2 * q] - c0x, dy = A.pos[2 * q + 1] - c0y;
-            r2 = fmax(r2, dx * dx + dy * dy);
-        }
-        const float R = float(3.0 * sqrt(r2));
-        if (!(R > 0)) return -3;
-        span = 2 * R;
-        n = 4;
-        cell.X(0) = -R; cell.Y(0) = -R; cell.I(0) = ID_LOCAL;
-        cell.X(1) = R;  cell.Y(1) = -R; cell.I(1) = ID_LOCAL;
-        cell.X(2) = R;  cell.Y(2) = R;  cell.I(2) = ID_LOCAL;
-        cell.X(3) = -R; cell.Y(3) = R;  cell.I(3) = ID_LOCAL;
-        for (int e = 0; e < A.start_n && n > 0; ++e) {
-            const int e1 = e + 1 < A.start_n ? e + 1 : 0;
-            const double p0x = A.start_xy[2 * e] - c0x, p0y = A.start_xy[2 * e + 1] - c0y;
-            const double dx = A.start_xy[2 * e1] - A.start_xy[2 * e];
-            const double dy = A.start_xy[2 * e1 + 1] - A.start_xy[2 * e + 1];
-            n = plane_cut(cell, n, cap, float(p0x), float(p0y), float(dy), float(-dx), domain_id(e));
-        }
-        if (n <= 0) return -4;  // the square misses the domain
-    } else {
-        // the whole domain: used to decide cells that emptied within the
-        // square; a non-empty result goes to FP64
-        n = A.start_n;
-        for (int k = 0; k < n; ++k) {
-            cell.X(k) = float(A.start_xy[2 * k] - c0x);
-            cell.Y(k) = float(A.start_xy[2 * k + 1] - c0y);
-            cell.I(k) = domain_id(k);
-            span = fmaxf(span, fabsf(cell.X(k)) + fabsf(cell.Y(k)));
-        }
-        span *= 2;
-    }
-    auto has_local = [&]() {
-        for (int k = 0; k < n; ++k)
-            if (cell.I(k) == ID_LOCAL) return true;
-        return false;
-    };
-    int stack[STACK];
-    int sp = 0;
-    stack[sp++] = 0;
-    int j = 0, je = 0;
-    int visits = 0;
-    while (true) {
-        const bool is_cut = j < je;
-        float ox = 0, oy = 0, nx = 0, ny = 0;
-        float lo0 = 0, lo1 = 0, hi0 = 0, hi1 = 0, maxw = 0;
-        int node = -1, nd_a = 0, nd_b = 0;
-        if (is_cut) {
-            if (j == s) {
-                ++j;
-                continue;
-            }
-            (void)SDOT_CHECK_IDX(j, A.n, 6);
-            const double vx = A.pos[2 * j] - c0x, vy = A.pos[2 * j + 1] - c0y;
-            const double x = 0.5 + 0.5 * (w0 - A.w[j]) / (vx * vx + vy * vy);
-            nx = float(vx);
-            ny = float(vy);
-            ox = float(x * vx);
-            oy = float(x * vy);
-        } else {
-            if (sp == 0) break;
-            if (++visits > A.max_nodes) {
-                flag_error(A.err, DE_ITER);
-                return -1;
-            }
-            node = stack[--sp];
-            const TreeNode<2> &nd = A.nodes[SDOT_CHECK_IDX(node, A.max_nodes, 4)];
-            lo0 = float(nd.lo[0] - c0x);
-            lo1 = float(nd.lo[1] - c0y);
-            hi0 = float(nd.hi[0] - c0x);
-            hi1 = float(nd.hi[1] - c0y);
-            maxw = float(nd.maxw);
-            nd_a = nd.a;
-            nd_b = nd.b;
-        }
-        // a cut classifies every vertex (and flags one too close to call);
-        // a node test stops at the first vertex that fails the eviction
-        // test by more than its rounding margin (mask 1: the box is needed)
-        unsigned mask = 0;
-        bool near = false;
-        if (is_cut) {
-            for (int k = 0; k < n; ++k) {
-                const float px = cell.X(k), py = cell.Y(k);
-                const float ex = ox - px, ey = oy - py;
-                const float d = ex * nx + ey * ny;
-                // rounding of d: the products, the bisector's origin, and the
-                // vertex, whose error scales with the edges it was cut from
-                near |= fabsf(d) <= F32_MARGIN * (fabsf(ex * nx) + fabsf(ey * ny) +
-                                                  (fabsf(ox) + fabsf(px) + span) * fabsf(nx) +
-                                                  (fabsf(oy) + fabsf(py) + span) * fabsf(ny));
-                mask |= unsigned(d < 0.0f) << k;
-            }
-        } else {
-            for (int k = 0; k < n; ++k) {
-                const float px = cell.X(k), py = cell.Y(k);
-                const float qx = fminf(hi0, fmaxf(lo0, px)) - px, qy = fminf(hi1, fmaxf(lo1, py)) - py;
-                const float uu = px * px + py * py, qq = qx * qx + qy * qy;
-                const float lhs = uu - w0f, rhs = qq - maxw;
-                const float emargin = F32_MARGIN * (uu + fabsf(w0f) + qq + fabsf(maxw));
-                if (!(lhs <= rhs - emargin)) {
-                    mask = 1u;
-                    break;
-                }
-            }
-        }
-        if (near) return -3;
-        const CutFacts f = cut_facts(mask, n);
-        if (is_cut) {
-            if (f.nb_out) {
-                if (f.nb_out == n && has_local()) return -4;  // empty within the square only
-                n = plane_cut_apply(cell, n, cap, ox, oy, nx, ny, j, f);
-                if (n <= 0) return n;
-            }
-            ++j;
-            continue;
-        }
-        if (f.nb_out == 0) continue;
-        if (nd_b < 0) {
-            const int first = nd_a, nch = -nd_b;
-            if (nch < 2 || nch > 4 || first < 1 || first + nch > A.max_nodes) {
-                guard_fail(A, 1, s, node);
-                return -2;
-            }
-            if (sp + nch > STACK) {
-                flag_error(A.err, DE_STACK);
-                return -1;
-            }
-            int ch[4];
-            order_children<false>(A, first, nch, c0x, c0y, 0.0, 0.0, ch);
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (c < nch) stack[sp++] = ch[c];
-        } else {
-            if (nd_a < 0 || nd_b > A.n) {
-                guard_fail(A, 2, s, node);
-                return -2;
-            }
-            j = nd_a;
-            je = nd_b;
-        }
-    }
-    return has_local() ? -3 : n;
-}
-
-// The FP64 polygon of a cell whose topology came from the FP32 build: vertex
-// k is the intersection of the lines of edges k - 1 and k (a weighted
-// bisector, or an edge of the starting polygon), solved in FP64 in
-// coordinates relative to c0 and shifted back.  X, Y, I as PolyView's.
-struct ReclipView {
-    const Cell2DArgs &A;
-    PolyView<float> poly;
-    int n;
-    double c0x, c0y, w0;
-    int cap = CAP_FAST_2D;  // vertex slots (bound of the debug checks)
-    mutable int ck = -1;
-    mutable double vx = 0, vy = 0;
-
-    SDOT_HDI int I(int k) const { return poly.I(k); }
-    // line a . u = b of the edge with this id (u relative to c0)
-    SDOT_HDI void line(int id, double &ax, double &ay, double &b) const {
-        if (id >= 0) {
-            const double dx = A.pos[2 * id] - c0x, dy = A.pos[2 * id + 1] - c0y;
-            ax = dx;
-            ay = dy;
-            b = 0.5 * (dx * dx + dy * dy) + 0.5 * (w0 - A.w[id]);
-        } else {
-            const int e = domain_edge(id), e1 = e + 1 < A.start_n ? e + 1 : 0;
-            const double p0x = A.start_xy[2 * e] - c0x, p0y = A.start_xy[2 * e + 1] - c0y;
-            const double p1x = A.start_xy[2 * e1] - c0x, p1y = A.start_xy[2 * e1 + 1] - c0y;
-            ax = p0y - p1y;
-            ay = p1x - p0x;
-            b = ax * p0x + ay * p0y;
-        }
-    }
-    // intersection of edges k - 1 and k; returns |sin| of their angle
-    SDOT_HDI double solve(int k, double &ux, double &uy) const {
-        double a1x, a1y, b1, a2x, a2y, b2;
-        line(I(k == 0 ? n - 1 : k - 1), a1x, a1y, b1);
-        line(I(k), a2x, a2y, b2);
-        const double det = a1x * a2y - a1y * a2x;
-        ux = (b1 * a2y - b2 * a1y) / det;
-        uy = (a1x * b2 - a2x * b1) / det;
-        return fabs(det) / (sqrt(a1x * a1x + a1y * a1y) * sqrt(a2x * a2x + a2y * a2y));
-    }
-    SDOT_HDI void vert(int k) const {
-        if (k == ck) return;
-        double ux, uy;
-        solve(k, ux, uy);
-        vx = c0x + ux;
-        vy = c0y + uy;
-        ck = k;
-    }
-    SDOT_HDI double X(int k) const {
-        vert(k);
-        return vx;
-    }
-    SDOT_HDI double Y(int k) const {
-        vert(k);
-        return vy;
-    }
-    // The FP32 topology is the FP64 one when: every FP64 vertex is near its
-    // FP32 vertex, no two consecutive edges are nearly parallel, and every
-    // FP64 edge runs the way its FP32 edge does and is not nearly of zero
-    // length (a reversed or vanishing edge marks a vertex where four cells
-    // nearly meet, whose topology depends on rounding).
-    SDOT_HDI bool consistent() const {
-        double vx0 = 0, vy0 = 0, px = 0, py = 0;
-        float gx = 0, gy = 0;
-        for (int k = 0; k <= n && n >= 2; ++k) {
-            const int kk = k == n ? 0 : k;
-            double ux, uy;
-            if (k == n) {
-                ux = vx0;
-                uy = vy0;
-            } else {
-                const double sn = solve(kk, ux, uy);
-                if (!(sn > 1e-6)) return false;
-            }
-            const float fx = poly.X(kk), fy = poly.Y(kk);
-            const double sc = fabs(double(fx)) + fabs(double(fy)) + 1e-300;
-            if (!(fabs(ux - fx) + fabs(uy - fy) <= 1e-4 * sc)) return false;
-            if (k == 0) {
-                vx0 = ux;
-                vy0 = uy;
-            } else {
-                const double ex = ux - px, ey = uy - py;
-                const double fex = double(fx) - gx, fey = double(fy) - gy;
-                if (!(ex * fex + ey * fey > 0)) return false;
-                if (fabs(ex) + fabs(ey) <= 1e-7 * (sc + fabs(px) + fabs(py))) return false;
-            }
-            px = ux;
-            py = uy;
-            gx = fx;
-            gy = fy;
-        }
-        return true;
-    }
-};
+// Vertex k relative to the Dirac at c0.
+template <class P>
+__device__ double rel_x(const P &cell, int k, double c0x) { return cell.X(k) - c0x; }
+template <class P>
+__device__ double rel_y(const P &cell, int k, double c0y) { return cell.Y(k) - c0y; }
+template <int CAP, int BS>
+__device__ double rel_x(const Ring<CAP, BS> &cell, int k, double) { return cell.ux(k); }
+template <int CAP, int BS>
+__device__ double rel_y(const Ring<CAP, BS> &cell, int k, double) { return cell.uy(k); }
 
 // Per-cell work once the polygon of Dirac s is built (n vertices; -1: a
 // capacity was exceeded, -2: a guard failed).  Returns false when a capacity
@@ -874,24 +707,35 @@ SDOT_KFN bool finish_cell(const Cell2DArgs &A, long long s, const P &cell, int n
     sink.trans = A.trans;
 
     if (DIRECT && !BALL) {
-        // reference order: fan from vertex 0, boundary items from edge (n-1 -> 0)
-        double tr2 = 0;
-        for (int i = 2; i < n; ++i) {
-            const double ax = cell.X(0), ay = cell.Y(0);
-            const double bx = cell.X(i - 1), by = cell.Y(i - 1), cx = cell.X(i), cy = cell.Y(i);
-            const double t2 = ax * (by - cy) + bx * (cy - ay) + cx * (ay - by);
-            tr2 += t2;
-            const double lea = 0.5 * t2 * A.coeff;
-            const double f = (1.0 / 3.0) * lea;
-            sink.momx += f * (ax + bx + cx);
-            sink.momy += f * (ay + by + cy);
-            sink.mass_c += lea;
-        }
-        sink.mass = A.coeff * (tr2 * 0.5);
+        // reference order: fan from vertex 0, boundary items from edge (n-1 ->
+        // 0), in coordinates about the Dirac (no cancellation of positions of
+        // the domain's size)
         sink.begin_piece(A.coeff);
-        for (int i1 = 0, i0 = n - 1; i1 < n; i0 = i1++) {
-            const double dx = cell.X(i1) - cell.X(i0), dy = cell.Y(i1) - cell.Y(i0);
-            sink.line(i0, sqrt(dx * dx + dy * dy));
+        if (n > 0) {
+            const double ax = rel_x(cell, 0, c0x), ay = rel_y(cell, 0, c0y);
+            double px = rel_x(cell, n - 1, c0x), py = rel_y(cell, n - 1, c0y);
+            double bx = ax, by = ay, tr2 = 0;
+            for (int i = 0; i < n; ++i) {
+                const double cx = i ? rel_x(cell, i, c0x) : ax, cy = i ? rel_y(cell, i, c0y) : ay;
+                sink.line(i ? i - 1 : n - 1, sqrt((cx - px) * (cx - px) + (cy - py) * (cy - py)));
+                px = cx;
+                py = cy;
+                if (i >= 2) {
+                    const double t2 = ax * (by - cy) + bx * (cy - ay) + cx * (ay - by);
+                    tr2 += t2;
+                    const double lea = 0.5 * t2 * A.coeff;
+                    const double f = (1.0 / 3.0) * lea;
+                    sink.momx += f * (ax + bx + cx);
+                    sink.momy += f * (ay + by + cy);
+                    sink.mass_c += lea;
+                }
+                bx = cx;
+                by = cy;
+            }
+            sink.mass = A.coeff * (tr2 * 0.5);
+            // moments about the origin, as the other modes leave them
+            sink.momx += c0x * sink.mass_c;
+            sink.momy += c0y * sink.mass_c;
         }
     } else if (DIRECT) {
         sink.begin_piece(A.coeff);
@@ -1002,79 +846,46 @@ __device__ void push_overflow(const Cell2DArgs &A, long long s) {
         flag_error(A.err, DE_CAPACITY);
 }
 
-// shared memory of the fast kernels, in half-doubles per vertex slot and
-// thread beyond the polygon: the per-edge accumulators of the image mode
+// Shared memory of a fast-tier block: polygons, and in the image modes the
+// per-edge accumulators.
+// Measured (1M clustered mix, FP64): 4.12 ms with one loop of mixed steps and
+// polygons moved in shared memory -> 3.25 ms; 77k warp instructions per warp
+// (95k), 7.6 of 32 lanes active, issue 71%: bound by instruction issue, over
+// half of it the vertex loops of the node tests.  Blocks of 32 / 64 / 128: 3.22
+// / 3.26 / 3.48 ms; 10 instead of 12 of them per SM: 3.40 ms.
+constexpr int BS = 64;  // threads of a fast-tier block
 template <int MODE>
-constexpr int smem_extra_halves() {
-    return MODE == DM_IMAGE || MODE == DM_IMAGE6 ? 2 : 0;
+constexpr size_t fast_smem() {
+    return size_t(CAP_FAST_2D) * BS * (20 + (MODE == DM_IMAGE || MODE == DM_IMAGE6 ? 8 : 0));
 }
 
 template <int MODE, bool BALL>
-// six blocks of T2D_MAX threads per SM: at most 85 registers per thread
-__global__ void __launch_bounds__(T2D_MAX, 6) k_cells2d(const Cell2DArgs A) {
+__global__ void __launch_bounds__(BS, 12) k_cells2d(const Cell2DArgs A) {
     extern __shared__ double smem[];
     constexpr int CAP = CAP_FAST_2D;
-    const int t = threadIdx.x, T2D = blockDim.x;
-    double *sx = smem;
-    double *sy = sx + CAP * T2D;
-    int *sid = reinterpret_cast<int *>(sy + CAP * T2D);
-    double *extra = sy + CAP * T2D + (CAP * T2D + 1) / 2;
-    PolyView<double> cell{sx + t, sy + t, sid + t, T2D, CAP};
-    double *acc = extra + t;
-    const long long s = blockIdx.x * (long long)T2D + t;
-    if (s >= A.n) return;
-    const int n = build_cell<MODE == DM_PERIODIC>(A, s, cell, CAP, A.pos[2 * s], A.pos[2 * s + 1], A.w[s]);
+    const int t = threadIdx.x;
+    double *acc = smem + 2 * CAP * BS + t;  // image modes, before the ids
+    double *sid = smem + (MODE == DM_IMAGE || MODE == DM_IMAGE6 ? 3 : 2) * CAP * BS;
+    const long long s = blockIdx.x * (long long)BS + t;
+    const bool live = s < A.n;
+    Ring<CAP, BS> cell;
+    cell.x = smem + t;
+    cell.y = smem + CAP * BS + t;
+    cell.id = reinterpret_cast<int *>(sid) + t;
+    cell.c0x = live ? A.pos[2 * s] : 0;
+    cell.c0y = live ? A.pos[2 * s + 1] : 0;
+    const int n = build_cell<MODE == DM_PERIODIC, CAP, BS>(A, s, live, cell, live ? A.w[s] : 0);
+    if (!live) return;
     SDOT_WORK_ADD(5, n > 0 ? n : 0);
     SDOT_WORK_ADD(6, 1);
     Out row(A.rows.cnt ? A.rows.col + s : nullptr, A.rows.cnt ? A.rows.val + s : nullptr, A.rows.stride, A.rows.cap);
     Out nbo(A.nb.cnt ? A.nb.col + s : nullptr, nullptr, A.nb.stride, A.nb.cap);
-    if (finish_cell<MODE, BALL>(A, s, cell, n, acc, T2D, row, nbo)) {
+    if (finish_cell<MODE, BALL>(A, s, cell, n, acc, BS, row, nbo)) {
         if (A.rows.cnt) A.rows.cnt[s] = row.cnt;
         if (A.nb.cnt) A.nb.cnt[s] = nbo.cnt;
     } else {
         push_overflow(A, s);
     }
-}
-
-// Fast tier of the mixed-precision path: FP32 build (polygon as floats in
-// shared memory), FP64 re-clip of its vertices and FP64 integration.  Cells
-// whose FP32 decisions were too close to call, whose topology does not
-// re-clip cleanly, or that overflow the capacity go to the FP64 warp tier.
-template <int MODE, bool BALL>
-// six blocks of T2D_MAX threads per SM, as the FP64 kernel (4% faster on the
-// 1M clustered mix than the unbounded 96 registers)
-__global__ void __launch_bounds__(T2D_MAX, 6) k_cells2d_mixed(const Cell2DArgs A) {
-    extern __shared__ double smem[];
-    constexpr int CAP = CAP_FAST_2D;
-    const int t = threadIdx.x, T2D = blockDim.x;
-    float *sx = reinterpret_cast<float *>(smem);
-    float *sy = sx + CAP * T2D;
-    int *sid = reinterpret_cast<int *>(sy + CAP * T2D);
-    double *extra = reinterpret_cast<double *>(sid + CAP * T2D);
-    PolyView<float> cell{sx + t, sy + t, sid + t, T2D, CAP};
-    double *acc = extra + t;
-    const long long s = blockIdx.x * (long long)T2D + t;
-    if (s >= A.n) return;
-    const double c0x = A.pos[2 * s], c0y = A.pos[2 * s + 1], w0 = A.w[s];
-    int n = build_cell_f32(A, s, cell, CAP, c0x, c0y, w0, true);
-    if (n == -4) {
-        n = build_cell_f32(A, s, cell, CAP, c0x, c0y, w0, false);
-        if (n > 0) n = -3;  // only an empty cell is decided by the domain-wide FP32 walk
-    }
-    const ReclipView view{A, cell, n > 0 ? n : 0, c0x, c0y, w0};
-    bool ok = n >= 0 || n == -2;
-    if (n > 0 && !view.consistent()) ok = false;
-    if (ok) {
-        Out row(A.rows.cnt ? A.rows.col + s : nullptr, A.rows.cnt ? A.rows.val + s : nullptr, A.rows.stride,
-                A.rows.cap);
-        Out nbo(A.nb.cnt ? A.nb.col + s : nullptr, nullptr, A.nb.stride, A.nb.cap);
-        ok = finish_cell<MODE, BALL>(A, s, view, n, acc, T2D, row, nbo);
-        if (ok) {
-            if (A.rows.cnt) A.rows.cnt[s] = row.cnt;
-            if (A.nb.cnt) A.nb.cnt[s] = nbo.cnt;
-        }
-    }
-    if (!ok) push_overflow(A, s);
 }
 
 // Polygon, accumulators and row buffers of one warp of the warp tier,
@@ -1249,29 +1060,6 @@ __global__ void __launch_bounds__(128) k_cells2d_wtier(const Cell2DArgs A, doubl
     }
 }
 
-// The block size of the fast kernels is picked once per kernel variant and
-// device by timing the candidates on the first evaluation large enough to
-// tell them apart (the results do not depend on it: one thread builds one
-// cell whatever the block).
-
-template <int MODE, bool BALL>
-size_t fast_smem(int bs, bool mixed) {
-    constexpr int CAP = CAP_FAST_2D;
-    const size_t extra = size_t(smem_extra_halves<MODE>()) * CAP * bs * 4;
-    return mixed ? size_t(CAP) * bs * 12 + extra : size_t(CAP) * bs * 16 + size_t(CAP * bs + 1) / 2 * 8 + extra;
-}
-
-template <int MODE, bool BALL>
-void launch_fast(const Cell2DArgs &a, int bs, cudaStream_t st) {
-    const size_t smem = fast_smem<MODE, BALL>(bs, a.mixed != 0);
-    if (a.mixed)
-        k_cells2d_mixed<MODE, BALL><<<ceil_div(a.n, bs), bs, smem, st>>>(a);
-    else
-        k_cells2d<MODE, BALL><<<ceil_div(a.n, bs), bs, smem, st>>>(a);
-    note_launch();
-    SDOT_CUDA(cudaGetLastError());
-}
-
 // Every cell into the warp tier's list (domain polygons larger than the fast
 // tier's polygons).
 __global__ void k_all_cells(int *list, int *cnt, long long n) {
@@ -1291,14 +1079,9 @@ template <int MODE, bool BALL>
 void launch_all(const Cell2DArgs &a, void *scratch, cudaStream_t st) {
     static PerDevice<int> attr_set;
     attr_set.once([] {
-        SDOT_CUDA(cudaFuncSetAttribute(k_cells2d<MODE, BALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(fast_smem<MODE, BALL>(T2D_MAX, false))));
-        SDOT_CUDA(cudaFuncSetAttribute(k_cells2d_mixed<MODE, BALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(fast_smem<MODE, BALL>(T2D_MAX, true))));
-        // 72% of the shared memory capacity (164 KB: 16 warps of 64-thread
-        // blocks) leaves the rest to L1 for the walk's tree, Diracs and stack;
-        // measured 2% faster on the 1M clustered mix than the largest carveout
-        SDOT_CUDA(cudaFuncSetAttribute(k_cells2d<MODE, BALL>, cudaFuncAttributePreferredSharedMemoryCarveout, 72));
+        // room for the twelve blocks per SM that the registers allow (2%
+        // faster than 72%, which holds ten)
+        SDOT_CUDA(cudaFuncSetAttribute(k_cells2d<MODE, BALL>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     });
     if (a.start_n > CAP_FAST_2D) {
         // the starting polygon alone overflows the fast tier: every cell is
@@ -1312,37 +1095,10 @@ void launch_all(const Cell2DArgs &a, void *scratch, cudaStream_t st) {
         SDOT_CUDA(cudaGetLastError());
         return;
     }
-    static PerDevice<int> tuned[2];  // best block size per device: FP64, mixed
-    PerDevice<int> &tu = tuned[a.mixed ? 1 : 0];
-    int best = tu.get();
-    if (!best && a.n >= (1 << 17)) {
-        // time each candidate on this evaluation's cells; every output of the
-        // trial runs is rewritten by the run that follows, and the overflow
-        // counters are zeroed before each run
-        const int cand[3] = {32, 64, 128};
-        float best_ms = 0;
-        cudaEvent_t e0, e1;
-        SDOT_CUDA(cudaEventCreate(&e0));
-        SDOT_CUDA(cudaEventCreate(&e1));
-        for (int bs : cand) {
-            reset_overflow(a, st);
-            SDOT_CUDA(cudaEventRecord(e0, st));
-            launch_fast<MODE, BALL>(a, bs, st);
-            SDOT_CUDA(cudaEventRecord(e1, st));
-            SDOT_CUDA(cudaEventSynchronize(e1));
-            float ms = 0;
-            SDOT_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            if (!best || ms < best_ms) {
-                best = bs;
-                best_ms = ms;
-            }
-        }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        tu.set(best);
-    }
     reset_overflow(a, st);
-    launch_fast<MODE, BALL>(a, best ? best : 64, st);
+    k_cells2d<MODE, BALL><<<ceil_div(a.n, BS), BS, fast_smem<MODE>(), st>>>(a);
+    note_launch();
+    SDOT_CUDA(cudaGetLastError());
     k_cells2d_wtier<MODE, BALL><<<WTIER_WARPS / 4, 128, 0, st>>>(a, static_cast<double *>(scratch), WTIER_WARPS,
                                                                   a.ovf_list, a.ovf_cnt);
     note_launch();
@@ -1382,10 +1138,7 @@ void cells2d_launch(const Cell2DArgs &a, void *scratch, cudaStream_t st) {
     if (a.mode == DM_SINGLE) {
         if (ball) launch_all<DM_SINGLE, true>(a, scratch, st); else launch_all<DM_SINGLE, false>(a, scratch, st);
     } else if (a.mode == DM_PERIODIC) {
-        // the mixed path has no periodic walk: the FP64 kernels run
-        Cell2DArgs b = a;
-        b.mixed = 0;
-        if (ball) launch_all<DM_PERIODIC, true>(b, scratch, st); else launch_all<DM_PERIODIC, false>(b, scratch, st);
+        if (ball) launch_all<DM_PERIODIC, true>(a, scratch, st); else launch_all<DM_PERIODIC, false>(a, scratch, st);
     } else if (a.mode == DM_IMAGE) {
         if (ball) launch_all<DM_IMAGE, true>(a, scratch, st); else launch_all<DM_IMAGE, false>(a, scratch, st);
     } else if (a.mode == DM_RASTER) {

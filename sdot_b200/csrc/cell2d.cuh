@@ -63,7 +63,6 @@ struct Cell2DArgs {
     const double *start_xy = nullptr;  // 2 * start_n
     double coeff = 1.0;                // single-item density
     int mode = DM_SINGLE;
-    int mixed = 0;                     // FP32 build + FP64 re-clip (SDOT_MIXED)
     int ball = 0;
     // image (nb_coeffs == 1)
     double img_lo[2] = {0, 0}, img_hi[2] = {1, 1};

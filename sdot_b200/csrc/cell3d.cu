@@ -297,13 +297,6 @@ __device__ __forceinline__ int cut3(Cell3<VB, MAXP> &C, Work3<VB, MAXP> &W, int 
     return 0;
 }
 
-// The distance of p from [lo, hi] (the signs read as integers: an FP64
-// minimum and maximum take several times the instructions).
-__device__ __forceinline__ double gap(double lo, double hi, double p) {
-    const double a = lo - p, b = p - hi;
-    return __double2hiint(a) >= 0 ? a : __double2hiint(b) >= 0 ? b : 0.0;
-}
-
 // A multilinear density rewritten about the cell's Dirac c: coefficients of
 // 1, u_x, u_y, u_z, u_x u_y, u_x u_z, u_y u_z, u_x u_y u_z for u = x - c.
 struct PolyRel {

@@ -30,10 +30,6 @@ constexpr int ID_ARC = -2;
 constexpr int ID_DOMAIN0 = -3;
 __host__ __device__ inline int domain_id(int e) { return ID_DOMAIN0 - e; }
 __host__ __device__ inline int domain_edge(int id) { return ID_DOMAIN0 - id; }
-// Edges of the local square that starts an FP32 build (mixed path); a cell
-// that keeps one is rebuilt in FP64, so these ids never reach an output.
-constexpr int ID_LOCAL = -(1 << 30);
-
 // Inside a piece (cell intersected with a domain item or a pixel):
 //  id >= 0       : came from edge `id` of the cell polygon
 //  id == PID_OWN : an edge of the item/pixel itself
@@ -145,6 +141,15 @@ __host__ __device__ inline void flag_error(unsigned *word, unsigned bits) {
     *word |= bits;
 #endif
 }
+
+#ifdef __CUDACC__
+// The distance of p from [lo, hi] (the signs read as integers: an FP64
+// minimum and maximum take several times the instructions).
+__device__ __forceinline__ double gap(double lo, double hi, double p) {
+    const double a = lo - p, b = p - hi;
+    return __double2hiint(a) >= 0 ? a : __double2hiint(b) >= 0 ? b : 0.0;
+}
+#endif
 
 // Sticky per-context error word written by kernels (never __trap).
 enum DevErr : unsigned {

@@ -34,7 +34,9 @@ class PowerDiagram:
     """Laguerre (power) diagram of weighted Diracs clipped to a domain.
 
     positions: (n, dim) array; weights: (n,) array (default zeros).
-    precision: "fp64" or "mixed".  radial_func: "unit" (FunctionEnum::Unit)
+    precision: "fp64" or "mixed" (allows FP32 clipping; the cells run in FP64
+    either way, which is faster here, the linear solves in FP32 with FP64
+    refinement).  radial_func: "unit" (FunctionEnum::Unit)
     or "in_ball_w05" (FunctionEnum::InBallW05: cells clipped by the disc of
     radius sqrt(w_i)).
     """

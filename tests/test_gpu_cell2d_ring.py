@@ -1,0 +1,47 @@
+"""2D cells at the edges of the fast tier's storage (polygons of 13 vertices,
+kept as an order over slots) and of its warps and blocks, against the C
+restatement (oracle/port.py), with the bounds of the 2D parity tests: 1e-12 of
+max(|value|, mean), 1e-11 for the Hessian of the near-circular cell, whose short
+edges are differences of nearby vertices."""
+import numpy as np
+import pytest
+
+from oracle import port
+from sdot_b200.power_diagram import PowerDiagram
+from tests.test_gpu_parity_2d import check_all
+
+pytestmark = pytest.mark.gpu
+
+
+def pair(p, w, **kw):
+    out = []
+    for cls in (PowerDiagram, port.PortPowerDiagram):
+        d = cls(p, w, **kw)
+        d.add_box_shape([0.0, 0.0], [1.0, 1.0])
+        out.append(d)
+    return out
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("k", list(range(3, 18)) + [40])
+def test_edges_of_one_cell(gpu_lib, k, precision):
+    # one cell of k edges: cuts that remove one, two and more vertices, over
+    # vertex 0 too (the Diracs' order is random), up to and past 13 vertices
+    rng = np.random.default_rng(8100 + k)
+    a = rng.permutation(k) * 2 * np.pi / k + rng.uniform(-0.3, 0.3, k) / k
+    d = 0.4 * rng.uniform(0.999, 1.001, k)
+    p = np.concatenate([[[0.5, 0.5]], 0.5 + d[:, None] * np.stack([np.cos(a), np.sin(a)], 1)])
+    g, r = pair(p, np.zeros(k + 1))
+    if precision == "mixed":
+        g = PowerDiagram(p, np.zeros(k + 1), precision="mixed")
+        g.add_box_shape([0.0, 0.0], [1.0, 1.0])
+    check_all(g, r, k + 1, rtol_hess=1e-11)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 127, 129, 1025])
+def test_walks_of_one_warp(gpu_lib, n):
+    # lanes whose walks end far apart: weights that empty some cells and make
+    # others reach over many, and a last warp of a few lanes
+    rng = np.random.default_rng(8200 + n)
+    g, r = pair(rng.random((n, 2)), rng.uniform(-1.0, 1.0, n) / n)
+    check_all(g, r, n, rtol_hess=1e-11)
