@@ -20,8 +20,6 @@
 namespace sdot {
 
 #define SDOT_HD __host__ __device__ __forceinline__
-// members of the streaming stages: left to the compiler's inlining choice
-// (forcing them inline multiplies the code of the nested pixel pipelines)
 #define SDOT_HDI __host__ __device__
 
 constexpr double kPi = 3.141592653589793238462643383279502884;
@@ -343,217 +341,184 @@ SDOT_HD void bisector(T c0x, T c0y, T w0, T c1x, T c1y, T w1, T &ox, T &oy, T &n
     oy = c0y + x * ny;
 }
 
-// ------------------------------------------------------------------------
-// Streaming stages.  A polygon is pushed vertex by vertex (push(x, y, tag),
-// tag = id of the edge leaving that vertex) then closed with finish().
-// Each stage forwards a transformed polygon to the next stage, so clipped
-// pieces never need their own vertex buffer.
-
-// Keep the half-plane  s * (coord - c) >= 0  (coord = x if axis == 0 else y).
-// New edges along the clip line get tag `own`.
-template <class Next>
-struct AxisClip {
-    Next &next;
-    int axis;
-    double c, s;
-    int own;
-    bool has_first = false;
-    double fx = 0, fy = 0;
-    int ft = 0;
-    double px = 0, py = 0;
-    int pt = 0;
-    SDOT_HDI AxisClip(Next &nx, int ax, double cc, double ss, int ow) : next(nx), axis(ax), c(cc), s(ss), own(ow) {}
-    SDOT_HDI double val(double x, double y) const { return s * ((axis == 0 ? x : y) - c); }
-    SDOT_HDI void edge(double ax, double ay, int at, double bx, double by) {
-        double va = val(ax, ay), vb = val(bx, by);
-        bool ina = va >= 0, inb = vb >= 0;
-        if (ina) {
-            next.push(ax, ay, at);
-            if (!inb) {
-                double t = va / (va - vb);
-                double ix = ax + t * (bx - ax), iy = ay + t * (by - ay);
-                if (axis == 0) ix = c; else iy = c;
-                next.push(ix, iy, own);
-            }
-        } else if (inb) {
-            double t = va / (va - vb);
-            double ix = ax + t * (bx - ax), iy = ay + t * (by - ay);
-            if (axis == 0) ix = c; else iy = c;
-            next.push(ix, iy, at);
+#ifdef __CUDACC__
+// Cuts the polygon q (m vertices; room for m + 1) in place to the half-plane
+// s (coord - c) >= 0, coord = x if axis == 0 else y; the new edge along the line
+// gets the id `own`.  Returns the new count.  The vertex after the one being
+// looked at is held in registers: what is written does not pass it, as each
+// vertex written in addition leaves the half-plane before one that is dropped.
+// (Where rounding crosses the line more often than twice, no more is written
+// than fits.)
+template <class P>
+__device__ __forceinline__ int axis_cut(const P &q, int m, int axis, double c, double s, int own) {
+    if (m == 0) return 0;
+    const double fx = q.X(0), fy = q.Y(0);
+    double ax = fx, ay = fy, va = s * ((axis == 0 ? ax : ay) - c);
+    int at = q.I(0), w = 0;
+    for (int k = 0; k < m; ++k) {
+        const bool more = k + 1 < m;
+        const double bx = more ? q.X(k + 1) : fx, by = more ? q.Y(k + 1) : fy;
+        const int bt = more ? q.I(k + 1) : 0;
+        const double vb = s * ((axis == 0 ? bx : by) - c);
+        const bool ina = va >= 0, inb = vb >= 0;
+        if (ina && w < q.cap) {
+            q.X(w) = ax;
+            q.Y(w) = ay;
+            q.I(w) = at;
+            ++w;
         }
-    }
-    SDOT_HDI void push(double x, double y, int tag) {
-        if (!has_first) {
-            has_first = true;
-            fx = x; fy = y; ft = tag;
-        } else {
-            edge(px, py, pt, x, y);
+        if (ina != inb && w < q.cap) {
+            const double t = va / (va - vb);
+            q.X(w) = axis == 0 ? c : ax + t * (bx - ax);
+            q.Y(w) = axis == 0 ? ay + t * (by - ay) : c;
+            q.I(w) = ina ? own : at;
+            ++w;
         }
-        px = x; py = y; pt = tag;
+        ax = bx;
+        ay = by;
+        at = bt;
+        va = vb;
     }
-    SDOT_HDI void finish() {
-        if (has_first) edge(px, py, pt, fx, fy);
-        next.finish();
-    }
-};
+    return w;
+}
 
 // Disc clipping restated from ConvexPolyhedron2::ball_cut
-// (ConvexPolyhedron2.tcc:534-666): each edge (P -> C) emits 0, 1 or 2
-// vertices (LINE keeps the edge's tag, ARC gets ID_ARC).  When nothing is
-// emitted, the result is the full disc unless the centre lies outside one
-// of the edges' half-planes (then it is empty).
-template <class Next>
-struct DiscClip {
-    Next &next;
-    double cx, cy, r;
-    int nin = 0, nout = 0;
-    bool center_out = false;
-    bool has_first = false;
-    double fx = 0, fy = 0;
-    int ft = 0;
-    double px = 0, py = 0;
-    int pt = 0;
-    SDOT_HDI DiscClip(Next &nx, double x, double y, double rr) : next(nx), cx(x), cy(y), r(rr) {}
-    SDOT_HDI double dist(double x, double y) const { return (x - cx) * (x - cx) + (y - cy) * (y - cy) - r * r; }
-    SDOT_HDI void unique_inter(double p0x, double p0y, double p1x, double p1y, double &ox, double &oy) const {
-        double dx = p1x - p0x, dy = p1y - p0y;
-        double a = dx * dx + dy * dy;
-        double b = (p0x - cx) * dx + (p0y - cy) * dy;
-        double c = (p0x - cx) * (p0x - cx) + (p0y - cy) * (p0y - cy) - r * r;
-        double d = sqrt(fmax(0.0, b * b - a * c));
-        double u = (-b + d) / a;
-        double v = (-b - d) / a;
+// (ConvexPolyhedron2.tcc:534-666): the edge a -> b of a polygon emits 0, 1 or 2
+// vertices of the clipped one (x, y, and whether an arc leaves it; else its
+// edge is the polygon's).  Returns their number.
+struct DiscEdge {
+    double x[2], y[2];
+    bool arc[2];
+};
+__device__ __forceinline__ int disc_edge(double ax, double ay, double bx, double by, double cx, double cy, double r,
+                                         DiscEdge &e) {
+    const double ux = ax - cx, uy = ay - cy, vx = bx - cx, vy = by - cy;
+    const double da = ux * ux + uy * uy - r * r, db = vx * vx + vy * vy - r * r;
+    e.x[0] = ax;
+    e.y[0] = ay;
+    e.arc[0] = e.arc[1] = false;
+    if (da <= 0 && db <= 0) return 1;
+    // the two crossings of the line: a + t (b - a), t = (-h -+ sqrt(h^2 - q c)) / q,
+    // taken from the end inside where one is
+    const bool from_b = da > 0 && db <= 0;
+    const double px = from_b ? bx : ax, py = from_b ? by : ay, dx = from_b ? ax - bx : bx - ax,
+                 dy = from_b ? ay - by : by - ay;
+    const double q = dx * dx + dy * dy;
+    const double h = (px - cx) * dx + (py - cy) * dy;
+    const double disc = h * h - q * (from_b ? db : da);
+    if (da <= 0 || db <= 0) {  // one crossing
+        const double d = sqrt(fmax(0.0, disc));
+        const double u = (-h + d) / q, v = (-h - d) / q;
         double t = fabs(u - 0.5) <= fabs(v - 0.5) ? u : v;
         t = fmin(1.0, fmax(0.0, t));
-        ox = p0x + t * dx;
-        oy = p0y + t * dy;
+        const int k = from_b ? 0 : 1;
+        e.x[k] = px + t * dx;
+        e.y[k] = py + t * dy;
+        e.arc[1] = true;
+        return k + 1;
     }
-    SDOT_HDI bool two_cuts(double p0x, double p0y, double p1x, double p1y, double &ax, double &ay, double &bx,
-                             double &by) const {
-        double dx = p1x - p0x, dy = p1y - p0y;
-        double a = dx * dx + dy * dy;
-        if (a == 0) return false;
-        double b = (p0x - cx) * dx + (p0y - cy) * dy;
-        double c = (p0x - cx) * (p0x - cx) + (p0y - cy) * (p0y - cy) - r * r;
-        double s = b * b - a * c;
-        if (s <= 0) return false;
-        double d = sqrt(s);
-        double u = (-b - d) / a;
-        double v = (-b + d) / a;
-        if (u > 0 && u < 1)
-            v = fmax(0.0, fmin(1.0, v));
-        else if (v > 0 && v < 1)
-            u = fmax(0.0, fmin(1.0, u));
-        else
-            return false;
-        ax = p0x + u * dx;
-        ay = p0y + u * dy;
-        bx = p0x + v * dx;
-        by = p0y + v * dy;
-        double a0 = atan2(ay - cy, ax - cx);
-        double a1 = atan2(by - cy, bx - cx);
-        return a0 != a1;
-    }
-    SDOT_HDI void emit(double x, double y, int tag) {
-        ++nout;
-        next.push(x, y, tag);
-    }
-    SDOT_HDI void edge(double ax, double ay, int at, double bx, double by) {
-        // outward normal of a counter-clockwise edge is (dy, -dx)
-        if ((cx - ax) * (by - ay) - (cy - ay) * (bx - ax) > 0) center_out = true;
-        double da = dist(ax, ay), db = dist(bx, by);
-        if (da <= 0) {
-            emit(ax, ay, at);
-            if (db > 0) {
-                double ix, iy;
-                unique_inter(ax, ay, bx, by, ix, iy);
-                emit(ix, iy, ID_ARC);
-            }
-        } else if (db <= 0) {
-            double ix, iy;
-            unique_inter(bx, by, ax, ay, ix, iy);
-            emit(ix, iy, at);
-        } else {
-            double qx, qy, sx, sy;
-            if (two_cuts(ax, ay, bx, by, qx, qy, sx, sy)) {
-                emit(qx, qy, at);
-                emit(sx, sy, ID_ARC);
-            }
-        }
-    }
-    SDOT_HDI void push(double x, double y, int tag) {
-        ++nin;
-        if (!has_first) {
-            has_first = true;
-            fx = x; fy = y; ft = tag;
-        } else {
-            edge(px, py, pt, x, y);
-        }
-        px = x; py = y; pt = tag;
-    }
-    SDOT_HDI void finish() {
-        if (has_first) edge(px, py, pt, fx, fy);
-        next.finish();
-    }
-    // radius of the result as the reference stores it: 0 if void, r otherwise
-    SDOT_HDI double result_radius() const {
-        if (nin == 0) return 0.0;
-        if (nout == 0 && center_out) return 0.0;
-        return r;
-    }
-};
-
-// Arc helpers restated from ConvexPolyhedron2::_arc_area / _centroid_arc /
-// _arc_length (ConvexPolyhedron2.tcc:2296-2381).
-SDOT_HD double arc_angles(double p0x, double p0y, double p1x, double p1y, double cx, double cy, double &a0) {
-    a0 = atan2(p0y - cy, p0x - cx);
-    double a1 = atan2(p1y - cy, p1x - cx);
-    if (a1 < a0) a1 += 2 * kPi;
-    return a1;
-}
-
-SDOT_HD double arc_area(double p0x, double p0y, double p1x, double p1y, double cx, double cy, double r) {
-    double a0;
-    double a1 = arc_angles(p0x, p0y, p1x, p1y, cx, cy, a0);
-    double ex = p0x - p1x, ey = p0y - p1y;
-    double d0 = sqrt(ex * ex + ey * ey) / 2;
-    double d1 = sqrt(fmax(0.0, r * r - d0 * d0));
-    double rs = r * r * (a1 - a0) / 2;
-    if (a1 - a0 > kPi)
-        rs += d1 * d0;
+    if (q == 0 || disc <= 0) return 0;
+    const double d = sqrt(disc);
+    double u = (-h - d) / q, v = (-h + d) / q;
+    if (u > 0 && u < 1)
+        v = fmax(0.0, fmin(1.0, v));
+    else if (v > 0 && v < 1)
+        u = fmax(0.0, fmin(1.0, u));
     else
-        rs -= d1 * d0;
-    return rs;
+        return 0;
+    e.x[0] = px + u * dx;
+    e.y[0] = py + u * dy;
+    e.x[1] = px + v * dx;
+    e.y[1] = py + v * dy;
+    e.arc[1] = true;
+    return atan2(e.y[0] - cy, e.x[0] - cx) != atan2(e.y[1] - cy, e.x[1] - cx) ? 2 : 0;
 }
 
-SDOT_HD void centroid_arc(double &ctx, double &cty, double &mea, double p0x, double p0y, double p1x, double p1y,
-                          double cx, double cy, double r, double coeff) {
+// Pushes the vertices of a polygon (m vertices; tag(k): the tag of edge k) to
+// sink.push(x, y, tag, closing), with BALL those of its intersection with the
+// disc (c, r), arcs tagged ID_ARC; with CLOSE the first one once more at the end
+// (closing).  One loop and one call of push, so that it is inlined once.
+// Returns the radius of the result as the reference stores it: r, 0 if void;
+// -1 without a disc.  A polygon that leaves no vertex stands for the full disc,
+// unless the centre lies outside one of its edges' half-planes.
+template <bool BALL, bool CLOSE, class P, class Tag, class S>
+__device__ __forceinline__ double stream_piece(const P &q, int m, const Tag &tag, double cx, double cy, double r, S &sink) {
+    int nout = 0, ft = 0;
+    bool center_out = false;
+    double fx = 0, fy = 0;
+    double ax = m > 0 ? q.X(0) : 0, ay = m > 0 ? q.Y(0) : 0;
+    const double qx = ax, qy = ay;
+    const int turns = m + (CLOSE ? 1 : 0);
+#pragma unroll 1
+    for (int k = 0; k < turns; ++k) {
+        DiscEdge e;
+        int cnt = 1, t = ft;
+        if (CLOSE && k == m) {
+            e.x[0] = fx;
+            e.y[0] = fy;
+            e.arc[0] = false;
+            if (!nout) cnt = 0;
+        } else {
+            const double bx = k + 1 < m ? q.X(k + 1) : qx, by = k + 1 < m ? q.Y(k + 1) : qy;
+            t = tag(k);
+            if (BALL) {
+                // outward normal of a counter-clockwise edge is (dy, -dx)
+                if ((cx - ax) * (by - ay) - (cy - ay) * (bx - ax) > 0) center_out = true;
+                cnt = disc_edge(ax, ay, bx, by, cx, cy, r, e);
+            } else {
+                e.x[0] = ax;
+                e.y[0] = ay;
+                e.arc[0] = false;
+            }
+            ax = bx;
+            ay = by;
+        }
+#pragma unroll 1
+        for (int o = 0; o < cnt; ++o) {
+            const double x = o ? e.x[1] : e.x[0], y = o ? e.y[1] : e.y[0];
+            const int g = (o ? e.arc[1] : e.arc[0]) ? ID_ARC : t;
+            const bool closing = CLOSE && k == m;
+            if (!nout) {
+                fx = x;
+                fy = y;
+                ft = g;
+            }
+            sink.push(x, y, g, closing);
+            ++nout;
+        }
+    }
+    if (!BALL) return -1.0;
+    return m == 0 || (nout == 0 && center_out) ? 0.0 : r;
+}
+
+// The segment of the disc (c, r) between the chord p0 -> p1 and the arc (area,
+// moments about the origin, angle of the arc), restated from
+// ConvexPolyhedron2::_arc_area / _centroid_arc / _arc_length
+// (ConvexPolyhedron2.tcc:2296-2381), which each take the angles anew.
+struct Arc {
+    double area, mx, my, angle;
+};
+__device__ __forceinline__ Arc arc_segment(double p0x, double p0y, double p1x, double p1y, double cx, double cy, double r) {
     p0x -= cx; p0y -= cy;
     p1x -= cx; p1y -= cy;
-    double a0 = atan2(p0y, p0x);
+    const double a0 = atan2(p0y, p0x);
     double a1 = atan2(p1y, p1x);
     if (a1 < a0) a1 += 2 * kPi;
-    double ex = p0x - p1x, ey = p0y - p1y;
-    double d0 = sqrt(ex * ex + ey * ey) / 2;
-    double d1 = sqrt(fmax(0.0, r * r - d0 * d0));
-    double tri_area = d1 * d0;
-    double tbx = (1.0 / 3.0) * (p0x + p1x), tby = (1.0 / 3.0) * (p0y + p1y);
-    double pie_area = r * r * (a1 - a0) / 2;
-    double f = 2.0 / 3.0 * (r * r * r) * sin((a1 - a0) / 2);
-    double pmx = f * cos((a1 + a0) / 2), pmy = f * sin((a1 + a0) / 2);
-    double lea;
-    if (a1 - a0 > kPi) {
-        ctx += coeff * (pmx + tri_area * tbx);
-        cty += coeff * (pmy + tri_area * tby);
-        lea = (pie_area + tri_area) * coeff;
-    } else {
-        ctx += coeff * (pmx - tri_area * tbx);
-        cty += coeff * (pmy - tri_area * tby);
-        lea = (pie_area - tri_area) * coeff;
-    }
-    ctx += lea * cx;
-    cty += lea * cy;
-    mea += lea;
+    const double ex = p0x - p1x, ey = p0y - p1y;
+    const double d0 = sqrt(ex * ex + ey * ey) / 2;
+    const double d1 = sqrt(fmax(0.0, r * r - d0 * d0));
+    const double sg = a1 - a0 > kPi ? 1.0 : -1.0;  // the triangle joins the pie or leaves it
+    const double tri = sg * d1 * d0, pie = r * r * (a1 - a0) / 2;
+    double sm, cm;
+    sincos((a1 + a0) / 2, &sm, &cm);
+    const double f = 2.0 / 3.0 * (r * r * r) * sin((a1 - a0) / 2);
+    Arc a;
+    a.angle = a1 - a0;
+    a.area = pie + tri;
+    a.mx = f * cm + tri * ((1.0 / 3.0) * (p0x + p1x)) + a.area * cx;
+    a.my = f * sm + tri * ((1.0 / 3.0) * (p0y + p1y)) + a.area * cy;
+    return a;
 }
+#endif
 
 }  // namespace sdot

@@ -13,11 +13,14 @@ from tests.test_gpu_parity_2d import check_all
 pytestmark = pytest.mark.gpu
 
 
-def pair(p, w, **kw):
+def pair(p, w, image=None, **kw):
     out = []
     for cls in (PowerDiagram, port.PortPowerDiagram):
         d = cls(p, w, **kw)
-        d.add_box_shape([0.0, 0.0], [1.0, 1.0])
+        if image is None:
+            d.add_box_shape([0.0, 0.0], [1.0, 1.0])
+        else:
+            d.set_image_density(image)
         out.append(d)
     return out
 
@@ -45,3 +48,16 @@ def test_walks_of_one_warp(gpu_lib, n):
     rng = np.random.default_rng(8200 + n)
     g, r = pair(rng.random((n, 2)), rng.uniform(-1.0, 1.0, n) / n)
     check_all(g, r, n, rtol_hess=1e-11)
+
+
+@pytest.mark.parametrize("n,res", [(1, (1, 1)), (3, (40, 7)), (40, (3, 5)), (300, (64, 64)), (2000, (5, 90))])
+@pytest.mark.parametrize("disc", [None, 0.2, 4.0])
+def test_pieces_of_pixels(gpu_lib, n, res, disc):
+    # pixels much larger and much smaller than the cells, cells cut by none to
+    # all four lines of a pixel, discs inside their cells and around them (the
+    # arcs' functions differ by a few ulp between device and host: 1e-11)
+    rng = np.random.default_rng(8300 + n)
+    w = rng.uniform(-0.1, 0.1, n) / n if disc is None else disc / n * rng.uniform(0.5, 2.0, n)
+    g, r = pair(rng.random((n, 2)), w, image=rng.uniform(0.5, 1.5, res),
+                radial_func="unit" if disc is None else "in_ball_w05")
+    check_all(g, r, n, rtol=1e-12 if disc is None else 1e-11, rtol_hess=1e-11)
