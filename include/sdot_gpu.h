@@ -109,7 +109,7 @@ int sdot_domain_measure(sdot_ctx *ctx, double *measure);
  * reference's traversal does (SpZGrid.tcc:558-561, :608-611); the image of
  * Dirac j under translation k has the cut id j + (k + 1) n in the neighbour
  * lists, and its Hessian entry goes to column j, the distance taken to the
- * image (get_der_integrals_wrt_weights.h:61-62).  count = 0 removes them.                                                                            */
+ * image (get_der_integrals_wrt_weights.h:61-62).  count = 0 removes them.   */
 int sdot_set_translations(sdot_ctx *ctx, const double *translations, int64_t count);
 
 /* ---- radial function ------------------------------------------------------
@@ -321,7 +321,8 @@ int sdot_evaluate(sdot_ctx *ctx);
 /* Device time in milliseconds of the last evaluation stages:
  * t[0] tree build, t[1] cell kernel, t[2] Hessian assembly.                  */
 int sdot_last_timings(const sdot_ctx *ctx, double *t3);
-/* Number of cells rebuilt by the large-capacity fallback in the last evaluation. */
+/* Number of cells rebuilt by the large-capacity fallback in the last evaluation
+ * (2D: of a diagram of more than 6,000 Diracs; smaller ones start there).      */
 int sdot_last_overflow_count(const sdot_ctx *ctx, int64_t *count);
 /* Number of kernels this library has launched in the process so far.
  * No reference counterpart (instrumentation).                               */

@@ -280,7 +280,7 @@ struct sdot_ctx {
     };
     DevStatus *dstat = nullptr, *hstat = nullptr;
     int *ovf_list = nullptr, *ovf_cnt = nullptr;
-    int *ovf_list2 = nullptr, *ovf_cnt2 = nullptr;  // 3D: third pass
+    int *ovf_list2 = nullptr, *ovf_cnt2 = nullptr;  // cells that overflow the second tier too
     unsigned char *hint3 = nullptr;                  // 3D: pass of each cell last time
     bool hint_valid = false;
     unsigned *err = nullptr;   // &dstat->err
@@ -381,9 +381,9 @@ struct sdot_ctx {
         err = &dstat->err;
         guard = dstat->guard;
         if (!hstat) SDOT_CUDA(cudaMallocHost(reinterpret_cast<void **>(&hstat), sizeof(DevStatus)));
+        dalloc(ovf_list2, ecap);
+        dalloc(ovf_cnt2, 1);
         if (dim == 3) {
-            dalloc(ovf_list2, ecap);
-            dalloc(ovf_cnt2, 1);
             dalloc(hint3, ecap);
             hint_valid = false;
         }
@@ -480,6 +480,8 @@ struct sdot_ctx {
         a.item_coeff = d_item_coeff;
         a.ovf_list = ovf_list;
         a.ovf_cnt = ovf_cnt;
+        a.ovf_list2 = ovf_list2;
+        a.ovf_cnt2 = ovf_cnt2;
         a.err = err;
         a.ntrans = int(trans_h.size() / 2);
         a.trans = d_trans;

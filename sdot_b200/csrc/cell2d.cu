@@ -46,7 +46,8 @@ static __device__ unsigned long long sdot_work[8];
 namespace {
 
 constexpr int STACK = 64;   // traversal stack (depth <= 17 levels, <= 3 pending siblings each)
-constexpr int WTIER_WARPS = 148 * 4;  // warps of the warp-per-cell tier (4 per SM; 8 or 16 measured no faster)
+constexpr int MID_WARPS = 148 * 16;   // warps of the warp tier in shared memory (16 per SM: 128 registers)
+constexpr int WTIER_WARPS = 148 * 4;  // warps of the warp tier in global scratch (few cells)
 
 // Records the first failed consistency guard and flags the error word; the
 // caller then skips the access.  Guards cover every index that comes from
@@ -488,8 +489,8 @@ struct Ring {
 // the eviction test holds for every vertex (SpZGrid.tcc:475-480), a leaf's
 // Diracs cut in index order (bisector SpZGrid.tcc:506-522).
 // The lanes run node tests together and cuts together: node steps go on until
-// at most WAIT lanes still look for a leaf while others hold one, then the
-// leaves are cut out of every cell that holds one.  (With one loop in which
+// at most WAIT of 32 lanes still look for a leaf while others hold one, then
+// the leaves are cut out of every cell that holds one.  (With one loop in which
 // each lane took whichever step its walk was at, every turn ran the node test,
 // the ordering of children, the cut test and the cut for some of the lanes:
 // 6.2 of 32 lanes active.)
@@ -550,7 +551,7 @@ __device__ int build_cell(const Cell2DArgs &A, long long s, bool live, Ring<CAP,
         while (true) {
             const bool want = !done && j >= je;
             const unsigned wm = __ballot_sync(FULL, want), hm = __ballot_sync(FULL, j < je);
-            if (!wm || (hm && __popc(wm) <= WAIT)) break;
+            if (!wm || (hm && 32 * __popc(wm) <= WAIT * A.lanes)) break;
             if (!want) continue;
             if (!has_top) {
                 if (!PER || sym + 1 >= A.ntrans) {
@@ -851,8 +852,8 @@ __global__ void __launch_bounds__(BS, fast_blocks(MODE, BALL)) k_cells2d(const C
     double *px = acc + (has_acc(MODE) ? CAP * BS : 0);
     int *sid = reinterpret_cast<int *>(px + (has_piece(MODE) ? 2 * PCAP * BS : 0));
     const PolyView<double> piece{px + t, px + PCAP * BS + t, sid + CAP * BS + t, BS, PCAP};
-    const long long s = blockIdx.x * (long long)BS + t;
-    const bool live = s < A.n;
+    const long long s = (blockIdx.x * (long long)BS + t) / 32 * A.lanes + (t & 31);
+    const bool live = (t & 31) < A.lanes && s < A.n;
     Ring<CAP, BS> cell;
     cell.x = smem + t;
     cell.y = smem + CAP * BS + t;
@@ -921,21 +922,35 @@ __device__ bool commit(const Rows &R, long long s, const int *col, const double 
     return true;
 }
 
-// Warp-per-cell build of one large cell (all lanes, same s): the walk of
-// build_cell, with the eviction test and the plane cuts spread over the
-// lanes, 32 vertices at a time.
+// The polygon of a warp's cell: contiguous, in coordinates about the Dirac.
+struct RelView {
+    PolyView<double> p;
+    double c0x, c0y;
+    int cap;
+    __device__ RelView(const PolyView<double> &q, double x, double y) : p(q), c0x(x), c0y(y), cap(q.cap) {}
+    __device__ double X(int k) const { return c0x + p.X(k); }
+    __device__ double Y(int k) const { return c0y + p.Y(k); }
+    __device__ int I(int k) const { return p.I(k); }
+};
+__device__ double rel_x(const RelView &cell, int k, double) { return cell.p.X(k); }
+__device__ double rel_y(const RelView &cell, int k, double) { return cell.p.Y(k); }
+
+// Warp-per-cell build of one cell (all lanes, same s): the walk of build_cell.
+// A popped box and a cut have the vertices spread over the lanes; when a box is
+// opened each of its children, and in a leaf each Dirac, is first tried by a
+// lane of its own against every vertex (polygons of at most 64), and only the
+// children that are needed now and the Diracs that cut go on, in their order:
+// most do not, and one after the other each waited for its reads.
 template <bool PER = false>
-__device__ int build_cell_coop(const Cell2DArgs &A, long long s, const PolyView<double> &cell, int cap, double c0x,
+__device__ int build_cell_warp(const Cell2DArgs &A, long long s, const PolyView<double> &cell, int cap, double c0x,
                                double c0y, double w0, int *wstack) {
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     int n = A.start_n;
-    if (lane == 0) {
-        for (int k = 0; k < n; ++k) {
-            cell.X(k) = A.start_xy[2 * k];
-            cell.Y(k) = A.start_xy[2 * k + 1];
-            cell.I(k) = domain_id(k);
-        }
+    for (int k = lane; k < n; k += 32) {
+        cell.X(k) = A.start_xy[2 * k] - c0x;
+        cell.Y(k) = A.start_xy[2 * k + 1] - c0y;
+        cell.I(k) = domain_id(k);
     }
     __syncwarp();
     int visits = 0;
@@ -943,6 +958,19 @@ __device__ int build_cell_coop(const Cell2DArgs &A, long long s, const PolyView<
     // (see build_cell)
     for (int sym = -1; sym < (PER ? A.ntrans : 0); ++sym) {
         const double tx = sym >= 0 ? A.trans[2 * sym] : 0.0, ty = sym >= 0 ? A.trans[2 * sym + 1] : 0.0;
+        // the box of a node about the Dirac, and whether vertex k needs it
+        struct Box {
+            double lo0, lo1, hi0, hi1, maxw;
+        };
+        auto box_of = [&](const TreeNode<2> &nd) {
+            return Box{(PER ? nd.lo[0] + tx : nd.lo[0]) - c0x, (PER ? nd.lo[1] + ty : nd.lo[1]) - c0y,
+                       (PER ? nd.hi[0] + tx : nd.hi[0]) - c0x, (PER ? nd.hi[1] + ty : nd.hi[1]) - c0y, nd.maxw};
+        };
+        auto fails = [&](const Box &b, int k) {
+            const double px = cell.X(k), py = cell.Y(k);
+            const double gx = gap(b.lo0, b.hi0, px), gy = gap(b.lo1, b.hi1, py);
+            return !(px * px + py * py - w0 <= gx * gx + gy * gy - b.maxw);
+        };
         if (lane == 0) wstack[0] = 0;
         __syncwarp();
         int sp = 1;
@@ -954,25 +982,10 @@ __device__ int build_cell_coop(const Cell2DArgs &A, long long s, const PolyView<
             const int node = wstack[--sp];
             __syncwarp();
             const TreeNode<2> nd = A.nodes[SDOT_CHECK_IDX(node, A.max_nodes, 4)];
-            const double lo0 = PER ? nd.lo[0] + tx : nd.lo[0], lo1 = PER ? nd.lo[1] + ty : nd.lo[1];
-            const double hi0 = PER ? nd.hi[0] + tx : nd.hi[0], hi1 = PER ? nd.hi[1] + ty : nd.hi[1];
+            const Box box = box_of(nd);
             bool need = false;
-            for (int base = 0; base < n; base += 32) {
-                const int k = base + lane;
-                bool fail = false;
-                if (k < n) {
-                    const double px = cell.X(k), py = cell.Y(k);
-                    const double qx = fmin(hi0, fmax(lo0, px));
-                    const double qy = fmin(hi1, fmax(lo1, py));
-                    const double lhs = (c0x - px) * (c0x - px) + (c0y - py) * (c0y - py) - w0;
-                    const double rhs = (qx - px) * (qx - px) + (qy - py) * (qy - py) - nd.maxw;
-                    fail = !(lhs <= rhs);
-                }
-                if (__any_sync(FULL, fail)) {
-                    need = true;
-                    break;
-                }
-            }
+            for (int base = 0; base < n && !need; base += 32)
+                need = __any_sync(FULL, base + lane < n && fails(box, base + lane));
             if (!need) continue;
             if (nd.b < 0) {
                 const int first = nd.a, nch = -nd.b;
@@ -984,29 +997,53 @@ __device__ int build_cell_coop(const Cell2DArgs &A, long long s, const PolyView<
                     if (lane == 0) flag_error(A.err, DE_STACK);
                     return -1;
                 }
-                int ch[4];
-                order_children<PER>(A, first, nch, c0x, c0y, tx, ty, ch);
-                if (lane == 0) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        if (c < nch) wstack[sp + c] = ch[c];
+                float key = -1;
+                bool keep = false;
+                if (lane < nch) {
+                    const TreeNode<2> &cn = A.nodes[first + lane];
+                    const double cx = 0.5 * (cn.lo[0] + cn.hi[0]), cy = 0.5 * (cn.lo[1] + cn.hi[1]);
+                    const double mx = c0x - (PER ? cx + tx : cx), my = c0y - (PER ? cy + ty : cy);
+                    key = float(mx * mx + my * my);
+                    const Box b = box_of(cn);
+                    keep = n > 64;
+                    for (int k = 0; k < n && !keep; ++k) keep = fails(b, k);
                 }
+                // farthest first (nearest popped first)
+                const unsigned km = __ballot_sync(FULL, keep);
+                int rank = 0;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float kc = __shfl_sync(FULL, key, c);
+                    rank += (km >> c & 1u) && (kc > key || (kc == key && c < lane));
+                }
+                if (keep) wstack[sp + rank] = first + lane;
+                sp += __popc(km);
                 __syncwarp();
-                sp += nch;
             } else {
                 if (nd.a < 0 || nd.b > A.n) {
                     if (lane == 0) guard_fail(A, 2, s, node);
                     return -2;
                 }
-                for (int j = nd.a; j < nd.b; ++j) {
-                    if (j == s && sym < 0) continue;
-                    const double c1x = PER ? A.pos[2 * j] + tx : A.pos[2 * j];
-                    const double c1y = PER ? A.pos[2 * j + 1] + ty : A.pos[2 * j + 1];
-                    const double w1 = A.w[j];
-                    double ox, oy, nx, ny;
-                    bisector(c0x, c0y, w0, c1x, c1y, w1, ox, oy, nx, ny);
-                    n = plane_cut_warp(cell, n, cap, ox, oy, nx, ny, PER ? j + (sym + 1) * int(A.n) : j, true);
-                    if (n <= 0) return n;
+                for (int j0 = nd.a; j0 < nd.b; j0 += 32) {
+                    // lane: Dirac j0 + lane, its bisector relative to c0
+                    const int j = j0 + lane;
+                    double ox = 0, oy = 0, nx = 0, ny = 0;
+                    bool cuts = false;
+                    if (j < nd.b && !(j == s && sym < 0)) {
+                        const double2 p = reinterpret_cast<const double2 *>(A.pos)[j];
+                        bisector(0.0, 0.0, w0, (PER ? p.x + tx : p.x) - c0x, (PER ? p.y + ty : p.y) - c0y, A.w[j], ox, oy,
+                                 nx, ny);
+                        cuts = n > 64;
+                        for (int k = 0; k < n && !cuts; ++k)
+                            cuts = (ox - cell.X(k)) * nx + (oy - cell.Y(k)) * ny < 0.0;
+                    }
+                    for (unsigned cm = __ballot_sync(FULL, cuts); cm; cm &= cm - 1) {
+                        const int l = __ffs(int(cm)) - 1;
+                        n = plane_cut_warp(cell, n, cap, __shfl_sync(FULL, ox, l), __shfl_sync(FULL, oy, l),
+                                           __shfl_sync(FULL, nx, l), __shfl_sync(FULL, ny, l),
+                                           PER ? j0 + l + (sym + 1) * int(A.n) : j0 + l, false);
+                        if (n <= 0) return n;
+                    }
                 }
             }
         }
@@ -1014,31 +1051,130 @@ __device__ int build_cell_coop(const Cell2DArgs &A, long long s, const PolyView<
     return n;
 }
 
-// Cells that overflowed the fast tier: one warp per cell, polygon of up to
-// CAP_HUGE_2D vertices in global scratch; lane 0 integrates the built cell.
-template <int MODE, bool BALL>
-__global__ void __launch_bounds__(128) k_cells2d_wtier(const Cell2DArgs A, double *scratch, int nwarps,
-                                                       const int *list, const int *list_cnt) {
-    constexpr int CAP = CAP_HUGE_2D;
+// finish_cell by a warp (single shapes without the disc clip): the lanes take
+// the edges.  Returns 0, 1 (a capacity was exceeded) or 2 (no room for the row).
+__device__ int finish_warp(const Cell2DArgs &A, long long s, const PolyView<double> &cell, int n) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const double c0x = A.pos[2 * s], c0y = A.pos[2 * s + 1];
+    if (n == -1) return 1;
+    const bool failed = n < 0;  // a failed guard: a NaN cell, not an overflow
+    if (failed) n = 0;
+    // a neighbour, or the image of Dirac j under translation k for an id j + (k + 1) n
+    auto site = [&](int id, int &j, double &x, double &y) {
+        const int k = int(id / A.n) - 1;
+        j = int(id % A.n);
+        x = A.pos[2 * j] + (k >= 0 ? A.trans[2 * k] : 0.0);
+        y = A.pos[2 * j + 1] + (k >= 0 ? A.trans[2 * k + 1] : 0.0);
+    };
+    int nrow = 0;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int id = k0 + lane < n ? cell.I(k0 + lane) : -1;
+        int j;
+        double x = c0x, y = c0y;
+        if (id >= 0) site(id, j, x, y);
+        const double dx = c0x - x, dy = c0y - y;
+        nrow += __popc(__ballot_sync(FULL, sqrt(dx * dx + dy * dy) != 0));
+    }
+    RowPut row(A.rows, s, nrow + 1), nb(A.nb, s, n);
+    if (!row.ok || !nb.ok) return 2;
+    double tr2 = 0, mx = 0, my = 0, mass = 0, der0 = 0;
+    const double ax = n > 0 ? cell.X(0) : 0, ay = n > 0 ? cell.Y(0) : 0;
+    int at = 0;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int k = k0 + lane;
+        bool entry = false;
+        int j = 0;
+        double v = 0;
+        if (k < n) {
+            const int k1 = k + 1 < n ? k + 1 : 0, id = cell.I(k);
+            const double bx = cell.X(k), by = cell.Y(k), cx = cell.X(k1), cy = cell.Y(k1);
+            if (id >= 0) {
+                double x, y;
+                site(id, j, x, y);
+                const double dx = c0x - x, dy = c0y - y, dist = sqrt(dx * dx + dy * dy);
+                entry = dist != 0;
+                v = entry ? 0.5 * (A.coeff * sqrt((cx - bx) * (cx - bx) + (cy - by) * (cy - by))) / dist : 0.0;
+                der0 += v;
+            }
+            nb.put(k, id, 0.0);
+            if (k >= 1 && k1) {  // triangle (0, k, k + 1)
+                const double t2 = ax * (by - cy) + bx * (cy - ay) + cx * (ay - by);
+                tr2 += t2;
+                const double lea = 0.5 * t2 * A.coeff;
+                mx += (1.0 / 3.0) * lea * (ax + bx + cx);
+                my += (1.0 / 3.0) * lea * (ay + by + cy);
+                mass += lea;
+            }
+        }
+        const unsigned em = __ballot_sync(FULL, entry);
+        if (entry) row.put(at + __popc(em & ((1u << lane) - 1u)), j, -v);
+        at += __popc(em);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        tr2 += __shfl_xor_sync(FULL, tr2, o);
+        mx += __shfl_xor_sync(FULL, mx, o);
+        my += __shfl_xor_sync(FULL, my, o);
+        mass += __shfl_xor_sync(FULL, mass, o);
+        der0 += __shfl_xor_sync(FULL, der0, o);
+    }
+    if (lane == 0) {
+        row.put(at, int(s), der0);
+        row.cnt = at + 1;
+        row.finish();
+        nb.finish();
+        const double none = nan("");
+        if (A.mass) A.mass[s] = failed ? none : A.coeff * (tr2 * 0.5);
+        if (A.mass_c) A.mass_c[s] = failed ? none : mass;
+        if (A.ctd) {
+            const double d = mass + (mass == 0);
+            A.ctd[2 * s] = failed ? none : (mx + c0x * mass) / d;
+            A.ctd[2 * s + 1] = failed ? none : (my + c0y * mass) / d;
+        }
+    }
+    return 0;
+}
+
+// Cells that overflowed the fast tier, one warp per cell: polygons of up to
+// CAP vertices in shared memory (MID), or in global scratch for those that
+// overflow that too.  The warp integrates a cell of a single shape; the disc
+// clip and the image and raster modes are done by lane 0.
+// 60,000 clustered Diracs: 8,700 cells pass 13 vertices while they are built (23
+// at most at their end).  With every polygon in global scratch, lane 0
+// integrating and one Dirac at a time, the cells took 3.1 ms at the starting
+// weights and 7.7 ms at the solved ones, now 1.4 and 3.8 ms.
+template <int MODE, bool BALL, bool MID>
+__global__ void __launch_bounds__(128, MID ? 4 : 1) k_cells2d_wtier(const Cell2DArgs A, double *scratch, int nwarps,
+                                                                    const int *list, const int *list_cnt,
+                                                                    int *next_list, int *next_cnt) {
+    constexpr int CAP = MID ? CAP_MID_2D : CAP_HUGE_2D;
+    extern __shared__ double wmem[];
     __shared__ int wstack[4][STACK];
     const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
     const int gw = blockIdx.x * 4 + wb;
     if (gw >= nwarps) return;
-    WarpScratch W(scratch + (long long)gw * warp_scratch_doubles(CAP), CAP);
-    const int cnt = *list_cnt;
+    WarpScratch W(MID ? wmem + wb * warp_scratch_doubles(CAP) : scratch + (long long)gw * warp_scratch_doubles(CAP), CAP);
+    const int cnt = list ? *list_cnt : int(A.n);
     for (int i = gw; i < cnt; i += nwarps) {
-        const long long s = list[i];
-        const int n = build_cell_coop<MODE == DM_PERIODIC>(A, s, W.cell, CAP, A.pos[2 * s], A.pos[2 * s + 1], A.w[s],
-                                                           wstack[wb]);
-        if (lane == 0) {
+        const long long s = list ? list[i] : i;
+        const double c0x = A.pos[2 * s], c0y = A.pos[2 * s + 1];
+        const int n = build_cell_warp<MODE == DM_PERIODIC>(A, s, W.cell, CAP, c0x, c0y, A.w[s], wstack[wb]);
+        int failed = 0;  // 1: a capacity was exceeded, 2: no room for the row
+        if constexpr ((MODE == DM_SINGLE || MODE == DM_PERIODIC) && !BALL) {
+            failed = finish_warp(A, s, W.cell, n);
+        } else if (lane == 0) {
             Out row(A.rows.cnt ? W.row_col : nullptr, W.row_val, 1, CAP + 1);
             Out nbo(A.nb.cnt ? W.nb_id : nullptr, nullptr, 1, 2 * CAP);
-            const bool built = finish_cell<MODE, BALL>(A, s, W.cell, n, W.acc, 1, row, nbo, W.piece);
-            bool ok = built;
-            if (ok && A.rows.cnt) ok = commit(A.rows, s, W.row_col, W.row_val, 1, row.cnt);
-            if (ok && A.nb.cnt) ok = commit(A.nb, s, W.nb_id, nullptr, 1, nbo.cnt);
-            if (!ok) {
-                atomicOr(A.err, built ? DE_SIDE : DE_CAPACITY);
+            if (!finish_cell<MODE, BALL>(A, s, RelView(W.cell, c0x, c0y), n, W.acc, 1, row, nbo, W.piece)) failed = 1;
+            if (!failed && A.rows.cnt && !commit(A.rows, s, W.row_col, W.row_val, 1, row.cnt)) failed = 2;
+            if (!failed && A.nb.cnt && !commit(A.nb, s, W.nb_id, nullptr, 1, nbo.cnt)) failed = 2;
+        }
+        if (lane == 0 && failed) {
+            if (MID && failed == 1) {
+                const int k = atomicAdd(next_cnt, 1);
+                if (k < A.n) next_list[k] = int(s);  // as push_overflow
+            } else {
+                atomicOr(A.err, failed == 2 ? DE_SIDE : DE_CAPACITY);
                 if (A.mass) A.mass[s] = nan("");
                 if (A.rows.cnt) A.rows.cnt[s] = 0;
                 if (A.nb.cnt) A.nb.cnt[s] = 0;
@@ -1059,9 +1195,21 @@ __global__ void k_all_cells(int *list, int *cnt, long long n) {
 // Counters the fast kernel appends to: zeroed before every launch of it.
 void reset_overflow(const Cell2DArgs &a, cudaStream_t st) {
     SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt, 0, sizeof(int), st));
+    SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt2, 0, sizeof(int), st));
     if (a.rows.side_used) SDOT_CUDA(cudaMemsetAsync(a.rows.side_used, 0, sizeof(unsigned long long), st));
     if (a.nb.side_used) SDOT_CUDA(cudaMemsetAsync(a.nb.side_used, 0, sizeof(unsigned long long), st));
 }
+
+// Up to this many Diracs a cell gets a warp from the start (single shapes
+// without the disc clip, whose cells a warp integrates): the walk of one thread
+// takes 100 to 200 us whatever their number.  Cells of 1,000 / 3,000 / 10,000
+// uniform Diracs: 150 / 190 / 203 us by threads, 62 / 94 / 199 us by warps (whose
+// 15 ns per cell lose to 2 ns beyond).
+constexpr long long WARP_CELLS = 6000;
+// Cells per warp of the fast tier: where there are too few warps to fill the
+// device, fewer cells per warp end sooner (10,000 Diracs: 201 -> 182 us with 12;
+// 30,000: 283 -> 291).
+int warp_lanes(long long n) { return n <= 16384 ? 12 : 32; }
 
 template <int MODE, bool BALL>
 void launch_all(const Cell2DArgs &a, void *scratch, cudaStream_t st) {
@@ -1071,24 +1219,32 @@ void launch_all(const Cell2DArgs &a, void *scratch, cudaStream_t st) {
         // faster than 72%, which holds ten)
         SDOT_CUDA(cudaFuncSetAttribute(k_cells2d<MODE, BALL>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     });
-    if (a.start_n > CAP_FAST_2D) {
-        // the starting polygon alone overflows the fast tier: every cell is
-        // built by the warp tier (polygons of up to CAP_HUGE_2D vertices)
-        reset_overflow(a, st);
+    reset_overflow(a, st);
+    constexpr bool BY_WARP = (MODE == DM_SINGLE || MODE == DM_PERIODIC) && !BALL;
+    const int *list = a.ovf_list, *cnt = a.ovf_cnt;
+    if (BY_WARP && a.start_n <= CAP_FAST_2D && a.n <= WARP_CELLS) {
+        list = cnt = nullptr;  // every cell
+    } else if (a.start_n <= CAP_FAST_2D) {
+        Cell2DArgs b = a;
+        b.lanes = warp_lanes(a.n);
+        k_cells2d<MODE, BALL><<<ceil_div(ceil_div(a.n, b.lanes), BS / 32), BS, fast_smem<MODE>(), st>>>(b);
+        note_launch();
+    } else {
+        // the starting polygon alone overflows the fast tier
         k_all_cells<<<ceil_div(a.n, 256), 256, 0, st>>>(a.ovf_list, a.ovf_cnt, a.n);
         note_launch();
-        k_cells2d_wtier<MODE, BALL><<<WTIER_WARPS / 4, 128, 0, st>>>(a, static_cast<double *>(scratch), WTIER_WARPS,
-                                                                      a.ovf_list, a.ovf_cnt);
-        note_launch();
-        SDOT_CUDA(cudaGetLastError());
-        return;
     }
-    reset_overflow(a, st);
-    k_cells2d<MODE, BALL><<<ceil_div(a.n, BS), BS, fast_smem<MODE>(), st>>>(a);
-    note_launch();
-    SDOT_CUDA(cudaGetLastError());
-    k_cells2d_wtier<MODE, BALL><<<WTIER_WARPS / 4, 128, 0, st>>>(a, static_cast<double *>(scratch), WTIER_WARPS,
-                                                                  a.ovf_list, a.ovf_cnt);
+    // a starting polygon that nearly fills the warps' shared memory goes on to
+    // the last tier at once
+    const bool mid = a.start_n <= CAP_MID_2D - 16;
+    if (mid) {
+        k_cells2d_wtier<MODE, BALL, true><<<MID_WARPS / 4, 128, 4 * warp_scratch_doubles(CAP_MID_2D) * sizeof(double),
+                                            st>>>(a, nullptr, MID_WARPS, list, cnt, a.ovf_list2, a.ovf_cnt2);
+        note_launch();
+    }
+    k_cells2d_wtier<MODE, BALL, false><<<WTIER_WARPS / 4, 128, 0, st>>>(
+        a, static_cast<double *>(scratch), WTIER_WARPS, mid ? a.ovf_list2 : a.ovf_list, mid ? a.ovf_cnt2 : a.ovf_cnt,
+        nullptr, nullptr);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
 }

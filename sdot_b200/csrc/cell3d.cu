@@ -387,39 +387,6 @@ __device__ void guard_fail3(const Cell3DArgs &A, int code, long long s, long lon
     flag_error(A.err, DE_GUARD);
 }
 
-// Destination of one row of cnt entries: its ELL slots, or a place in the side
-// buffer for a long row (called by the whole warp; ok: false when the side
-// buffer is full).  Rows that are not wanted (R.cnt null) are skipped.
-struct RowPut {
-    const Rows &R;
-    long long s, off = 0;
-    int cnt;
-    bool side, ok = true;
-    __device__ RowPut(const Rows &r, long long s_, int c) : R(r), s(s_), cnt(c), side(r.cnt && c > r.cap) {
-        if (!side) return;
-        unsigned long long o = 0;
-        if ((threadIdx.x & 31) == 0) o = atomicAdd(R.side_used, (unsigned long long)cnt);
-        o = __shfl_sync(FULL, o, 0);
-        off = (long long)o;
-        ok = off + cnt <= R.side_cap;
-    }
-    __device__ void put(int k, int c, double v) const {
-        if (!R.cnt || !ok) return;
-        if (side) {
-            R.side_col[off + k] = c;
-            if (R.side_val) R.side_val[off + k] = v;
-        } else {
-            R.col[k * R.stride + s] = c;
-            if (R.val) R.val[k * R.stride + s] = v;
-        }
-    }
-    __device__ void finish() const {  // one lane
-        if (!R.cnt) return;
-        if (side) R.side[s] = off;
-        R.cnt[s] = cnt;
-    }
-};
-
 // The outputs of a cell that could not be built.
 __device__ void fail_cell(const Cell3DArgs &A, long long s) {
     if (A.mass) A.mass[s] = nan("");

@@ -41,13 +41,29 @@ def test_edges_of_one_cell(gpu_lib, k, precision):
     check_all(g, r, k + 1, rtol_hess=1e-11)
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 127, 129, 1025])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 127, 129, 1025, 6000, 6001, 16384, 16386, 16417])
 def test_walks_of_one_warp(gpu_lib, n):
     # lanes whose walks end far apart: weights that empty some cells and make
-    # others reach over many, and a last warp of a few lanes
+    # others reach over many, and a last warp of a few lanes; a warp per cell up
+    # to 6,000 Diracs, warps of 12 cells up to 16,384
     rng = np.random.default_rng(8200 + n)
     g, r = pair(rng.random((n, 2)), rng.uniform(-1.0, 1.0, n) / n)
     check_all(g, r, n, rtol_hess=1e-11)
+
+
+@pytest.mark.parametrize("k", [13, 47, 48, 49, 63, 64, 65, 200])
+def test_large_cells_among_many(gpu_lib, k):
+    # cells past the fast tier in a diagram that starts there, around the
+    # capacity of the warps' shared memory: a ring of k Diracs about one in the
+    # middle of 7,000 others, which are kept out of the ring
+    rng = np.random.default_rng(8400 + k)
+    q = rng.random((12000, 2))
+    q = q[np.hypot(q[:, 0] - 0.5, q[:, 1] - 0.5) > 0.35][:7000]
+    a = np.arange(k) * 2 * np.pi / k + rng.uniform(-0.2, 0.2, k) / k
+    d = 0.25 * rng.uniform(0.9999, 1.0001, k)
+    p = np.concatenate([q, 0.5 + d[:, None] * np.stack([np.cos(a), np.sin(a)], 1), [[0.5, 0.5]]])
+    g, r = pair(p, np.zeros(len(p)))
+    check_all(g, r, len(p), rtol_hess=1e-11)
 
 
 @pytest.mark.parametrize("n,res", [(1, (1, 1)), (3, (40, 7)), (40, (3, 5)), (300, (64, 64)), (2000, (5, 90))])
