@@ -68,7 +68,7 @@ template <int VB, int MAXP>
 struct Work3 {
     unsigned out[VB];                    // the vertices outside a cut
     unsigned rm[MAXP / 32], hm[MAXP / 32];  // faces of the removed vertices, faces that are cut through
-    int first[MAXP];                     // lowest vertex of each face
+    int first[MAXP];                     // where the polygon of each face begins
     unsigned short ta[MAXP], tb[MAXP];   // new vertex with this face second, third
     unsigned short req[MAXP];            // edges to cut: vertex outside | edge << 10
     unsigned short list[MAXP];           // faces in slot order
@@ -399,9 +399,12 @@ __device__ void fail_cell(const Cell3DArgs &A, long long s) {
     if (A.nb.cnt) A.nb.cnt[s] = 0;
 }
 
-// The faces of the cell in slot order into W.list, and the lowest vertex of
-// each into W.first; returns their number, or -1 where the numbers of faces
-// and vertices are not those of a polyhedron (V = 2 F - 4).
+// The faces of the cell in slot order into W.list, and for each the vertex its
+// polygon is taken from into W.first (below the vertex, the slot of the face
+// after it: the one with the lowest such slot, which does not depend on where
+// the pass keeps its vertices, so that every pass sums alike); returns the
+// number of faces, or -1 where the numbers of faces and vertices are not those
+// of a polyhedron (V = 2 F - 4).
 template <int VB, int MAXP>
 __device__ __forceinline__ int list_faces(const Cell3<VB, MAXP> &C, Work3<VB, MAXP> &W, int nr) {
     const int lane = threadIdx.x & 31;
@@ -409,7 +412,7 @@ __device__ __forceinline__ int list_faces(const Cell3<VB, MAXP> &C, Work3<VB, MA
 #pragma unroll
     for (int w = 0; w < MAXP / 32; ++w) {
         const unsigned lw = C.live[w];
-        W.first[32 * w + lane] = 32 * VB;
+        W.first[32 * w + lane] = 1 << 30;
         if (lw >> lane & 1u) W.list[nf + __popc(lw & ((1u << lane) - 1u))] = (unsigned short)(32 * w + lane);
         nf += __popc(lw);
     }
@@ -419,19 +422,22 @@ __device__ __forceinline__ int list_faces(const Cell3<VB, MAXP> &C, Work3<VB, MA
         nv += __popc(al);
         if (al >> lane & 1u)
 #pragma unroll
-            for (int i = 0; i < 3; ++i) atomicMin(&W.first[C.fp[i][lane + 32 * r]], lane + 32 * r);
+            for (int i = 0; i < 3; ++i) {
+                const int v = lane + 32 * r;
+                atomicMin(&W.first[C.fp[i][v]], int(C.fp[i == 2 ? 0 : i + 1][v]) << 10 | v);
+            }
     }
     __syncwarp();
     return nv == (nf ? 2 * nf - 4 : 0) ? nf : -1;
 }
 
 // Walks the polygon of face f counter-clockwise and calls tri(x0, y0, z0, e1,
-// e2) for the triangles of its fan from the lowest vertex (e1, e2 from that
+// e2) for the triangles of its fan from its first vertex (e1, e2 from that
 // vertex).  At most 32 VB steps; false where the walk does not close.
 template <int VB, int MAXP, class F>
 __device__ __forceinline__ bool walk_face(const Cell3<VB, MAXP> &C, const Work3<VB, MAXP> &W, int f, F &&tri) {
-    const int v0 = W.first[f];
-    if (v0 >= 32 * VB) return false;
+    if (W.first[f] >= 1 << 30) return false;
+    const int v0 = W.first[f] & 1023;
     const double x0 = C.x[v0], y0 = C.y[v0], z0 = C.z[v0];
     auto step = [&](int v) { return int(C.fp[0][v] == f ? C.nb[1][v] : C.fp[1][v] == f ? C.nb[2][v] : C.nb[0][v]); };
     int v = step(v0);
