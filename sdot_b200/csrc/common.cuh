@@ -143,6 +143,34 @@ __host__ __device__ inline void flag_error(unsigned *word, unsigned bits) {
 }
 
 #ifdef __CUDACC__
+// (Cooperative launches: every block is resident.  sync: two words, zeroed
+// before the launch: the arrivals, and a mark that a wait was given up.)
+// Waits for every block of the grid; false when the wait was given up (by any
+// block).  target counts the arrivals expected so far.  The release and the
+// acquire, with the block's own barriers around them, order the plain reads and
+// writes of all threads (and drop what the L1 cache holds of other blocks').
+__device__ inline bool grid_barrier(unsigned *sync, unsigned &target) {
+    __shared__ int ok;
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sync[0]) : "memory");
+        ok = 0;
+        for (unsigned k = 0; k < (1u << 24); ++k) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&sync[0]) : "memory");
+            if (int(v - target) >= 0) {
+                ok = 1;
+                break;
+            }
+            if ((k & 1023u) == 1023u && *(volatile unsigned *)&sync[1]) break;
+        }
+        if (!ok) atomicExch(&sync[1], 1u);
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
 // The distance of p from [lo, hi] (the signs read as integers: an FP64
 // minimum and maximum take several times the instructions).
 __device__ __forceinline__ double gap(double lo, double hi, double p) {

@@ -19,9 +19,11 @@ void scan_exclusive_total(const T *in, T *out, long long n, void *tmp, cudaStrea
 // ---------------------------------------------------------- radix sort ----
 // Sorts keys ascending, carrying values, stable.  `bits` is the number of
 // significant key bits (passes = ceil(bits / 8)).  Result ends in
-// (keys_out, vals_out); the *_alt buffers are scratch of n items each.
-size_t radix_tmp_size(long long n);
+// (keys_out, vals_out); the *_alt buffers are scratch of n items each, tmp of
+// radix_tmp_size() bytes, sync two words zeroed before the call.
+size_t radix_tmp_size();
 void radix_sort_pairs(const unsigned *keys_in, const unsigned *vals_in, unsigned *keys_out, unsigned *vals_out,
-                      unsigned *keys_alt, unsigned *vals_alt, long long n, int bits, void *tmp, cudaStream_t st);
+                      unsigned *keys_alt, unsigned *vals_alt, long long n, int bits, void *tmp, unsigned *sync,
+                      cudaStream_t st);
 
 }  // namespace sdot

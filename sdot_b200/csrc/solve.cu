@@ -706,32 +706,6 @@ __device__ double grid_sum(const double *partial, double *sh) {
     return a;
 }
 
-// Waits for every block of the grid; false when the wait was given up (by any
-// block).  target counts the arrivals expected so far.  The release and the
-// acquire, with the block's own barriers around them, order the plain reads and
-// writes of all threads (and drop what the L1 cache holds of other blocks').
-__device__ bool grid_barrier(unsigned *sync, unsigned &target) {
-    __shared__ int ok;
-    __syncthreads();
-    target += gridDim.x;
-    if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sync[0]) : "memory");
-        ok = 0;
-        for (unsigned k = 0; k < (1u << 24); ++k) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&sync[0]) : "memory");
-            if (int(v - target) >= 0) {
-                ok = 1;
-                break;
-            }
-            if ((k & 1023u) == 1023u && *(volatile unsigned *)&sync[1]) break;
-        }
-        if (!ok) atomicExch(&sync[1], 1u);
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
 // r - A z of row i with z_j = f(j); the aggregate's sum of it to rc (whole
 // warps call this: rows past n give 0)
 template <int B>

@@ -17,15 +17,6 @@ __device__ __forceinline__ double from_ord_bits(unsigned long long b) {
 }
 
 template <int D>
-__global__ void k_bbox_init(unsigned long long *bits) {
-    int t = threadIdx.x;
-    if (t < D) {
-        bits[t] = ~0ull;
-        bits[D + t] = 0ull;
-    }
-}
-
-template <int D>
 __global__ void k_bbox(const double *pos, long long n, unsigned long long *bits) {
     __shared__ unsigned long long smin[D], smax[D];
     if (threadIdx.x < D) {
@@ -53,12 +44,6 @@ __global__ void k_bbox(const double *pos, long long n, unsigned long long *bits)
     }
 }
 
-template <int D>
-__global__ void k_bbox_final(const unsigned long long *bits, double *bbox) {
-    int t = threadIdx.x;
-    if (t < 2 * D) bbox[t] = from_ord_bits(bits[t]);
-}
-
 __device__ __forceinline__ unsigned spread2(unsigned v) {  // 16 bits -> even bits
     v &= 0xffffu;
     v = (v | (v << 8)) & 0x00ff00ffu;
@@ -77,13 +62,14 @@ __device__ __forceinline__ unsigned spread3(unsigned v) {  // 10 bits -> every t
 }
 
 template <int D>
-__global__ void k_morton(const double *pos, long long n, const double *bbox, int bits, unsigned *keys, unsigned *vals) {
+__global__ void k_morton(const double *pos, long long n, const unsigned long long *bbox, int bits, unsigned *keys,
+                         unsigned *vals) {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double top = double((1u << bits) - 1u);
     unsigned q[D];
     for (int d = 0; d < D; ++d) {
-        double lo = bbox[d], hi = bbox[D + d];
+        const double lo = from_ord_bits(bbox[d]), hi = from_ord_bits(bbox[D + d]);
         double ext = hi - lo;
         double t = ext > 0 ? (pos[D * i + d] - lo) / ext * double(1u << bits) : 0.0;
         t = fmin(fmax(t, 0.0), top);
@@ -110,134 +96,240 @@ __global__ void k_gather(const double *pos, const double *w, const unsigned *ord
     inv[i] = int(s);
 }
 
-template <int D>
-__global__ void k_gather_w(const double *w, const int *idx, long long n, double *w_s) {
-    long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    w_s[s] = w[idx[s]];
-}
-
-template <int D>
-__global__ void k_tree_init(TreeNode<D> *nodes, int *level, int *counters, int npass, long long n) {
-    nodes[0].a = 0;
-    nodes[0].b = int(n);
-    level[0] = 0;
-    counters[0] = 1;
-    counters[1] = 0;
-    counters[2] = 1;
-    for (int p = 3; p < npass + 3; ++p) counters[p] = 1;
-}
-
-// First index of [lo, hi) whose key is >= v, found by the 32 lanes of a warp
-// together (every lane gets it): each round probes 32 evenly spaced keys and
-// keeps the stretch between the last one below v and the next, so a range of
-// r keys takes about log32(r) dependent reads instead of log2(r).
-__device__ __forceinline__ int warp_lower_bound(const unsigned *keys, int lo, int hi, unsigned long long v) {
+// First indices of [a, b) whose keys are >= v + (c << shift), c = 1 .. C - 1,
+// into st[c] (st[0] = a, st[C] = b), found by the 32 lanes of a warp together
+// (every lane gets them): each round probes 32 evenly spaced keys of every
+// stretch and keeps the part between the last one below and the next, so a range
+// of r keys takes about log32(r) dependent reads, those of the C - 1 searches at
+// once.
+template <int C>
+__device__ __forceinline__ void warp_bounds(const unsigned *keys, int a, int b, unsigned long long v, int shift, int *st) {
     const int lane = threadIdx.x & 31;
-    while (hi - lo > 32) {
-        const int step = (hi - lo + 31) / 32;
-        const int i = lo + lane * step;
-        const bool below = i < hi && (unsigned long long)keys[i] < v;
-        const int cnt = __popc(__ballot_sync(0xffffffffu, below));  // probes 0 .. cnt - 1 are below v
-        if (cnt == 0) return lo;
-        const int nlo = lo + (cnt - 1) * step + 1;
-        const int nhi = lo + cnt * step;
-        lo = nlo;
-        if (nhi < hi) hi = nhi;
+    int lo[C], hi[C];
+#pragma unroll
+    for (int c = 1; c < C; ++c) {
+        lo[c] = a;
+        hi[c] = b;
     }
-    const int i = lo + lane;
-    const bool below = i < hi && (unsigned long long)keys[i] < v;
-    return lo + __popc(__ballot_sync(0xffffffffu, below));
+    for (bool last = false; !last;) {
+        last = true;
+        unsigned k[C];
+        int step[C];
+#pragma unroll
+        for (int c = 1; c < C; ++c) {
+            step[c] = hi[c] - lo[c] > 32 ? (hi[c] - lo[c] + 31) / 32 : 1;
+            last &= step[c] == 1;
+            const int i = lo[c] + lane * step[c];
+            k[c] = i < hi[c] ? keys[i] : 0u;
+        }
+#pragma unroll
+        for (int c = 1; c < C; ++c) {
+            const int i = lo[c] + lane * step[c];
+            const bool below = i < hi[c] && (unsigned long long)k[c] < v + ((unsigned long long)c << shift);
+            const int cnt = __popc(__ballot_sync(0xffffffffu, below));  // probes 0 .. cnt - 1 are below
+            if (step[c] == 1) {
+                lo[c] += cnt;
+                hi[c] = lo[c];
+            } else if (cnt == 0) {
+                hi[c] = lo[c];
+            } else {
+                const int nhi = lo[c] + cnt * step[c];
+                lo[c] += (cnt - 1) * step[c] + 1;
+                if (nhi < hi[c]) hi[c] = nhi;
+            }
+        }
+    }
+    st[0] = a;
+    st[C] = b;
+#pragma unroll
+    for (int c = 1; c < C; ++c) st[c] = lo[c];
 }
 
-// One level of the top-down split, one warp per node of the level: the node's
-// key range is cut at the 2^D child prefixes of its next Morton level (single-
-// child levels skipped); children are appended at the node counter.
 template <int D>
-__global__ void k_split(TreeNode<D> *nodes, int *level, int *counters, int pass, const unsigned *keys, int bits,
-                        int max_per_leaf, int max_nodes) {
-    const int beg = counters[1 + pass], end = counters[2 + pass];
+struct TreeArgs {
+    TreeNode<D> *nodes;
+    int *level, *counters;   // counters: see DeviceTree
+    const unsigned *keys;
+    const double *pos;
+    double *w;
+    const double *w_orig;    // refresh: the new weights, caller order
+    const int *idx;
+    long long n;
+    int bits, max_per_leaf, max_nodes, npass;
+    unsigned *sync;
+};
+
+// Levels of the tree, in one cooperative kernel of blocks of 1024.  BUILD: the
+// top-down split, level by level, one warp per node: its key range is cut at the
+// 2^D child prefixes of its next Morton level (single-child levels skipped), the
+// children are appended to the next level; then boxes and maximum weights
+// bottom-up, the leaves of all levels at once.  Otherwise (new weights): the
+// weights gathered, and the maximum weights bottom-up.
+// As launches, a level was one kernel to split, one to note the count and one to
+// reduce, for the 17 levels a key has and not the 6 to 11 of a tree: 51 launches,
+// 170 us of the 230 of a build of 10,000 Diracs and 345 of 450 us at 1M; the
+// refresh 17 launches, 54 us.
+constexpr int TREE_TB = 1024;
+template <int D, bool BUILD>
+__global__ void __launch_bounds__(TREE_TB, 1) k_tree(const TreeArgs<D> A) {
     constexpr int C = 1 << D;
     const int lane = threadIdx.x & 31;
-    const int warp = int((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
-    const int nwarps = int((gridDim.x * (long long)blockDim.x) >> 5);
-    for (int node = beg + warp; node < end; node += nwarps) {
-        int a = nodes[node].a, b = nodes[node].b, L = level[node];
-        while (true) {
-            if (b - a <= max_per_leaf || L >= bits) break;  // leaf
-            int shift = D * (bits - L - 1);
-            unsigned long long prefix = (unsigned long long)keys[a] >> (shift + D);
-            int st[C + 1];
-            st[0] = a;
-            st[C] = b;
-            for (int c = 1; c < C; ++c)
-                st[c] = warp_lower_bound(keys, st[c - 1], b, ((prefix << D) | (unsigned long long)c) << shift);
-            int ne = 0;
-            for (int c = 0; c < C; ++c) ne += st[c + 1] > st[c];
-            if (ne == 1) {
-                ++L;
-                continue;
-            }
-            int first = 0;
-            if (lane == 0) first = atomicAdd(&counters[0], ne);
-            first = __shfl_sync(0xffffffffu, first, 0);
-            if (first + ne > max_nodes) break;  // cannot happen: nodes <= 2n
-            if (lane == 0) {
-                int k = 0;
-                for (int c = 0; c < C; ++c) {
-                    if (st[c + 1] > st[c]) {
-                        nodes[first + k].a = st[c];
-                        nodes[first + k].b = st[c + 1];
-                        level[first + k] = L + 1;
-                        ++k;
+    const int warp = int((blockIdx.x * TREE_TB + threadIdx.x) >> 5), nwarps = int(gridDim.x * TREE_TB >> 5);
+    const int thread = blockIdx.x * TREE_TB + threadIdx.x, nthreads = gridDim.x * TREE_TB;
+    int *const start = A.counters + 1, *const added = A.counters + A.npass + 4;
+    unsigned target = 0;
+    int depth = 0;  // levels in use
+    if (BUILD) {
+        // nodes [beg, end) are the level's; added[p]: how many it gives the next
+        int beg = 0, end = 1;
+        for (int p = 0; p < A.npass && beg < end; ++p) {
+            for (int node = beg + warp; node < end; node += nwarps) {
+                const int a = A.nodes[node].a, b = A.nodes[node].b;
+                int L = A.level[node];
+                while (b - a > A.max_per_leaf && L < A.bits) {
+                    const int shift = D * (A.bits - L - 1);
+                    const unsigned long long prefix = (unsigned long long)A.keys[a] >> (shift + D);
+                    int st[C + 1];
+                    warp_bounds<C>(A.keys, a, b, (prefix << D) << shift, shift, st);
+                    int ne = 0;
+#pragma unroll
+                    for (int c = 0; c < C; ++c) ne += st[c + 1] > st[c];
+                    ++L;
+                    if (ne == 1) continue;
+                    int first = 0;
+                    if (lane == 0) first = end + atomicAdd(&added[p], ne);
+                    first = __shfl_sync(0xffffffffu, first, 0);
+                    if (first + ne > A.max_nodes) break;  // cannot happen: nodes <= 2n
+                    if (lane == 0) {
+                        int k = first;
+#pragma unroll
+                        for (int c = 0; c < C; ++c)
+                            if (st[c + 1] > st[c]) {
+                                A.nodes[k].a = st[c];
+                                A.nodes[k].b = st[c + 1];
+                                A.level[k] = L;
+                                ++k;
+                            }
+                        A.nodes[node].a = first;
+                        A.nodes[node].b = -ne;
                     }
+                    break;
                 }
-                nodes[node].a = first;
-                nodes[node].b = -ne;
             }
-            break;
+            if (!grid_barrier(A.sync, target)) {
+                A.nodes[0].a = -1;  // the walks' guard reports it
+                A.nodes[0].b = 1;
+                return;
+            }
+            depth = p + 1;
+            beg = end;
+            end += added[p];
+            if (thread == 0) start[p + 1] = beg;
         }
-        if (lane == 0) level[node] = L;
+        if (thread == 0)
+            for (int p = depth; p <= A.npass; ++p) start[p] = p == 0 ? 0 : beg;
+    } else {
+        while (depth < A.npass && start[depth] < start[depth + 1]) ++depth;
+        for (long long s = thread; s < A.n; s += nthreads) A.w[s] = A.w_orig[A.idx[s]];
+        if (!grid_barrier(A.sync, target)) {
+            A.nodes[0].a = -1;
+            A.nodes[0].b = 1;
+            return;
+        }
     }
-}
-
-__global__ void k_mark_pass(int *counters, int pass) { counters[3 + pass] = counters[0]; }
-
-template <int D>
-__global__ void k_reduce(TreeNode<D> *nodes, const int *counters, int pass, const double *pos, const double *w,
-                         bool bbox_too) {
-    const int beg = counters[1 + pass], end = counters[2 + pass];
-    for (int node = beg + blockIdx.x * blockDim.x + threadIdx.x; node < end; node += gridDim.x * blockDim.x) {
-        TreeNode<D> nd = nodes[node];
-        double lo[D], hi[D], mw = -1.0 / 0.0;
-        for (int d = 0; d < D; ++d) { lo[d] = 1.0 / 0.0; hi[d] = -1.0 / 0.0; }
-        if (nd.b > 0) {
-            for (int s = nd.a; s < nd.b; ++s) {
-                mw = fmax(mw, w[s]);
-                if (bbox_too)
-                    for (int d = 0; d < D; ++d) {
-                        double v = pos[D * (long long)s + d];
-                        lo[d] = fmin(lo[d], v);
-                        hi[d] = fmax(hi[d], v);
-                    }
+    // ---- bottom-up.  The ranges of the levels, from the level counts or starts
+    auto range = [&](int p, int &beg, int &end) {
+        if (BUILD) {
+            beg = 0;
+            end = 1;
+            for (int q = 0; q < p; ++q) {
+                beg = end;
+                end += added[q];
             }
         } else {
-            for (int c = nd.a; c < nd.a - nd.b; ++c) {
-                const TreeNode<D> &ch = nodes[c];
+            beg = start[p];
+            end = start[p + 1];
+        }
+    };
+    int beg, total;
+    range(depth - 1, beg, total);
+    for (int node = thread; node < total; node += nthreads) {
+        const int a = A.nodes[node].a, b = A.nodes[node].b;
+        if (b <= 0) continue;
+        double lo[D], hi[D], mw = -1.0 / 0.0;
+        for (int d = 0; d < D; ++d) {
+            lo[d] = 1.0 / 0.0;
+            hi[d] = -1.0 / 0.0;
+        }
+        for (int s = a; s < b; ++s) {
+            mw = fmax(mw, A.w[s]);
+            if (BUILD)
+                for (int d = 0; d < D; ++d) {
+                    const double v = A.pos[D * (long long)s + d];
+                    lo[d] = fmin(lo[d], v);
+                    hi[d] = fmax(hi[d], v);
+                }
+        }
+        A.nodes[node].maxw = mw;
+        if (BUILD)
+            for (int d = 0; d < D; ++d) {
+                A.nodes[node].lo[d] = lo[d];
+                A.nodes[node].hi[d] = hi[d];
+            }
+    }
+    for (int p = depth - 2; p >= 0; --p) {  // the last level holds leaves only
+        if (!grid_barrier(A.sync, target)) {
+            A.nodes[0].a = -1;
+            A.nodes[0].b = 1;
+            return;
+        }
+        int end;
+        range(p, beg, end);
+        for (int node = beg + thread; node < end; node += nthreads) {
+            const int a = A.nodes[node].a, nch = -A.nodes[node].b;
+            if (nch <= 0) continue;
+            double lo[D], hi[D], mw = -1.0 / 0.0;
+            for (int d = 0; d < D; ++d) {
+                lo[d] = 1.0 / 0.0;
+                hi[d] = -1.0 / 0.0;
+            }
+            for (int c = a; c < a + nch; ++c) {
+                const TreeNode<D> &ch = A.nodes[c];
                 mw = fmax(mw, ch.maxw);
-                if (bbox_too)
+                if (BUILD)
                     for (int d = 0; d < D; ++d) {
                         lo[d] = fmin(lo[d], ch.lo[d]);
                         hi[d] = fmax(hi[d], ch.hi[d]);
                     }
             }
+            A.nodes[node].maxw = mw;
+            if (BUILD)
+                for (int d = 0; d < D; ++d) {
+                    A.nodes[node].lo[d] = lo[d];
+                    A.nodes[node].hi[d] = hi[d];
+                }
         }
-        nodes[node].maxw = mw;
-        if (bbox_too)
-            for (int d = 0; d < D; ++d) {
-                nodes[node].lo[d] = lo[d];
-                nodes[node].hi[d] = hi[d];
-            }
+    }
+    if (BUILD && thread == 0) A.counters[0] = total;
+}
+
+// Start of a build: the box of nothing, the root over every Dirac, no children
+// counted, no arrival at the barrier.
+template <int D>
+__global__ void k_tree_init(unsigned long long *bits, TreeNode<D> *nodes, int *level, int *counters, int npass, long long n,
+                            unsigned *sync) {
+    const int t = threadIdx.x;
+    if (t < D) {
+        bits[t] = ~0ull;
+        bits[D + t] = 0ull;
+    }
+    if (t < npass) counters[npass + 4 + t] = 0;
+    if (t < 4) sync[t] = 0;
+    if (t == 0) {
+        nodes[0].a = 0;
+        nodes[0].b = int(n);
+        level[0] = 0;
+        counters[1] = 0;
     }
 }
 
@@ -249,6 +341,19 @@ template <class T>
 void dev_free(T *&p) {
     if (p) cudaFree(p);
     p = nullptr;
+}
+
+template <int D, bool BUILD>
+void tree_launch(const TreeArgs<D> &a, cudaStream_t st) {
+    // one block per SM at most: all resident
+    int sms = 0, dev = 0;
+    SDOT_CUDA(cudaGetDevice(&dev));
+    SDOT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int g = int(std::min<long long>(sms, (a.n + 511) / 512));
+    TreeArgs<D> b = a;
+    void *args[] = {&b};
+    SDOT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(k_tree<D, BUILD>), dim3(g), dim3(TREE_TB), args, 0, st));
+    note_launch();
 }
 
 int grid_for(long long n, int tb) {
@@ -314,16 +419,16 @@ void DeviceTree<D>::reserve(long long nn) {
     dev_alloc(inv, cap_n);
     dev_alloc(nodes, max_nodes);
     dev_alloc(node_level, max_nodes);
-    dev_alloc(counters, npass + 4);
+    dev_alloc(counters, 2 * npass + 8);
+    dev_alloc(sync, 4);
     dev_alloc(keys, cap_n);
     dev_alloc(keys2, cap_n);
     dev_alloc(keys3, cap_n);
     dev_alloc(vals, cap_n);
     dev_alloc(vals2, cap_n);
     dev_alloc(vals3, cap_n);
-    tmp_bytes = radix_tmp_size(cap_n);
+    tmp_bytes = radix_tmp_size();
     SDOT_CUDA(cudaMalloc(&tmp, tmp_bytes));
-    dev_alloc(bbox, 2 * D);
     dev_alloc(bbox_bits, 2 * D);
 }
 
@@ -339,12 +444,12 @@ template <int D>
 void DeviceTree<D>::release() {
     drop_graphs();
     dev_free(pos); dev_free(w); dev_free(idx); dev_free(inv);
-    dev_free(nodes); dev_free(node_level); dev_free(counters);
+    dev_free(nodes); dev_free(node_level); dev_free(counters); dev_free(sync);
     dev_free(keys); dev_free(keys2); dev_free(keys3);
     dev_free(vals); dev_free(vals2); dev_free(vals3);
     if (tmp) cudaFree(tmp);
     tmp = nullptr;
-    dev_free(bbox); dev_free(bbox_bits);
+    dev_free(bbox_bits);
     cap_n = 0;
 }
 
@@ -372,32 +477,20 @@ void DeviceTree<D>::build(const double *pos_orig, const double *w_orig, long lon
 
 template <int D>
 void DeviceTree<D>::build_launches(const double *pos_orig, const double *w_orig, cudaStream_t st) {
-    k_bbox_init<D><<<1, 32, 0, st>>>(bbox_bits);
+    k_tree_init<D><<<1, 32, 0, st>>>(bbox_bits, nodes, node_level, counters, npass, n, sync);
     note_launch();
     k_bbox<D><<<grid_for(n, TB), TB, 0, st>>>(pos_orig, n, bbox_bits);
     note_launch();
-    k_bbox_final<D><<<1, 32, 0, st>>>(bbox_bits, bbox);
-    note_launch();
-    k_morton<D><<<ceil_div(n, TB), TB, 0, st>>>(pos_orig, n, bbox, key_bits, keys, vals);
+    k_morton<D><<<ceil_div(n, TB), TB, 0, st>>>(pos_orig, n, bbox_bits, key_bits, keys, vals);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
-    radix_sort_pairs(keys, vals, keys2, vals2, keys3, vals3, n, D * key_bits, tmp, st);
+    radix_sort_pairs(keys, vals, keys2, vals2, keys3, vals3, n, D * key_bits, tmp, sync + 2, st);
     k_gather<D><<<ceil_div(n, TB), TB, 0, st>>>(pos_orig, w_orig, vals2, n, pos, w, idx, inv);
     note_launch();
-    k_tree_init<D><<<1, 1, 0, st>>>(nodes, node_level, counters, npass, n);
-    note_launch();
-    const int g = grid_for(n / 2 + 1, TB);
-    for (int p = 0; p < npass; ++p) {
-        k_split<D><<<g, TB, 0, st>>>(nodes, node_level, counters, p, keys2, key_bits, max_per_leaf, max_nodes);
-        note_launch();
-        k_mark_pass<<<1, 1, 0, st>>>(counters, p);
-        note_launch();
-    }
-    for (int p = npass - 1; p >= 0; --p) {
-        k_reduce<D><<<g, TB, 0, st>>>(nodes, counters, p, pos, w, true);
-        note_launch();
-    }
     SDOT_CUDA(cudaGetLastError());
+    tree_launch<D, true>(TreeArgs<D>{nodes, node_level, counters, keys2, pos, w, nullptr, idx, n, key_bits, max_per_leaf,
+                                     max_nodes, npass, sync},
+                         st);
 }
 
 template <int D>
@@ -420,20 +513,10 @@ void DeviceTree<D>::update_weights(const double *w_orig, cudaStream_t st) {
 
 template <int D>
 void DeviceTree<D>::weights_launches(const double *w_orig, cudaStream_t st) {
-    k_gather_w<D><<<ceil_div(n, TB), TB, 0, st>>>(w_orig, idx, n, w);
-    note_launch();
-    refresh_maxw(st);
-}
-
-template <int D>
-void DeviceTree<D>::refresh_maxw(cudaStream_t st) {
-    if (n == 0) return;
-    const int g = grid_for(n / 2 + 1, TB);
-    for (int p = npass - 1; p >= 0; --p) {
-        k_reduce<D><<<g, TB, 0, st>>>(nodes, counters, p, pos, w, false);
-        note_launch();
-    }
-    SDOT_CUDA(cudaGetLastError());
+    SDOT_CUDA(cudaMemsetAsync(sync, 0, 2 * sizeof(unsigned), st));
+    tree_launch<D, false>(TreeArgs<D>{nodes, node_level, counters, keys2, pos, w, w_orig, idx, n, key_bits, max_per_leaf,
+                                      max_nodes, npass, sync},
+                          st);
 }
 
 template struct DeviceTree<2>;

@@ -39,20 +39,21 @@ struct DeviceTree {
     int *inv = nullptr;       // original -> sorted
     TreeNode<D> *nodes = nullptr;
     int *node_level = nullptr;
-    int *counters = nullptr;  // [0] node count, [1 + p] start of pass p
+    // [0] node count, [1 + p] first node of level p (npass + 1 of them),
+    // [npass + 4 + p] nodes that level p gave the next (builds)
+    int *counters = nullptr;
+    unsigned *sync = nullptr;  // grid barriers: of the level kernel, of the sort
     int npass = 0;
     // scratch
     unsigned *keys = nullptr, *keys2 = nullptr, *keys3 = nullptr;
     unsigned *vals = nullptr, *vals2 = nullptr, *vals3 = nullptr;
     void *tmp = nullptr;
     size_t tmp_bytes = 0;
-    double *bbox = nullptr;   // 2 * D doubles (min, max) of the positions
-    unsigned long long *bbox_bits = nullptr;
+    unsigned long long *bbox_bits = nullptr;  // min and max of the positions, as ordered bits
 
     // build() and update_weights() replay their launches from CUDA graphs,
     // captured on the first call for the same input buffers, size and leaf
-    // size (about 80 and 20 small launches; direct launches where the stream
-    // cannot be captured)
+    // size (direct launches where the stream cannot be captured)
     cudaGraphExec_t build_graph = nullptr, weights_graph = nullptr;
     const void *bg_pos = nullptr, *bg_w = nullptr, *wg_w = nullptr;
     long long bg_n = -1, wg_n = -1;
@@ -68,8 +69,6 @@ struct DeviceTree {
     void build(const double *pos_orig, const double *w_orig, long long n, cudaStream_t st);
     // new weights (original order, device pointer): re-gather and refresh maxw
     void update_weights(const double *w_orig, cudaStream_t st);
-    // refresh the node max weights from the sorted weights already in `w`
-    void refresh_maxw(cudaStream_t st);
 };
 
 extern template struct DeviceTree<2>;
