@@ -702,14 +702,11 @@ struct sdot_ctx {
         SDOT_CUDA(cudaEventRecord(ev[2], stream));
         csr_sort_merge(rows, n, perm(), cnt_orig, dim == 2, stream);
         scan_exclusive_total<long long>(cnt_orig, offsets, n, scan_tmp, stream);
-        unpermute(s_mass, o_mass, n, 1, perm(), stream);
-        unpermute(s_mass_c, o_mass_c, n, 1, perm(), stream);
-        unpermute(s_ctd, o_ctd, n, dim, perm(), stream);
+        // outputs in caller order; nnz and the empty cells to the status block,
+        // which comes back (with error bits, overflow count, guard) in one copy
+        unpermute(s_mass, o_mass, s_mass_c, o_mass_c, s_ctd, o_ctd, n, dim, perm(), offsets, &dstat->nnz, &dstat->n_void,
+                  stream);
         SDOT_CUDA(cudaEventRecord(ev[3], stream));
-        // the status block (nnz, empty cells, error bits, overflow count,
-        // guard) comes back in one copy
-        SDOT_CUDA(cudaMemcpyAsync(&dstat->nnz, offsets + n, sizeof(long long), cudaMemcpyDeviceToDevice, stream));
-        count_zeros(s_mass, n, &dstat->n_void, stream);
         SDOT_CUDA(cudaMemcpyAsync(hstat, dstat, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
         SDOT_CUDA(cudaStreamSynchronize(stream));
         nnz = hstat->nnz;
@@ -775,7 +772,12 @@ struct sdot_ctx {
 
     void evaluate_neighbors() {
         if (!nb_dirty) return;
-        evaluate();
+        // the walk alone: the lists need no integrals (an evaluation, when one
+        // is asked for too, is a pass of its own)
+        check_domain();
+        reserve_eval();
+        SDOT_CUDA(cudaMemsetAsync(dstat, 0, sizeof(DevStatus), stream));
+        ensure_tree();
         if (!nb.cnt || nb.stride < ecap) alloc_rows(nb, ecap, dim == 3 ? NBCAP_3D : NBCAP_2D, false);
         if (!nb_offsets) dalloc(nb_offsets, ecap + 1);
         for (int attempt = 0;; ++attempt) {

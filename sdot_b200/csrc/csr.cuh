@@ -28,9 +28,9 @@ void rows_append(const Rows &dst, const Rows &src, long long n, unsigned *err, c
 void accum_pass(double *mass, double *mass_c, double *mom, const double *t_mass, const double *t_mass_c,
                 const double *t_ctd, long long n, int dim, cudaStream_t st);
 void centroids_final(double *ctd, const double *mom, const double *mass_c, long long n, int dim, cudaStream_t st);
-// *count += number of i < n with m[i] == 0 (the empty cells)
-void count_zeros(const double *m, long long n, unsigned long long *count, cudaStream_t st);
-// out[idx[s] * d + k] = in[s * d + k]
-void unpermute(const double *in, double *out, long long n, int d, const int *idx, cudaStream_t st);
+// Masses (m and mc) and centroids (c, d coordinates) to caller order; *n_void +=
+// the number of zeros in m (the empty cells); *nnz = offsets[n].
+void unpermute(const double *m, double *om, const double *mc, double *omc, const double *c, double *oc, long long n, int d,
+               const int *idx, const long long *offsets, long long *nnz, unsigned long long *n_void, cudaStream_t st);
 
 }  // namespace sdot

@@ -80,9 +80,9 @@ struct CellGeo {
     double cx, cy, mass;
 };
 
-// vertices, mass and centroid of cell s (sorted order); false past the
-// capacity (or for an edge id this pass does not handle)
-__device__ bool cell_geo(const DpArgs &A, long long s, CellGeo &g) {
+// the edges of cell s (sorted order); false past the capacity (or for an edge id
+// this pass does not handle)
+__device__ bool cell_edges(const DpArgs &A, long long s, CellGeo &g) {
     const int m = A.nb.cnt[s];
     if (m > DP_CAP) return false;
     g.m = m;
@@ -96,6 +96,13 @@ __device__ bool cell_geo(const DpArgs &A, long long s, CellGeo &g) {
         if (id >= 0 ? id >= nid : id > ID_DOMAIN0 || domain_edge(id) >= A.start_n) return false;
         g.id[k] = id;
     }
+    return true;
+}
+
+// its vertices, mass and centroid too
+__device__ bool cell_geo(const DpArgs &A, long long s, CellGeo &g) {
+    if (!cell_edges(A, s, g)) return false;
+    const int m = g.m;
     // vertex k: the intersection of edges k - 1 and k
     for (int k = 0; k < m; ++k) {
         double a1x, a1y, b1, a2x, a2y, b2;
@@ -208,7 +215,7 @@ __global__ void k_dp_count(DpArgs A, long long *nblocks, unsigned *err) {
     long long col[DP_ROW];
     unsigned char ord[DP_ROW];
     long long cnt = 0;
-    if (!cell_geo(A, s, g)) {
+    if (!cell_edges(A, s, g)) {
         atomicOr(err, unsigned(DE_CAPACITY));
     } else {
         cnt = distinct(col, ord, sorted_items(A, s, g, col, ord));
