@@ -382,7 +382,7 @@ struct sdot_ctx {
         guard = dstat->guard;
         if (!hstat) SDOT_CUDA(cudaMallocHost(reinterpret_cast<void **>(&hstat), sizeof(DevStatus)));
         dalloc(ovf_list2, ecap);
-        dalloc(ovf_cnt2, 1);
+        dalloc(ovf_cnt2, 3);  // the count, and the cursors of the 3D passes over the lists
         if (dim == 3) {
             dalloc(hint3, ecap);
             hint_valid = false;

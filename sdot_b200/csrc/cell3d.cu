@@ -90,10 +90,11 @@ __device__ __forceinline__ void each_block(int nr, F &&f) {
 }
 
 // Cuts the cell by qx x + qy y + qz z <= qb.
-// Outcome: 0 done, 1 a capacity was exceeded, 2 degenerate geometry.
+// Outcome: 0 done (changed is set where a vertex was outside), 1 a capacity was
+// exceeded, 2 degenerate geometry.
 template <int VB, int MAXP>
 __device__ __forceinline__ int cut3(Cell3<VB, MAXP> &C, Work3<VB, MAXP> &W, int &nr, double qx, double qy, double qz,
-                                    double qb, int qid) {
+                                    double qb, int qid, bool &changed) {
     constexpr int PW = MAXP / 32;
     // the small cells keep the masks of faces in registers, and give the
     // places of removed vertices to new ones, so that most use one block
@@ -111,6 +112,7 @@ __device__ __forceinline__ int cut3(Cell3<VB, MAXP> &C, Work3<VB, MAXP> &W, int 
         kept |= al & ~om;
     });
     if (!any) return 0;
+    changed = true;
     if (!SMALL && lane < PW) W.rm[lane] = W.hm[lane] = 0;
     __syncwarp();
     if (!kept) {  // nothing is left
@@ -540,15 +542,16 @@ __device__ int voxel_integrals(const Cell3DArgs &A, Cell3<VB, MAXP> &C, Work3<VB
                 nr = nr0;
                 // the voxel's six planes, relative to c0
                 const int ii[3] = {ix, iy, iz};
+                bool cut = false;
                 for (int d = 0; d < 3; ++d) {
                     const double vlo = A.img_lo[d] + ps[d] * ii[d] - c0[d];
                     const double vhi = A.img_lo[d] + ps[d] * (ii[d] + 1) - c0[d];
                     double a[3] = {0, 0, 0};
                     a[d] = -1.0;
-                    int st = cut3(C, W, nr, a[0], a[1], a[2], -vlo, domain_id(200 + 2 * d));
+                    int st = cut3(C, W, nr, a[0], a[1], a[2], -vlo, domain_id(200 + 2 * d), cut);
                     if (st) return st;
                     a[d] = 1.0;
-                    st = cut3(C, W, nr, a[0], a[1], a[2], vhi, domain_id(201 + 2 * d));
+                    st = cut3(C, W, nr, a[0], a[1], a[2], vhi, domain_id(201 + 2 * d), cut);
                     if (st) return st;
                 }
                 const int nf = list_faces(C, W, nr);
@@ -576,6 +579,37 @@ __device__ int voxel_integrals(const Cell3DArgs &A, Cell3<VB, MAXP> &C, Work3<VB
     return 0;
 }
 
+// The squared distance from c0 of the farthest vertex, rounded up to 20 bits
+// (more than a relative 4e-7 above it), so that what is ruled out by it is so
+// by a margin beyond the rounding of the exact tests.
+template <int VB, class C3>
+__device__ __forceinline__ int farthest(const C3 &C, int nr) {
+    const int lane = threadIdx.x & 31;
+    double m = 0;
+    each_block<VB>(nr, [&](int r) {
+        if (!(C.alive[r] >> lane & 1u)) return;
+        const int v = lane + 32 * r;
+        const double d = C.x[v] * C.x[v] + C.y[v] * C.y[v] + C.z[v] * C.z[v];
+        m = d > m ? d : m;
+    });
+    return int(__reduce_max_sync(FULL, unsigned(__double2hiint(m)))) + 2;
+}
+
+// Squares outside (TINY, HUGE_SQ) are not compared: they may have lost their
+// digits.
+constexpr double TINY = 1e-290, HUGE_SQ = 1e300;
+// Boxes waiting beyond which a sweep is worth its loads.
+constexpr int SWEEP_MIN = 2;
+
+// A box is evicted if every vertex u has |u|^2 - w0 <= d(u)^2 - maxw, d its
+// distance from the box.  With D the box's distance from c0 and every |u| <= R
+// <= D, d(u) >= D - |u|, and that holds if 2 D R <= D^2 + w0 - maxw.
+__device__ __forceinline__ bool beyond(const TreeNode<3> &nd, double c0x, double c0y, double c0z, double w0, double r2) {
+    const double gx = gap(nd.lo[0], nd.hi[0], c0x), gy = gap(nd.lo[1], nd.hi[1], c0y), gz = gap(nd.lo[2], nd.hi[2], c0z);
+    const double d2 = gx * gx + gy * gy + gz * gz, t = d2 + (w0 - nd.maxw), q = t * t;
+    return t > 0 && d2 >= r2 && q >= 4 * (r2 * d2) && q > TINY && q < HUGE_SQ;
+}
+
 // Builds and integrates the cell of sorted Dirac s.  Returns 0 (outputs
 // written), 1 (a capacity was exceeded: retry in the next pass), 2 (failed:
 // outputs written as NaN / empty row, error flagged).
@@ -588,13 +622,15 @@ __device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<VB
     int nr;
     init_box(C, nr, A, c0x, c0y, c0z);
     int status = 0;
+    bool changed = true;  // since r2 was taken
+    int r2h = 0;          // high word of a bound of their squared distance from c0
     // a convex shape: its half-spaces cut the box first (relative to c0:
     // a . u <= b - a . c0), as ConvexPolyhedronAssembly::add_convex_polyhedron
     // cuts its box (ConvexPolyhedronAssembly.tcc:7-33)
     for (int k = 0; k < A.nplanes && status == 0; ++k) {
         const double ax = A.planes[4 * k], ay = A.planes[4 * k + 1], az = A.planes[4 * k + 2];
         const double b = A.planes[4 * k + 3] - (ax * c0x + ay * c0y + az * c0z);
-        status = cut3(C, W, nr, ax, ay, az, b, domain_id(6 + k));
+        status = cut3(C, W, nr, ax, ay, az, b, domain_id(6 + k), changed);
     }
     if (lane == 0) W.stack[0] = 0;
     __syncwarp();
@@ -604,6 +640,29 @@ __device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<VB
             if (lane == 0) flag_error(A.err, DE_ITER);
             status = 2;
             break;
+        }
+        // After a cut the boxes waiting are tried against the ball that holds
+        // the cell, one per lane (the 32 nearest): most of those that would
+        // fail the vertex test when popped go here, many at a time
+        if (changed) {
+            changed = false;
+            r2h = farthest<VB>(C, nr);
+            if (sp > SWEEP_MIN) {
+                const int base = max(sp - 32, 0);
+                bool keep = false;
+                int mine = 0;
+                if (base + lane < sp) {
+                    mine = W.stack[base + lane];
+                    const TreeNode<3> nd = A.nodes[mine];
+                    keep = !beyond(nd, c0x, c0y, c0z, w0, __hiloint2double(r2h, 0));
+                }
+                const unsigned km = __ballot_sync(FULL, keep);
+                __syncwarp();
+                if (keep) W.stack[base + __popc(km & ((1u << lane) - 1u))] = mine;
+                __syncwarp();
+                sp = base + __popc(km);
+                if (sp == 0) break;
+            }
         }
         const int node = W.stack[--sp];
         __syncwarp();
@@ -647,6 +706,7 @@ __device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<VB
                 const double mx = 0.5 * (cn.lo[0] + cn.hi[0]) - c0x, my = 0.5 * (cn.lo[1] + cn.hi[1]) - c0y,
                              mz = 0.5 * (cn.lo[2] + cn.hi[2]) - c0z;
                 key = float(mx * mx + my * my + mz * mz);
+                if (beyond(cn, c0x, c0y, c0z, w0, __hiloint2double(r2h, 0))) key = -1.f;  // not pushed
             }
             int rank = 0;
 #pragma unroll
@@ -654,21 +714,35 @@ __device__ __forceinline__ int cell3d(const Cell3DArgs &A, long long s, Cell3<VB
                 const float kc = __shfl_sync(FULL, key, c);
                 rank += c < nch && (kc > key || (kc == key && c < lane));
             }
-            if (lane < nch) W.stack[sp + rank] = first + lane;
+            const unsigned pm = __ballot_sync(FULL, lane < nch && !(key < 0));
+            if (pm >> lane & 1u) W.stack[sp + rank] = first + lane;
             __syncwarp();
-            sp += nch;
+            sp += __popc(pm);
         } else {
             if (nd.a < 0 || nd.b > A.n) {
                 if (lane == 0) guard_fail3(A, 2, s, node);
                 status = 2;
                 break;
             }
-            for (int j = nd.a; j < nd.b && status == 0; ++j) {
-                if (j == s) continue;
-                // weighted bisector, relative to c0: V . u <= 1/2 |V|^2 + 1/2 (w0 - w1)
-                const double vx = A.pos[3 * j] - c0x, vy = A.pos[3 * j + 1] - c0y, vz = A.pos[3 * j + 2] - c0z;
-                const double qb = 0.5 * (vx * vx + vy * vy + vz * vz) + 0.5 * (w0 - A.w[j]);
-                status = cut3(C, W, nr, vx, vy, vz, qb, j);
+            for (int j0 = nd.a; j0 < nd.b && status == 0; j0 += 32) {
+                // weighted bisectors, one per lane, relative to c0: V . u <=
+                // 1/2 |V|^2 + 1/2 (w0 - w1); those that miss the ball cut
+                // nothing, the others are tried in index order
+                bool near = false;
+                double vx = 0, vy = 0, vz = 0, qb = 0;
+                if (j0 + lane < nd.b && j0 + lane != s) {
+                    const int j = j0 + lane;
+                    vx = A.pos[3 * j] - c0x, vy = A.pos[3 * j + 1] - c0y, vz = A.pos[3 * j + 2] - c0z;
+                    const double v2 = vx * vx + vy * vy + vz * vz;
+                    qb = 0.5 * v2 + 0.5 * (w0 - A.w[j]);
+                    const double q = qb * qb;
+                    near = !(qb > 0 && q >= __hiloint2double(r2h, 0) * v2 && q > TINY && q < HUGE_SQ);
+                }
+                for (unsigned todo = __ballot_sync(FULL, near); todo && status == 0; todo &= todo - 1) {
+                    const int l = __ffs(int(todo)) - 1;
+                    status = cut3(C, W, nr, __shfl_sync(FULL, vx, l), __shfl_sync(FULL, vy, l), __shfl_sync(FULL, vz, l),
+                                  __shfl_sync(FULL, qb, l), j0 + l, changed);
+                }
             }
         }
     }
@@ -786,37 +860,48 @@ constexpr size_t warp_smem_bytes() {
 // outgrow it run again with 192 vertices and 128 faces, then with 640 vertices
 // and 256 faces (508 vertices): every pass in shared memory.
 //
-// Bound by instruction issue (62% of the cycles, 22 of 32 lanes active; 28
-// effective cuts, 50 others and 98 box tests per uniform cell) and by the
-// latency of FP64 and shared memory between them, so the first pass takes the
-// occupancy of 80 registers (12 blocks; 8, 10, 14, 16 blocks of the
-// multilinear kernel: 14.9, 11.6, 10.0, 9.9 ms at 96 registers and more spills
-// for the last two; 10 to 16 are within 5% at constant density).  Measured
-// against the faces held as polygons, four passes, the last two in global
-// memory: 200,000 Diracs of the 3D mix 30.9 -> 10.2 ms, 20,000 clustered ones
-// 13.1 -> 2.8 ms, whole evaluations 31.7 -> 11.0 and 13.9 -> 3.5 ms.
-struct Pass0 { static constexpr int VB = 2, MAXP = 64, WARPS = 2, BLOCKS = 12, POLY_BLOCKS = 16; };
-struct Pass1 { static constexpr int VB = 6, MAXP = 128, WARPS = 1, BLOCKS = 14, POLY_BLOCKS = 10; };
-struct Pass2 { static constexpr int VB = 20, MAXP = 256, WARPS = 1, BLOCKS = 5, POLY_BLOCKS = 5; };
+// Bound by instruction issue and by the latency of FP64 and shared memory
+// between the instructions (28 effective cuts per uniform cell), so the first
+// pass takes the occupancy of 80 registers (20, 24, 28, 32 blocks at constant
+// density: 0.81, 0.74, 0.77, 0.81 ms for 20,000 uniform Diracs; 18, 24, 26, 20
+// of the multilinear kernel 7.9, 7.3, 7.6, 7.9 ms for 200,000).  One warp a
+// block: with two the block waited for the longer cell (9.5 -> 8.5 ms).
+// The tests against the ball took the place of most of the 98 box tests and 50
+// ineffective cuts of a cell that the vertices were tried for before: with the
+// blocks chosen anew, 200,000 Diracs of the 3D mix 10.2 -> 7.3 ms, 20,000
+// uniform ones 1.13 -> 0.74.  The larger passes fetch their cells (with a fixed
+// share each, 20,000 clustered Diracs took 2.7 instead of 2.2 ms).
+// Against the faces held as polygons, four passes, the last two in global
+// memory: 30.9 -> 7.3 ms and 13.1 -> 2.2 ms, whole evaluations 31.7 -> 7.9 and
+// 13.9 -> 2.7 ms.
+struct Pass0 { static constexpr int VB = 2, MAXP = 64, BLOCKS = 24, POLY_BLOCKS = 24; };
+struct Pass1 { static constexpr int VB = 6, MAXP = 128, BLOCKS = 16, POLY_BLOCKS = 10; };
+struct Pass2 { static constexpr int VB = 20, MAXP = 256, BLOCKS = 5, POLY_BLOCKS = 5; };
 
 template <class P, int PASS, int DENS>
-__global__ void __launch_bounds__(32 * P::WARPS, DENS == D_IMAGE ? 1 : DENS == D_POLY ? P::POLY_BLOCKS : P::BLOCKS)
-    k_cells3d(const Cell3DArgs A, const int *list, const int *list_cnt, int *next_list, int *next_cnt) {
+__global__ void __launch_bounds__(32, DENS == D_IMAGE ? 1 : DENS == D_POLY ? P::POLY_BLOCKS : P::BLOCKS)
+    k_cells3d(const Cell3DArgs A, const int *list, const int *list_cnt, int *cursor, int *next_list, int *next_cnt) {
     extern __shared__ double smem3[];
     constexpr int VB = P::VB, MAXP = P::MAXP;
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gw = blockIdx.x * P::WARPS + wib;
-    char *base = reinterpret_cast<char *>(smem3) + warp_smem_bytes<VB, MAXP, DENS>() * wib;
+    const int lane = threadIdx.x;
+    char *base = reinterpret_cast<char *>(smem3);
     using C3 = Cell3<VB, MAXP>;
     using W3 = Work3<VB, MAXP>;
     C3 &C = *reinterpret_cast<C3 *>(base);
     W3 &W = *reinterpret_cast<W3 *>(base + sizeof(C3));
     C3 *B = reinterpret_cast<C3 *>(base + sizeof(C3) + sizeof(W3));
     double *wa = reinterpret_cast<double *>(base + 2 * sizeof(C3) + sizeof(W3));
-    const long long cnt = list ? *list_cnt : A.n;
-    const int nwarps = gridDim.x * P::WARPS;
-    for (long long i = gw; i < cnt; i += nwarps) {
-        const long long s = list ? list[i] : i;
+    // the first pass has a block per cell; the others' blocks fetch the next
+    // entry of their list until it is used up (fewer than n of them, so the
+    // cursor stays an int)
+    const long long cnt = PASS == 0 ? A.n : *list_cnt;
+    auto fetch = [&] {
+        int k = 0;
+        if (lane == 0) k = atomicAdd(cursor, 1);
+        return (long long)__shfl_sync(FULL, k, 0);
+    };
+    for (long long i = PASS == 0 ? blockIdx.x : fetch(); i < cnt; i = PASS == 0 ? cnt : fetch()) {
+        const long long s = PASS == 0 ? i : list[i];
         if (PASS == 0 && A.use_hint && A.hint) {
             // a cell that needed a larger pass last time goes straight there
             const int h = A.hint[s];
@@ -827,7 +912,7 @@ __global__ void __launch_bounds__(32 * P::WARPS, DENS == D_IMAGE ? 1 : DENS == D
                     else
                         A.ovf_list2[atomicAdd(A.ovf_cnt2, 1)] = int(s);
                 }
-                continue;
+                return;
             }
         }
         const int r = cell3d<VB, MAXP, DENS, PASS>(A, s, C, W, B, wa);
@@ -844,28 +929,28 @@ __global__ void __launch_bounds__(32 * P::WARPS, DENS == D_IMAGE ? 1 : DENS == D
 }
 
 template <class P, int PASS, int DENS>
-void launch3(const Cell3DArgs &a, const int *list, const int *list_cnt, int *next_list, int *next_cnt, long long blocks,
-             cudaStream_t st) {
-    const size_t smem = warp_smem_bytes<P::VB, P::MAXP, DENS>() * P::WARPS;
+void launch3(const Cell3DArgs &a, const int *list, const int *list_cnt, int *cursor, int *next_list, int *next_cnt,
+             long long blocks, cudaStream_t st) {
+    const size_t smem = warp_smem_bytes<P::VB, P::MAXP, DENS>();
     static PerDevice<int> attr;
     attr.once([&] {
         SDOT_CUDA(cudaFuncSetAttribute(k_cells3d<P, PASS, DENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     });
-    k_cells3d<P, PASS, DENS><<<int(blocks), 32 * P::WARPS, smem, st>>>(a, list, list_cnt, next_list, next_cnt);
+    k_cells3d<P, PASS, DENS><<<int(blocks), 32, smem, st>>>(a, list, list_cnt, cursor, next_list, next_cnt);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
 }
 
 template <int DENS>
 void launch_passes(const Cell3DArgs &a, cudaStream_t st) {
-    // one block per two cells: the hardware hands them out as blocks end
-    launch3<Pass0, 0, DENS>(a, nullptr, nullptr, a.ovf_list, a.ovf_cnt, (a.n + Pass0::WARPS - 1) / Pass0::WARPS, st);
+    // one block per cell: the hardware hands them out as blocks end
+    launch3<Pass0, 0, DENS>(a, nullptr, nullptr, nullptr, a.ovf_list, a.ovf_cnt, a.n, st);
     // the larger passes take the overflow lists (their lengths are on the
     // device): as many blocks as fit the device, or one per cell
-    launch3<Pass1, 1, DENS>(a, a.ovf_list, a.ovf_cnt, a.ovf_list2, a.ovf_cnt2,
+    launch3<Pass1, 1, DENS>(a, a.ovf_list, a.ovf_cnt, a.ovf_cnt2 + 1, a.ovf_list2, a.ovf_cnt2,
                             std::min<long long>(a.n, 148LL * Pass1::BLOCKS), st);
-    launch3<Pass2, 2, DENS>(a, a.ovf_list2, a.ovf_cnt2, nullptr, nullptr, std::min<long long>(a.n, 148LL * Pass2::BLOCKS),
-                            st);
+    launch3<Pass2, 2, DENS>(a, a.ovf_list2, a.ovf_cnt2, a.ovf_cnt2 + 2, nullptr, nullptr,
+                            std::min<long long>(a.n, 148LL * Pass2::BLOCKS), st);
 }
 
 }  // namespace
@@ -873,7 +958,7 @@ void launch_passes(const Cell3DArgs &a, cudaStream_t st) {
 void cells3d_launch(const Cell3DArgs &a, cudaStream_t st) {
     if (a.n == 0) return;
     SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt, 0, sizeof(int), st));
-    SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt2, 0, sizeof(int), st));
+    SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt2, 0, 3 * sizeof(int), st));  // and the cursors
     if (a.rows.side_used) SDOT_CUDA(cudaMemsetAsync(a.rows.side_used, 0, sizeof(unsigned long long), st));
     if (a.nb.side_used) SDOT_CUDA(cudaMemsetAsync(a.nb.side_used, 0, sizeof(unsigned long long), st));
     if (a.img)

@@ -42,7 +42,7 @@ struct Cell3DArgs {
     int *ovf_list = nullptr;  // cells handed to the second pass
     int *ovf_cnt = nullptr;
     int *ovf_list2 = nullptr;  // cells handed to the third pass
-    int *ovf_cnt2 = nullptr;
+    int *ovf_cnt2 = nullptr;   // its length, then the two passes' cursors (3 ints)
     // per cell (sorted order): the pass (0..2) its last build needed; with
     // use_hint the first pass sends each cell straight to that pass (the
     // positions, hence the tree order, must not have changed)
