@@ -13,17 +13,21 @@
 // 3 x 3 blocks (rows: centroid x, centroid y, mass; columns: position x,
 // position y, weight), corrected by the centroid and divided by
 // mass + (mass == 1) as the reference divides (.h:178-182), sorted by column
-// and merged.  One thread per cell; cells of more than DP_CAP vertices report
-// a capacity error.
+// and merged.  Eight lanes per cell, an edge each; cells of more than DP_CAP
+// vertices report a capacity error.
 #include "derpos.cuh"
+
+#include <climits>
 
 namespace sdot {
 
 namespace {
 
-constexpr int TB = 128;
 constexpr int DP_CAP = 64;   // vertices of a cell
 constexpr int DP_ROW = 65;   // blocks of a row (one per edge and the diagonal)
+constexpr int LANES = 8;     // lanes per cell: an edge each up to 8 edges (a cell has 6 on average)
+constexpr int TB = 64;
+constexpr int CELLS = TB / LANES;
 
 struct DpArgs {
     Rows nb;
@@ -39,13 +43,13 @@ struct DpArgs {
 
 // position of the Dirac (or periodic image) on the other side of an edge with this id
 __device__ void other_site(const DpArgs &A, int id, double &x, double &y, double &w, int &j) {
-    j = int(id % A.n);
-    const int k = int(id / A.n) - 1;
+    const unsigned n = unsigned(A.n), t = A.ntrans ? unsigned(id) / n : 0;
+    j = int(unsigned(id) - t * n);
     x = A.pos[2 * j];
     y = A.pos[2 * j + 1];
-    if (k >= 0) {
-        x += A.trans[2 * k];
-        y += A.trans[2 * k + 1];
+    if (t) {
+        x += A.trans[2 * (t - 1)];
+        y += A.trans[2 * (t - 1) + 1];
     }
     w = A.w[j];
 }
@@ -71,67 +75,72 @@ __device__ void edge_line(const DpArgs &A, int id, double c0x, double c0y, doubl
     }
 }
 
-// a cell rebuilt from its row of cut ids
+// The edges of a cell in shared memory.
+struct RowIds {
+    int id[DP_CAP];
+    int col[DP_ROW];   // caller column of every item (edge k, or m for the diagonal); -1: a domain edge
+    int head[DP_ROW];  // the same where no item before it has this column, else INT_MAX
+};
+
+// The cell rebuilt from them: its vertices; and where it lies.
 struct CellGeo {
     int m;
+    const int *id;
     double c0x, c0y, w0;
-    double vx[DP_CAP], vy[DP_CAP];
-    int id[DP_CAP];
+    const double *vx, *vy;
     double cx, cy, mass;
 };
 
-// the edges of cell s (sorted order); false past the capacity (or for an edge id
-// this pass does not handle)
-__device__ bool cell_edges(const DpArgs &A, long long s, CellGeo &g) {
-    const int m = A.nb.cnt[s];
-    if (m > DP_CAP) return false;
-    g.m = m;
-    g.c0x = A.pos[2 * s];
-    g.c0y = A.pos[2 * s + 1];
-    g.w0 = A.w[s];
+// Lanes of one cell: the group's place in the warp.
+struct Group {
+    int lane;       // in the group
+    unsigned mask;  // of its lanes
+    __device__ Group() : lane(threadIdx.x & (LANES - 1)), mask(0xffu << (threadIdx.x & 24)) {}
+    template <class T>
+    __device__ T sum(T v) const {
+#pragma unroll
+        for (int o = LANES / 2; o; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+};
+
+// Edges and columns of cell s (sorted order), and the number of distinct
+// columns; -1 past the capacity (or for an edge id that this pass does not
+// handle).  Columns are unique but for periodic images.
+__device__ int load_row(const DpArgs &A, long long s, const Group &g, RowIds &r, int &m) {
+    m = A.nb.cnt[s];
+    if (m > DP_CAP) return -1;
     const long long nid = (A.ntrans + 1LL) * A.n;
-    for (int k = 0; k < m; ++k) {
+    bool ok = true;
+    for (int k = g.lane; k < m; k += LANES) {
         const int id = *A.nb.colp(s, k);
         // a Dirac (or an image) or a domain edge; anything else (an arc) is not handled
-        if (id >= 0 ? id >= nid : id > ID_DOMAIN0 || domain_edge(id) >= A.start_n) return false;
-        g.id[k] = id;
+        const bool known = id >= 0 ? id < nid : id <= ID_DOMAIN0 && domain_edge(id) < A.start_n;
+        ok = ok && known;
+        r.id[k] = id;
+        r.col[k] = known && id >= 0 ? A.idx[A.ntrans ? int(unsigned(id) % unsigned(A.n)) : id] : -1;
     }
-    return true;
-}
-
-// its vertices, mass and centroid too
-__device__ bool cell_geo(const DpArgs &A, long long s, CellGeo &g) {
-    if (!cell_edges(A, s, g)) return false;
-    const int m = g.m;
-    // vertex k: the intersection of edges k - 1 and k
-    for (int k = 0; k < m; ++k) {
-        double a1x, a1y, b1, a2x, a2y, b2;
-        edge_line(A, g.id[k == 0 ? m - 1 : k - 1], g.c0x, g.c0y, g.w0, a1x, a1y, b1);
-        edge_line(A, g.id[k], g.c0x, g.c0y, g.w0, a2x, a2y, b2);
-        const double det = a1x * a2y - a1y * a2x;
-        g.vx[k] = g.c0x + (b1 * a2y - b2 * a1y) / det;
-        g.vy[k] = g.c0y + (a1x * b2 - a2x * b1) / det;
+    if (g.lane == 0) r.col[m] = A.idx[s];
+    if (__any_sync(g.mask, !ok)) return -1;
+    __syncwarp(g.mask);
+    int heads = 0;
+    for (int k = g.lane; k <= m; k += LANES) {
+        const int c = r.col[k];
+        bool head = c >= 0;
+        for (int q = 0; q < k; ++q) head = head && r.col[q] != c;
+        r.head[k] = head ? c : INT_MAX;
+        heads += head;
     }
-    // mass and centroid: fan from vertex 0 (add_centroid_contrib, ConvexPolyhedron2.tcc:1047-1074)
-    double mass = 0, mx = 0, my = 0;
-    for (int k = 2; k < m; ++k) {
-        const double ax = g.vx[0], ay = g.vy[0], bx = g.vx[k - 1], by = g.vy[k - 1], cx = g.vx[k], cy = g.vy[k];
-        const double lea = 0.5 * (ax * (by - cy) + bx * (cy - ay) + cx * (ay - by)) * A.coeff;
-        mx += lea * (1.0 / 3.0) * (ax + bx + cx);
-        my += lea * (1.0 / 3.0) * (ay + by + cy);
-        mass += lea;
-    }
-    g.mass = mass;
-    g.cx = mass != 0 ? mx / mass : 0.0;
-    g.cy = mass != 0 ? my / mass : 0.0;
-    return true;
+    heads = g.sum(heads);
+    __syncwarp(g.mask);
+    return heads;
 }
 
 // The block of the edge leaving vertex i0 (a Dirac on the other side): t
 // receives the off-diagonal block (row-major, rows centroid x, centroid y,
-// mass; columns x, y, weight), d0 accumulates the diagonal's share.  Returns
-// the caller column.
-__device__ long long edge_block(const DpArgs &A, const CellGeo &g, int i0, double *t, double *d0) {
+// mass; columns x, y, weight), d0 (if not null) accumulates the diagonal's
+// share.
+__device__ void edge_block(const DpArgs &A, const CellGeo &g, int i0, double *t, double *d0) {
     const int i1 = i0 + 1 < g.m ? i0 + 1 : 0;
     double x1, y1, w1;
     int j;
@@ -148,23 +157,22 @@ __device__ long long edge_block(const DpArgs &A, const CellGeo &g, int i0, doubl
     const double dist = sqrt((x1 - g.c0x) * (x1 - g.c0x) + (y1 - g.c0y) * (y1 - g.c0y));
     const double bd = 0.5 * meas / dist;
     for (int k = 0; k < 9; ++k) t[k] = 0;
-    d0[8] += bd;
+    if (d0) d0[8] += bd;
     t[8] = -bd;
     for (int q = 0; q < 2; ++q) {
         const double value = 0.5 * P[q] / dist;
-        d0[3 * q + 2] += value;
+        if (d0) d0[3 * q + 2] += value;
         t[3 * q + 2] = -value;
     }
     for (int d = 0; d < 2; ++d) {
-        d0[6 + d] += (P[d] - meas * c0[d]) / dist;
+        if (d0) d0[6 + d] += (P[d] - meas * c0[d]) / dist;
         t[6 + d] = (meas * c1[d] - P[d]) / dist;
     }
     for (int d = 0; d < 2; ++d)
         for (int q = 0; q < 2; ++q) {
-            d0[3 * q + d] += (M[d][q] - P[q] * c0[d]) / dist;
+            if (d0) d0[3 * q + d] += (M[d][q] - P[q] * c0[d]) / dist;
             t[3 * q + d] = (P[q] * c1[d] - M[d][q]) / dist;
         }
-    return A.idx[j];
 }
 
 // centroid correction, as the reference divides (.h:178-182)
@@ -175,108 +183,121 @@ __device__ void correct(const CellGeo &g, double *t) {
         for (int e = 0; e < 3; ++e) t[3 * r + e] = (t[3 * r + e] - t[6 + e] * c[r]) / div;
 }
 
-// The row's items in column order: ord[0..cnt) the item indices (edge index,
-// or m for the diagonal) sorted by (column, index); col[] their columns.
-// Returns the number of items (equal columns not merged yet).
-__device__ int sorted_items(const DpArgs &A, long long s, const CellGeo &g, long long *col, unsigned char *ord) {
-    int cnt = 0;
-    for (int k = 0; k < g.m; ++k) {
-        if (g.id[k] < 0) continue;  // a domain edge
-        double x, y, w;
-        int j;
-        other_site(A, g.id[k], x, y, w, j);
-        col[k] = A.idx[j];
-        ord[cnt++] = (unsigned char)k;
-    }
-    col[g.m] = A.idx[s];
-    ord[cnt++] = (unsigned char)g.m;
-    for (int i = 1; i < cnt; ++i) {
-        const unsigned char x = ord[i];
-        int q = i - 1;
-        while (q >= 0 && (col[ord[q]] > col[x] || (col[ord[q]] == col[x] && ord[q] > x))) {
-            ord[q + 1] = ord[q];
-            --q;
-        }
-        ord[q + 1] = x;
-    }
-    return cnt;
-}
-
-__device__ int distinct(const long long *col, const unsigned char *ord, int cnt) {
-    int d = 0;
-    for (int i = 0; i < cnt; ++i) d += i == 0 || col[ord[i]] != col[ord[i - 1]];
-    return d;
-}
-
-__global__ void k_dp_count(DpArgs A, long long *nblocks, unsigned *err) {
-    const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(TB) k_dp_count(DpArgs A, long long *nblocks, unsigned *err) {
+    __shared__ RowIds rows[CELLS];
+    const Group g;
+    const long long s = blockIdx.x * (long long)CELLS + threadIdx.x / LANES;
     if (s >= A.n) return;
-    CellGeo g;
-    long long col[DP_ROW];
-    unsigned char ord[DP_ROW];
-    long long cnt = 0;
-    if (!cell_edges(A, s, g)) {
-        atomicOr(err, unsigned(DE_CAPACITY));
-    } else {
-        cnt = distinct(col, ord, sorted_items(A, s, g, col, ord));
-    }
-    nblocks[A.idx[s]] = cnt;
+    int m;
+    const int cnt = load_row(A, s, g, rows[threadIdx.x / LANES], m);
+    if (g.lane) return;
+    if (cnt < 0) atomicOr(err, unsigned(DE_CAPACITY));
+    nblocks[A.idx[s]] = cnt < 0 ? 0 : cnt;
 }
 
 // block offsets boff (caller order, exclusive scan of the counts) -> CSR of
 // 3 n rows: row 3 i + d holds, for every block of Dirac i, its row d; the
-// items of one column are corrected, then added in (column, index) order
-__global__ void k_dp_write(DpArgs A, const long long *boff, long long *off, long long *cols, double *vals, double *v) {
-    const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+// items of one column are corrected, then added in index order (the diagonal
+// last).
+// Bound by its loads of neighbours and its stores (54 entries of 16 bytes a
+// cell).  Lanes of a cell share its lines and vertices through shared memory
+// and store blocks that lie side by side; a thread per cell kept 2 KB of local
+// memory each and stored 72 bytes apart.  100,000 Diracs, the whole call with
+// the count: 1035 -> 862 us.
+__global__ void __launch_bounds__(TB) k_dp_write(DpArgs A, const long long *boff, long long *off, long long *cols,
+                                                 double *vals, double *v) {
+    struct Cell {
+        RowIds r;
+        double ax[DP_CAP], ay[DP_CAP], b[DP_CAP], vx[DP_CAP], vy[DP_CAP];
+    };
+    __shared__ Cell cells[CELLS];
+    Cell &C = cells[threadIdx.x / LANES];
+    const Group gr;
+    const long long s = blockIdx.x * (long long)CELLS + threadIdx.x / LANES;
     if (s >= A.n) return;
     const long long i = A.idx[s];
     const long long base = 9 * boff[i];
-    if (s == 0) off[3 * A.n] = 9 * boff[A.n];
+    if (s == 0 && gr.lane == 0) off[3 * A.n] = 9 * boff[A.n];
     CellGeo g;
-    if (!cell_geo(A, s, g)) {
-        for (int d = 0; d < 3; ++d) {
-            off[3 * i + d] = base;
-            v[3 * i + d] = 0;
+    const int cnt = load_row(A, s, gr, C.r, g.m);
+    if (cnt < 0) {
+        if (gr.lane < 3) {
+            off[3 * i + gr.lane] = base;
+            v[3 * i + gr.lane] = 0;
         }
         return;
     }
-    v[3 * i] = g.cx;
-    v[3 * i + 1] = g.cy;
-    v[3 * i + 2] = g.mass;
-    long long col[DP_ROW];
-    unsigned char ord[DP_ROW];
-    const int items = sorted_items(A, s, g, col, ord);
-    const int cnt = distinct(col, ord, items);
-    for (int d = 0; d < 3; ++d) off[3 * i + d] = base + 3LL * cnt * d;
+    const int m = g.m;
+    g.id = C.r.id;
+    g.vx = C.vx;
+    g.vy = C.vy;
+    g.c0x = A.pos[2 * s];
+    g.c0y = A.pos[2 * s + 1];
+    g.w0 = A.w[s];
+    for (int k = gr.lane; k < m; k += LANES)
+        edge_line(A, C.r.id[k], g.c0x, g.c0y, g.w0, C.ax[k], C.ay[k], C.b[k]);
+    __syncwarp(gr.mask);
+    // vertex k: the intersection of edges k - 1 and k
+    for (int k = gr.lane; k < m; k += LANES) {
+        const int q = k == 0 ? m - 1 : k - 1;
+        const double a1x = C.ax[q], a1y = C.ay[q], b1 = C.b[q], a2x = C.ax[k], a2y = C.ay[k], b2 = C.b[k];
+        const double det = a1x * a2y - a1y * a2x;
+        C.vx[k] = g.c0x + (b1 * a2y - b2 * a1y) / det;
+        C.vy[k] = g.c0y + (a1x * b2 - a2x * b1) / det;
+    }
+    __syncwarp(gr.mask);
+    // mass and centroid: fan from vertex 0 (add_centroid_contrib, ConvexPolyhedron2.tcc:1047-1074)
+    double mass = 0, mx = 0, my = 0;
+    for (int k = 2 + gr.lane; k < m; k += LANES) {
+        const double ax = C.vx[0], ay = C.vy[0], bx = C.vx[k - 1], by = C.vy[k - 1], cx = C.vx[k], cy = C.vy[k];
+        const double lea = 0.5 * (ax * (by - cy) + bx * (cy - ay) + cx * (ay - by)) * A.coeff;
+        mx += lea * (1.0 / 3.0) * (ax + bx + cx);
+        my += lea * (1.0 / 3.0) * (ay + by + cy);
+        mass += lea;
+    }
+    mass = gr.sum(mass);
+    mx = gr.sum(mx);
+    my = gr.sum(my);
+    g.mass = mass;
+    g.cx = mass != 0 ? mx / mass : 0.0;
+    g.cy = mass != 0 ? my / mass : 0.0;
+    if (gr.lane < 3) {
+        v[3 * i + gr.lane] = gr.lane == 0 ? g.cx : gr.lane == 1 ? g.cy : g.mass;
+        off[3 * i + gr.lane] = base + 3LL * cnt * gr.lane;
+    }
     // the diagonal: every edge's share
-    double d0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, t[9], dummy[9];
-    for (int k = 0; k < g.m; ++k)
-        if (g.id[k] >= 0) edge_block(A, g, k, t, d0);
+    double d0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, t[9];
+    for (int k = gr.lane; k < m; k += LANES)
+        if (C.r.id[k] >= 0) edge_block(A, g, k, t, d0);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) d0[q] = gr.sum(d0[q]);
     correct(g, d0);
-    int b = -1;
-    double acc[9];
-    for (int it = 0; it < items; ++it) {
-        const int k = ord[it];
-        if (k == g.m) {
-            for (int q = 0; q < 9; ++q) t[q] = d0[q];
+    for (int k = gr.lane; k <= m; k += LANES) {
+        const int c = C.r.head[k];
+        if (c == INT_MAX) continue;
+        double acc[9];
+        if (k == m) {
+            for (int q = 0; q < 9; ++q) acc[q] = d0[q];
         } else {
-            for (int q = 0; q < 9; ++q) dummy[q] = 0;
-            edge_block(A, g, k, t, dummy);
-            correct(g, t);
+            edge_block(A, g, k, acc, nullptr);
+            correct(g, acc);
         }
-        const bool first = it == 0 || col[ord[it - 1]] != col[k];
-        if (first) {
-            ++b;
-            for (int q = 0; q < 9; ++q) acc[q] = t[q];
-        } else {
+        int b = 0;  // its place: the columns before it
+        for (int e = 0; e <= m; ++e) {
+            b += C.r.head[e] < c;
+            if (e <= k || C.r.col[e] != c) continue;
+            if (e == m) {
+                for (int q = 0; q < 9; ++q) t[q] = d0[q];
+            } else {
+                edge_block(A, g, e, t, nullptr);
+                correct(g, t);
+            }
             for (int q = 0; q < 9; ++q) acc[q] += t[q];
         }
-        const bool last = it + 1 == items || col[ord[it + 1]] != col[k];
-        if (!last) continue;
         for (int d = 0; d < 3; ++d)
             for (int e = 0; e < 3; ++e) {
                 const long long o = base + 3LL * cnt * d + 3 * b + e;
-                cols[o] = 3 * col[k] + e;
+                cols[o] = 3LL * c + e;
                 vals[o] = acc[3 * d + e];
             }
     }
@@ -289,7 +310,7 @@ void derpos_count(const Rows &nb, long long n, const double *pos, const double *
                   unsigned *err, cudaStream_t st) {
     if (n <= 0) return;
     const DpArgs A{nb, n, pos, w, idx, start_n, start_xy, coeff, ntrans, trans};
-    k_dp_count<<<ceil_div(n, TB), TB, 0, st>>>(A, nblocks, err);
+    k_dp_count<<<ceil_div(n, CELLS), TB, 0, st>>>(A, nblocks, err);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
 }
@@ -299,7 +320,7 @@ void derpos_write(const Rows &nb, long long n, const double *pos, const double *
                   long long *off, long long *cols, double *vals, double *v, cudaStream_t st) {
     if (n <= 0) return;
     const DpArgs A{nb, n, pos, w, idx, start_n, start_xy, coeff, ntrans, trans};
-    k_dp_write<<<ceil_div(n, TB), TB, 0, st>>>(A, boff, off, cols, vals, v);
+    k_dp_write<<<ceil_div(n, CELLS), TB, 0, st>>>(A, boff, off, cols, vals, v);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
 }
