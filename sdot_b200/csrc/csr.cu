@@ -1,117 +1,156 @@
 // Hessian row assembly (see csr.cuh).
 #include "csr.cuh"
 
+#include <climits>
+
 namespace sdot {
 
 namespace {
 
 constexpr int TB = 256;
 
-// Merging never lengthens a row.  A side-buffer row whose merged count fits
-// the ELL width is moved to its ELL slots, so that Rows::colp (which picks
-// the storage from the count) stays consistent.
-// STAGE (2D rows, short): rows of at most SM_ROW entries (every row of the
-// fast tier) are sorted in shared memory: one gather of idx per entry, then
-// the insertion sort and the merge on the staged copy (24% faster on the 1M
-// 2D mix); longer rows, and every row without STAGE (3D rows are longer, and
-// the staging area would cost them occupancy), are sorted in place.
-constexpr int SM_ROW = 16;
+// Rows are sorted by counting: an entry's place is the number of smaller
+// columns in its row, so every entry finds it for itself from the row's keys
+// (original columns) in shared memory.  L lanes take a row of up to L E entries
+// (8 lanes in 2D, where a row has 7 on average, 16 in 3D, where it has 16);
+// rows longer than that a whole warp, one after another, up to SM_LONG entries,
+// and longer ones one lane by insertion in place.
+// Bound by the latency of two dependent gathers at small n and by their
+// sectors at large n.  In 3D against insertion in global memory by a thread a
+// row (with what follows it): 200,000 Diracs 300 -> 132 us, 20,000 clustered
+// ones (rows of up to 200 entries) 190 -> 36, 20,000 uniform ones 103 -> 34.
 constexpr int SM_TB = 128;
+constexpr int SM_E = 4;
+constexpr int SM_LONG = 256;
+constexpr int SM_ROW = 16;
+// 2D diagrams of more Diracs have a thread per row instead (k_sort_merge_staged):
+// 10,000 Diracs 26 us by lanes and 34 us by threads with what follows, 147,000
+// 58 and 56, 1M 286 and 212.
+constexpr long long SM_LANES_2D = 131072;
 
-template <bool STAGE>
-__global__ void __launch_bounds__(STAGE ? SM_TB : TB) k_sort_merge(Rows R, long long n, const int *idx,
-                                                                   long long *cnt_orig) {
-    __shared__ int s_key[STAGE ? SM_ROW * SM_TB : 1], s_col[STAGE ? SM_ROW * SM_TB : 1];
-    __shared__ double s_val[STAGE ? SM_ROW * SM_TB : 1];
-    const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const int m = R.cnt[s];
-#ifdef SDOT_CHECKS
-    if (m < 0 || m > 4096 || (m > R.cap && (R.side[s] < 0 || R.side[s] + m > R.side_cap))) {
-        check_fail(20, __LINE__, m);
-        R.cnt[s] = 0;
-        cnt_orig[idx[s]] = 0;
-        return;
+// Sorts and merges row s of m <= L E entries with the L lanes of `mask`; key:
+// room for m.  Merging never lengthens a row; a side-buffer row whose merged
+// count fits the ELL width is moved to its ELL slots, so that Rows::colp (which
+// picks the storage from the count) stays consistent.
+template <int L, int E>
+__device__ __forceinline__ void sort_row(const Rows &R, long long s, int m, const int *idx, long long *cnt_orig, int lane,
+                                         unsigned mask, int *key) {
+    int c[E], place[E];
+    double v[E];
+    bool head[E];
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        const int k = lane + L * q;
+        if (k >= m) continue;
+        c[q] = *R.colp(s, k);
+        v[q] = *R.valp(s, k);
+        key[k] = idx[c[q]];
     }
+    __syncwarp(mask);
+    int gone = 0;
+    auto count = [&](bool first) {
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            const int k = lane + L * q;
+            if (k >= m || (!first && !head[q])) continue;
+            const int mine = key[k];
+            int p = 0;
+            bool again = false;
+            if (first) head[q] = true;
+            for (int e = 0; e < m; ++e) {
+                const int ke = key[e];
+                p += ke < mine;
+                if (first && ke == mine) {
+                    if (e < k) head[q] = false;
+                    again |= e > k;
+                }
+            }
+            place[q] = p;
+            if (first && !head[q]) ++gone;
+            if (!first || !again || !head[q]) continue;
+            // the sum of the equal columns' values, smallest first
+            double sum = 0, last = 0;
+            int at = -1;
+            bool number = true;
+            for (int done = 0;; ++done) {
+                double best = 0;
+                int b = -1;
+                for (int e = 0; e < m; ++e) {
+                    if (key[e] != mine) continue;
+                    const double x = *R.valp(s, e);
+                    number &= x == x;
+                    const bool left = !done || x > last || (x == last && e > at);
+                    if (left && (b < 0 || x < best)) {
+                        best = x;
+                        b = e;
+                    }
+                }
+                if (b < 0 || !number) break;
+                sum = done ? sum + best : best;
+                last = best;
+                at = b;
+            }
+            v[q] = number ? sum : nan("");
+        }
+    };
+    count(true);
+    if (__any_sync(mask, gone)) {
+        // without the merged ones
+#pragma unroll
+        for (int q = 0; q < E; ++q)
+            if (lane + L * q < m && !head[q]) key[lane + L * q] = INT_MAX;
+        __syncwarp(mask);
+        count(false);
+#pragma unroll
+        for (int o = L / 2; o; o >>= 1) gone += __shfl_xor_sync(mask, gone, o);
+    }
+    __syncwarp(mask);
+    const int o = m - gone;
+    const bool side = o > R.cap;
+#pragma unroll
+    for (int q = 0; q < E; ++q) {
+        if (lane + L * q >= m || !head[q]) continue;
+        const long long to = side ? R.side[s] + place[q] : place[q] * R.stride + s;
+        (side ? R.side_col : R.col)[to] = c[q];
+        (side ? R.side_val : R.val)[to] = v[q];
+    }
+    if (lane == 0) {
+        R.cnt[s] = o;
+        cnt_orig[idx[s]] = o;
+    }
+}
+
+// The same in place by one lane (a row of any length).
+__device__ void sort_row_serial(const Rows &R, long long s, int m, const int *idx, long long *cnt_orig) {
+    for (int i = 1; i < m; ++i) {
+        const int c = *R.colp(s, i);
+        const double v = *R.valp(s, i);
+        const int oc = idx[c];
+        int j = i - 1;
+        while (j >= 0) {
+            const int cj = *R.colp(s, j);
+            const int ocj = idx[cj];
+            const double vj = *R.valp(s, j);
+            if (ocj < oc || (ocj == oc && !(vj > v))) break;
+            *R.colp(s, j + 1) = cj;
+            *R.valp(s, j + 1) = vj;
+            --j;
+        }
+        *R.colp(s, j + 1) = c;
+        *R.valp(s, j + 1) = v;
+    }
+    // merge equal columns
+    int o = 0;
     for (int i = 0; i < m; ++i) {
         const int c = *R.colp(s, i);
-        if (c < 0 || c >= n) {
-            check_fail(21, __LINE__, c);
-            *R.colp(s, i) = int(s);
+        const double v = *R.valp(s, i);
+        if (i + 1 < m && *R.colp(s, i + 1) == c) {
+            *R.valp(s, i + 1) += v;
+            continue;
         }
-    }
-#endif
-    int o = 0;
-    if (STAGE && m <= SM_ROW) {
-        // entry i of this thread at [i * SM_TB + t]: no bank conflicts
-        const int t = threadIdx.x;
-        for (int i = 0; i < m; ++i) {
-            const int c = *R.colp(s, i);
-            s_col[i * SM_TB + t] = c;
-            s_val[i * SM_TB + t] = *R.valp(s, i);
-            s_key[i * SM_TB + t] = idx[c];
-        }
-        // insertion sort by (original column, value), as below
-        for (int i = 1; i < m; ++i) {
-            const int oc = s_key[i * SM_TB + t], c = s_col[i * SM_TB + t];
-            const double v = s_val[i * SM_TB + t];
-            int j = i - 1;
-            while (j >= 0) {
-                const int ocj = s_key[j * SM_TB + t];
-                const double vj = s_val[j * SM_TB + t];
-                if (ocj < oc || (ocj == oc && !(vj > v))) break;
-                s_key[(j + 1) * SM_TB + t] = ocj;
-                s_col[(j + 1) * SM_TB + t] = s_col[j * SM_TB + t];
-                s_val[(j + 1) * SM_TB + t] = vj;
-                --j;
-            }
-            s_key[(j + 1) * SM_TB + t] = oc;
-            s_col[(j + 1) * SM_TB + t] = c;
-            s_val[(j + 1) * SM_TB + t] = v;
-        }
-        // merge equal columns (each into the next) and write back
-        for (int i = 0; i < m; ++i) {
-            const int c = s_col[i * SM_TB + t];
-            const double v = s_val[i * SM_TB + t];
-            if (i + 1 < m && s_col[(i + 1) * SM_TB + t] == c) {
-                s_val[(i + 1) * SM_TB + t] += v;
-                continue;
-            }
-            *R.colp(s, o) = c;
-            *R.valp(s, o) = v;
-            ++o;
-        }
-    } else {
-        // insertion sort in place
-        for (int i = 1; i < m; ++i) {
-            const int c = *R.colp(s, i);
-            const double v = *R.valp(s, i);
-            const int oc = idx[c];
-            int j = i - 1;
-            while (j >= 0) {
-                const int cj = *R.colp(s, j);
-                const int ocj = idx[cj];
-                const double vj = *R.valp(s, j);
-                if (ocj < oc || (ocj == oc && !(vj > v))) break;
-                *R.colp(s, j + 1) = cj;
-                *R.valp(s, j + 1) = vj;
-                --j;
-            }
-            *R.colp(s, j + 1) = c;
-            *R.valp(s, j + 1) = v;
-        }
-        // merge equal columns
-        for (int i = 0; i < m; ++i) {
-            const int c = *R.colp(s, i);
-            const double v = *R.valp(s, i);
-            if (i + 1 < m && *R.colp(s, i + 1) == c) {
-                *R.valp(s, i + 1) += v;
-                continue;
-            }
-            *R.colp(s, o) = c;
-            *R.valp(s, o) = v;
-            ++o;
-        }
+        *R.colp(s, o) = c;
+        *R.valp(s, o) = v;
+        ++o;
     }
     if (m > R.cap && o <= R.cap) {
         for (int k = 0; k < o; ++k) {
@@ -120,6 +159,112 @@ __global__ void __launch_bounds__(STAGE ? SM_TB : TB) k_sort_merge(Rows R, long 
             R.col[k * R.stride + s] = c;
             R.val[k * R.stride + s] = v;
         }
+    }
+    R.cnt[s] = o;
+    cnt_orig[idx[s]] = o;
+}
+
+#ifdef SDOT_CHECKS
+// Row s checked by lane `lane` of `lanes`: its length (0 if it cannot be), columns out of range replaced.
+__device__ int check_row(const Rows &R, long long s, long long n, int m, int lane, int lanes) {
+    if (m < 0 || m > 4096 || (m > R.cap && (R.side[s] < 0 || R.side[s] + m > R.side_cap))) {
+        if (lane == 0) check_fail(20, __LINE__, m);
+        return 0;
+    }
+    for (int i = lane; i < m; i += lanes) {
+        const int c = *R.colp(s, i);
+        if (c < 0 || c >= n) {
+            check_fail(21, __LINE__, c);
+            *R.colp(s, i) = int(s);
+        }
+    }
+    return m;
+}
+#endif
+
+template <int L>
+__global__ void __launch_bounds__(SM_TB) k_sort_merge(Rows R, long long n, const int *idx, long long *cnt_orig) {
+    __shared__ int keys[SM_TB / 32][SM_LONG];
+    const int lane = threadIdx.x & (L - 1), wl = threadIdx.x & 31;
+    const unsigned mask = (L == 32 ? ~0u : (1u << L) - 1u) << (wl - lane);
+    const long long s = (blockIdx.x * (long long)SM_TB + threadIdx.x) / L;
+    int m = s < n ? R.cnt[s] : 0;
+#ifdef SDOT_CHECKS
+    if (s < n) m = check_row(R, s, n, m, lane, L);
+    __syncwarp(mask);
+#endif
+    int *key = keys[threadIdx.x / 32];
+    const bool fits = m <= L * SM_E;
+    if (s < n && fits) sort_row<L, SM_E>(R, s, m, idx, cnt_orig, lane, mask, key + (wl - lane) * SM_E);
+    __syncwarp();
+    unsigned longer = __ballot_sync(0xffffffffu, lane == 0 && s < n && !fits);
+    for (; longer; longer &= longer - 1) {
+        const int from = __ffs(int(longer)) - 1;
+        const long long sl = __shfl_sync(0xffffffffu, s, from);
+        const int ml = __shfl_sync(0xffffffffu, m, from);
+        if (ml <= SM_LONG)
+            sort_row<32, SM_LONG / 32>(R, sl, ml, idx, cnt_orig, wl, 0xffffffffu, key);
+        else if (wl == 0)
+            sort_row_serial(R, sl, ml, idx, cnt_orig);
+        __syncwarp();
+    }
+}
+
+// The rows of a large 2D diagram, a thread each: rows of at most SM_ROW entries
+// (every row of the fast tier) by insertion in shared memory, longer ones in
+// place.  Neighbouring threads read and write neighbouring entries, which the
+// lanes of a row do not.
+__global__ void __launch_bounds__(SM_TB) k_sort_merge_staged(Rows R, long long n, const int *idx, long long *cnt_orig) {
+    __shared__ int s_key[SM_ROW * SM_TB], s_col[SM_ROW * SM_TB];
+    __shared__ double s_val[SM_ROW * SM_TB];
+    const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    int m = R.cnt[s];
+#ifdef SDOT_CHECKS
+    m = check_row(R, s, n, m, 0, 1);
+#endif
+    if (m > SM_ROW) {
+        sort_row_serial(R, s, m, idx, cnt_orig);
+        return;
+    }
+    int o = 0;
+    // entry i of this thread at [i * SM_TB + t]: no bank conflicts
+    const int t = threadIdx.x;
+    for (int i = 0; i < m; ++i) {
+        const int c = *R.colp(s, i);
+        s_col[i * SM_TB + t] = c;
+        s_val[i * SM_TB + t] = *R.valp(s, i);
+        s_key[i * SM_TB + t] = idx[c];
+    }
+    // insertion sort by (original column, value)
+    for (int i = 1; i < m; ++i) {
+        const int oc = s_key[i * SM_TB + t], c = s_col[i * SM_TB + t];
+        const double v = s_val[i * SM_TB + t];
+        int j = i - 1;
+        while (j >= 0) {
+            const int ocj = s_key[j * SM_TB + t];
+            const double vj = s_val[j * SM_TB + t];
+            if (ocj < oc || (ocj == oc && !(vj > v))) break;
+            s_key[(j + 1) * SM_TB + t] = ocj;
+            s_col[(j + 1) * SM_TB + t] = s_col[j * SM_TB + t];
+            s_val[(j + 1) * SM_TB + t] = vj;
+            --j;
+        }
+        s_key[(j + 1) * SM_TB + t] = oc;
+        s_col[(j + 1) * SM_TB + t] = c;
+        s_val[(j + 1) * SM_TB + t] = v;
+    }
+    // merge equal columns (each into the next) and write back
+    for (int i = 0; i < m; ++i) {
+        const int c = s_col[i * SM_TB + t];
+        const double v = s_val[i * SM_TB + t];
+        if (i + 1 < m && s_col[(i + 1) * SM_TB + t] == c) {
+            s_val[(i + 1) * SM_TB + t] += v;
+            continue;
+        }
+        *R.colp(s, o) = c;
+        *R.valp(s, o) = v;
+        ++o;
     }
     R.cnt[s] = o;
     cnt_orig[idx[s]] = o;
@@ -245,13 +390,16 @@ void csr_read_checks(unsigned long long out[3]) {
 
 void csr_sort_merge(const Rows &R, long long n, const int *idx, long long *cnt_orig, bool short_rows, cudaStream_t st) {
     if (n <= 0) return;
-    if (short_rows)
-        k_sort_merge<true><<<ceil_div(n, SM_TB), SM_TB, 0, st>>>(R, n, idx, cnt_orig);
+    if (short_rows && n > SM_LANES_2D)
+        k_sort_merge_staged<<<ceil_div(n, SM_TB), SM_TB, 0, st>>>(R, n, idx, cnt_orig);
+    else if (short_rows)
+        k_sort_merge<8><<<ceil_div(n * 8, SM_TB), SM_TB, 0, st>>>(R, n, idx, cnt_orig);
     else
-        k_sort_merge<false><<<ceil_div(n, TB), TB, 0, st>>>(R, n, idx, cnt_orig);
+        k_sort_merge<16><<<ceil_div(n * 16, SM_TB), SM_TB, 0, st>>>(R, n, idx, cnt_orig);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
 }
+
 void csr_write(const Rows &R, long long n, const int *idx, const long long *offsets, long long *cols, double *vals,
                cudaStream_t st) {
     if (n <= 0) return;
