@@ -46,7 +46,10 @@ static __device__ unsigned long long sdot_work[8];
 namespace {
 
 constexpr int STACK = 64;   // traversal stack (depth <= 17 levels, <= 3 pending siblings each)
-constexpr int MID_WARPS = 148 * 16;   // warps of the warp tier in shared memory (16 per SM: 128 registers)
+// Warps (blocks) per SM of the warp tier in shared memory: 12 / 16 / 20 / 24 /
+// 28 solve 60,000 clustered Diracs in 321 / 313 / 309 / 306 / 308 ms.
+constexpr int MID_BLOCKS = 24;
+constexpr int MID_WARPS = 148 * MID_BLOCKS;
 constexpr int WTIER_WARPS = 148 * 4;  // warps of the warp tier in global scratch (few cells)
 
 // Records the first failed consistency guard and flags the error word; the
@@ -1142,23 +1145,29 @@ __device__ int finish_warp(const Cell2DArgs &A, long long s, const PolyView<doub
 // 60,000 clustered Diracs: 8,700 cells pass 13 vertices while they are built (23
 // at most at their end).  With every polygon in global scratch, lane 0
 // integrating and one Dirac at a time, the cells took 3.1 ms at the starting
-// weights and 7.7 ms at the solved ones, now 1.4 and 3.8 ms.
+// weights and 7.7 ms at the solved ones, then 1.4 and 3.8 ms; with one warp a
+// block, more of them and a cursor in place of fixed shares 3.5 ms at the solved
+// ones (the longest walks last: a cell takes up to a millisecond).
 template <int MODE, bool BALL, bool MID>
-__global__ void __launch_bounds__(128, MID ? 4 : 1) k_cells2d_wtier(const Cell2DArgs A, double *scratch, int nwarps,
-                                                                    const int *list, const int *list_cnt,
-                                                                    int *next_list, int *next_cnt) {
+__global__ void __launch_bounds__(32, !MID ? 4 : BALL || (MODE != DM_SINGLE && MODE != DM_PERIODIC) ? 16 : MID_BLOCKS)
+    k_cells2d_wtier(const Cell2DArgs A, double *scratch, const int *list, const int *list_cnt, int *cursor,
+                    int *next_list, int *next_cnt) {
     constexpr int CAP = MID ? CAP_MID_2D : CAP_HUGE_2D;
     extern __shared__ double wmem[];
-    __shared__ int wstack[4][STACK];
-    const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
-    const int gw = blockIdx.x * 4 + wb;
-    if (gw >= nwarps) return;
-    WarpScratch W(MID ? wmem + wb * warp_scratch_doubles(CAP) : scratch + (long long)gw * warp_scratch_doubles(CAP), CAP);
+    __shared__ int wstack[STACK];
+    const int lane = threadIdx.x;
+    WarpScratch W(MID ? wmem : scratch + (long long)blockIdx.x * warp_scratch_doubles(CAP), CAP);
     const int cnt = list ? *list_cnt : int(A.n);
-    for (int i = gw; i < cnt; i += nwarps) {
+    // the first cells by block, the others as blocks come free
+    auto fetch = [&] {
+        int k = 0;
+        if (lane == 0) k = atomicAdd(cursor, 1);
+        return int(gridDim.x) + __shfl_sync(0xffffffffu, k, 0);
+    };
+    for (int i = blockIdx.x; i < cnt; i = fetch()) {
         const long long s = list ? list[i] : i;
         const double c0x = A.pos[2 * s], c0y = A.pos[2 * s + 1];
-        const int n = build_cell_warp<MODE == DM_PERIODIC>(A, s, W.cell, CAP, c0x, c0y, A.w[s], wstack[wb]);
+        const int n = build_cell_warp<MODE == DM_PERIODIC>(A, s, W.cell, CAP, c0x, c0y, A.w[s], wstack);
         int failed = 0;  // 1: a capacity was exceeded, 2: no room for the row
         if constexpr ((MODE == DM_SINGLE || MODE == DM_PERIODIC) && !BALL) {
             failed = finish_warp(A, s, W.cell, n);
@@ -1195,7 +1204,7 @@ __global__ void k_all_cells(int *list, int *cnt, long long n) {
 // Counters the fast kernel appends to: zeroed before every launch of it.
 void reset_overflow(const Cell2DArgs &a, cudaStream_t st) {
     SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt, 0, sizeof(int), st));
-    SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt2, 0, sizeof(int), st));
+    SDOT_CUDA(cudaMemsetAsync(a.ovf_cnt2, 0, 3 * sizeof(int), st));  // and the cursors
     if (a.rows.side_used) SDOT_CUDA(cudaMemsetAsync(a.rows.side_used, 0, sizeof(unsigned long long), st));
     if (a.nb.side_used) SDOT_CUDA(cudaMemsetAsync(a.nb.side_used, 0, sizeof(unsigned long long), st));
 }
@@ -1238,12 +1247,12 @@ void launch_all(const Cell2DArgs &a, void *scratch, cudaStream_t st) {
     // the last tier at once
     const bool mid = a.start_n <= CAP_MID_2D - 16;
     if (mid) {
-        k_cells2d_wtier<MODE, BALL, true><<<MID_WARPS / 4, 128, 4 * warp_scratch_doubles(CAP_MID_2D) * sizeof(double),
-                                            st>>>(a, nullptr, MID_WARPS, list, cnt, a.ovf_list2, a.ovf_cnt2);
+        k_cells2d_wtier<MODE, BALL, true><<<MID_WARPS, 32, warp_scratch_doubles(CAP_MID_2D) * sizeof(double), st>>>(
+            a, nullptr, list, cnt, a.ovf_cnt2 + 1, a.ovf_list2, a.ovf_cnt2);
         note_launch();
     }
-    k_cells2d_wtier<MODE, BALL, false><<<WTIER_WARPS / 4, 128, 0, st>>>(
-        a, static_cast<double *>(scratch), WTIER_WARPS, mid ? a.ovf_list2 : a.ovf_list, mid ? a.ovf_cnt2 : a.ovf_cnt,
+    k_cells2d_wtier<MODE, BALL, false><<<WTIER_WARPS, 32, 0, st>>>(
+        a, static_cast<double *>(scratch), mid ? a.ovf_list2 : a.ovf_list, mid ? a.ovf_cnt2 : a.ovf_cnt, a.ovf_cnt2 + 2,
         nullptr, nullptr);
     note_launch();
     SDOT_CUDA(cudaGetLastError());

@@ -18,11 +18,9 @@ enum DomainMode : int { DM_SINGLE = 0, DM_MULTI = 1, DM_IMAGE = 2, DM_IMAGE6 = 3
 // overflow it are rebuilt by a warp each, with polygons of up to 64 vertices in
 // shared memory, and those that overflow this by a warp each with polygons in
 // global scratch.  Beyond that the call reports ST_CAPACITY.
-// 13 fast vertices (260 B of shared memory per cell): with the fast
-// kernel's shared-memory carveout an SM holds more warps than with 14 or 16,
-// and the few cells of 14 or more vertices on the 1M clustered mix cost less
-// in the warp tier than the smaller occupancy would (measured: 13 vertices
-// 4.13 ms, 12: 4.16, 14: 4.23, 16: 4.54).
+// 13 fast vertices (260 B of shared memory per cell): with more an SM holds
+// fewer warps, and the few cells of 14 or more vertices on the 1M clustered mix
+// cost less in the warp tier than the smaller occupancy would.
 constexpr int CAP_FAST_2D = 13;
 static_assert(CAP_FAST_2D <= 32, "the fast tier keeps one bit per vertex in a 32-bit mask");
 constexpr int CAP_MID_2D = 64;
@@ -123,7 +121,7 @@ struct Cell2DArgs {
     int *ovf_list = nullptr;
     int *ovf_cnt = nullptr;
     int *ovf_list2 = nullptr;
-    int *ovf_cnt2 = nullptr;
+    int *ovf_cnt2 = nullptr;       // its length, then the cursors of the two warp tiers (3 ints)
     // raster outputs (DM_RASTER): per pixel (x-fastest) the sums of m x_i,
     // m y_i and m over the cells i, m the integral of cell i over the pixel
     // (ras, 3 doubles per pixel), and the largest caller index of a cell of
