@@ -672,11 +672,12 @@ namespace {
 // dependent reads of the L2 and the block's sum).  Blocks of 128, 256, 512
 // threads: 32 / 29 / 35 us and 59 / 45 / 52 us.  A hardware cluster of 16
 // blocks has a barrier of 0.7 us, but its 16 SMs take 8 us for a phase of 10,000
-// rows.  Two blocks per SM pay from several 100,000 rows on, where the passes
-// are bound by the loads in flight (Newton at 1M rows 1.79 -> 1.56 s, at
-// 200,000 0.247 -> 0.262 s).
+// rows.  From several 100,000 rows on the passes are bound by the loads in flight
+// and blocks of 512 pay (Newton at 300,000 / 500,000 / 1M rows, 1M clamped
+// clusters: 0.142 / 0.255 / 1.53 / 1.86 s; with 256 0.132 / 0.280 / 1.85 / 2.17;
+// two blocks of 256 per SM - / 0.278 / 1.61 / 2.16; more of them spill).
 constexpr int MGT = 256;
-constexpr int MANY_PER_SM = 2;
+constexpr int MGT_MANY = 512;
 constexpr long long MANY_ROWS = 400000;
 constexpr int SOLO = 512;       // rows of the largest level one block does alone
 constexpr int SOLO_ALL = 640;   // rows of all such levels together (512 + 64 + 8, and a margin)
@@ -716,13 +717,16 @@ __device__ void restrict_row(double t, long long i, long long n, double *rc) {
 
 // The phases.  Each is a function of its own: in one body the compiler keeps
 // the addresses of all of them in registers and spills inside the loops (1.6 KB
-// a thread; the barriers empty the L1 cache that would hold them).
+// a thread; the barriers empty the L1 cache that would hold them), and they take
+// the block's size at run time: compiled for each size, with more registers for
+// the smaller, they took 4% longer at 10,000 rows.
 template <class M, class T>
 __device__ __noinline__ double phase_a(const PcgArgs<M, T> &a, const T *pold, T *pnew, double beta, double gd) {
-    const long long step = (long long)gridDim.x * MGT;
+    const int nt = blockDim.x;
+    const long long step = (long long)gridDim.x * nt;
     auto pv = [&](long long j) { return double(T(double(a.z[j]) + beta * double(pold[j]))); };
     double pq = 0;
-    for (long long i = blockIdx.x * (long long)MGT + threadIdx.x; i < a.n; i += step) {
+    for (long long i = blockIdx.x * (long long)nt + threadIdx.x; i < a.n; i += step) {
         const double pi = pv(i);
         double v = a.A.row_sum(i, pv);
         if (i == a.gauge) v += gd * pi;
@@ -738,10 +742,11 @@ __device__ __noinline__ double phase_a(const PcgArgs<M, T> &a, const T *pold, T 
 template <class M, class T>
 __device__ __noinline__ double phase_b(const PcgArgs<M, T> &a, const T *p, const T *sold, T *snew, double alpha,
                                        double gd, bool update) {
-    const long long step = (long long)gridDim.x * MGT;
+    const int nt = blockDim.x;
+    const long long step = (long long)gridDim.x * nt;
     auto sv = [&](long long j) { return double(T(double(sold[j]) - alpha * double(a.qs[j]))); };
     double rs = 0;
-    for (long long i0 = blockIdx.x * (long long)MGT; i0 < a.n; i0 += step) {
+    for (long long i0 = blockIdx.x * (long long)nt; i0 < a.n; i0 += step) {
         const long long i = i0 + threadIdx.x;
         double t = 0;
         if (i < a.n) {
@@ -765,11 +770,12 @@ __device__ __noinline__ double phase_b(const PcgArgs<M, T> &a, const T *p, const
 
 template <class M, class T>
 __device__ __noinline__ double phase_d(const PcgArgs<M, T> &a, const T *s, double gd) {
-    const long long step = (long long)gridDim.x * MGT;
+    const int nt = blockDim.x;
+    const long long step = (long long)gridDim.x * nt;
     const double *zc = a.pl.lev[1].zo;
     auto zv = [&](long long j) { return double(s[j]) + zc[j / MG_BF]; };
     double rs = 0;
-    for (long long i = blockIdx.x * (long long)MGT + threadIdx.x; i < a.n; i += step) {
+    for (long long i = blockIdx.x * (long long)nt + threadIdx.x; i < a.n; i += step) {
         const double zi = zv(i), ri = double(a.r[i]);
         double v = a.A.row_sum(i, zv);
         if (i == a.gauge) v += gd * zi;
@@ -808,9 +814,9 @@ struct SoloMem {
 template <class T>
 __device__ __noinline__ void coarse_solo(const MgPlan<T> &pl, int solo, SoloMem &S) {
     double *sr = S.r, *sz = S.z;
-    const int tid = threadIdx.x, L = pl.L;
+    const int tid = threadIdx.x, nt = blockDim.x, L = pl.L;
     const int n0 = int(pl.lev[solo].n);
-    for (int i = tid; i < n0; i += MGT) sr[i] = pl.lev[solo].r[i];
+    for (int i = tid; i < n0; i += nt) sr[i] = pl.lev[solo].r[i];
     __syncthreads();
     int at = 0;
     for (int l = solo; l < L; ++l) {
@@ -819,7 +825,7 @@ __device__ __noinline__ void coarse_solo(const MgPlan<T> &pl, int solo, SoloMem 
         const int nl = int(v.n);
         const EllViewT<double> A{v.cnt, v.col, v.val, v.n};
         at += nl;
-        for (int i0 = 0; i0 < nl; i0 += MGT) {
+        for (int i0 = 0; i0 < nl; i0 += nt) {
             const int i = i0 + tid;
             double t = 0;
             if (i < nl) t = r[i] - A.row_sum(i, [&](long long j) { return MG_OMEGA * dinv[j] * r[j]; });
@@ -842,14 +848,14 @@ __device__ __noinline__ void coarse_solo(const MgPlan<T> &pl, int solo, SoloMem 
         const double *r = sr + at, *dinv = S.dinv + at;
         const EllViewT<double> A{v.cnt, v.col, v.val, v.n};
         auto zv = [&](long long j) { return MG_OMEGA * dinv[j] * r[j] + zc[j / MG_B]; };
-        for (int i = tid; i < nl; i += MGT) sz[at + i] = zv(i) + MG_OMEGA * dinv[i] * (r[i] - A.row_sum(i, zv));
+        for (int i = tid; i < nl; i += nt) sz[at + i] = zv(i) + MG_OMEGA * dinv[i] * (r[i] - A.row_sum(i, zv));
         __syncthreads();
     }
-    for (int i = tid; i < n0; i += MGT) pl.lev[solo].zo[i] = sz[i];
+    for (int i = tid; i < n0; i += nt) pl.lev[solo].zo[i] = sz[i];
 }
 
-template <class M, class T, int PER_SM>
-__global__ void __launch_bounds__(MGT, PER_SM) k_pcg_mg(const __grid_constant__ PcgArgs<M, T> param) {
+template <class M, class T, int NT>
+__global__ void __launch_bounds__(NT, 1) k_pcg_mg(const __grid_constant__ PcgArgs<M, T> param) {
     __shared__ double sh[33];
     __shared__ SoloMem solo_mem;
     // the arguments in shared memory: read through the L1 cache, which the
@@ -857,11 +863,11 @@ __global__ void __launch_bounds__(MGT, PER_SM) k_pcg_mg(const __grid_constant__ 
     using Args = PcgArgs<M, T>;
     static_assert(sizeof(Args) % 8 == 0, "copied by 8 bytes");
     __shared__ double arg_mem[sizeof(Args) / 8];
-    for (int i = threadIdx.x; i < int(sizeof(Args) / 8); i += MGT)
+    for (int i = threadIdx.x; i < int(sizeof(Args) / 8); i += NT)
         arg_mem[i] = reinterpret_cast<const double *>(&param)[i];
     const Args &a = *reinterpret_cast<const Args *>(arg_mem);
     __syncthreads();
-    const int tid = threadIdx.x, L = a.pl.L, t0 = blockIdx.x * MGT, step = gridDim.x * MGT;
+    const int tid = threadIdx.x, L = a.pl.L, t0 = blockIdx.x * NT, step = gridDim.x * NT;
     const double gd = a.gauge >= 0 ? a.scal[S_GDIAG] : 0.0;
     double *p_pq = a.partial, *p_rr = a.partial + gridDim.x, *p_rz = a.partial + 2 * gridDim.x;
     // the levels [solo, L] are one block's
@@ -869,10 +875,10 @@ __global__ void __launch_bounds__(MGT, PER_SM) k_pcg_mg(const __grid_constant__ 
     while (solo > 1 && a.pl.lev[solo - 1].n <= SOLO) --solo;
     if (blockIdx.x == 0) {
         const int nc = int(a.pl.lev[L].n);
-        for (int i = tid; i < nc * nc; i += MGT) solo_mem.cinv[i] = a.pl.cinv[i];
+        for (int i = tid; i < nc * nc; i += NT) solo_mem.cinv[i] = a.pl.cinv[i];
         int at = 0;
         for (int l = solo; l < L; at += int(a.pl.lev[l].n), ++l)
-            for (int i = tid; i < int(a.pl.lev[l].n); i += MGT) solo_mem.dinv[at + i] = a.pl.lev[l].dinv[i];
+            for (int i = tid; i < int(a.pl.lev[l].n); i += NT) solo_mem.dinv[at + i] = a.pl.lev[l].dinv[i];
         __syncthreads();
     }
     unsigned target = 0;
@@ -954,9 +960,10 @@ PcgResult pcg_run_mg(const M &A, long long n, long long gauge_row, const T *b, T
     SDOT_CUDA(cudaGetDevice(&dev));
     SDOT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const bool many = n > MANY_ROWS;
-    void (*const kernel)(PcgArgs<M, T>) = many ? k_pcg_mg<M, T, MANY_PER_SM> : k_pcg_mg<M, T, 1>;
-    // all blocks are resident: the kernels are compiled for these numbers per SM
-    const int g = int(std::min<long long>((n + MGT - 1) / MGT, std::min(many ? MANY_PER_SM * sms : sms, 2 * PCG_BLOCKS)));
+    const int nt = many ? MGT_MANY : MGT;
+    void (*const kernel)(PcgArgs<M, T>) = many ? k_pcg_mg<M, T, MGT_MANY> : k_pcg_mg<M, T, MGT>;
+    // all blocks are resident: one per SM
+    const int g = int(std::min<long long>((n + nt - 1) / nt, std::min(sms, 2 * PCG_BLOCKS)));
     k_init_mg<T><<<grid_of(n), TB, 0, st>>>(b, x, w.r, pl.s0, w.dinv, pl.p1, w.q, pl.qs, w.z, n);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
@@ -971,7 +978,7 @@ PcgResult pcg_run_mg(const M &A, long long n, long long gauge_row, const T *b, T
         a.iters = std::min(chunk, max_iter - it);
         SDOT_CUDA(cudaMemsetAsync(pl.sync, 0, 2 * sizeof(unsigned), st));
         void *args[] = {&a};
-        SDOT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(kernel), dim3(g), dim3(MGT), args, 0, st));
+        SDOT_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(kernel), dim3(g), dim3(nt), args, 0, st));
         note_launch();
         SDOT_CUDA(cudaMemcpyAsync(hs, w.scal, sizeof(hs), cudaMemcpyDeviceToHost, st));
         SDOT_CUDA(cudaStreamSynchronize(st));

@@ -299,3 +299,17 @@ def test_multilevel_solve_sizes(gpu_lib, dim, n):
     ref = w["jacobi", "fp64"]
     for x in w.values():
         assert np.abs(x - ref).max() <= 1e-9 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n", [400_001, 401_409])
+def test_multilevel_solve_larger_blocks(gpu_lib, n):
+    # more than 400,000 rows: blocks of 512 threads, a row more than the line
+    # and a ragged last block; the solved cells have their target masses
+    from sdot_b200.power_diagram import PowerDiagram
+
+    p = np.random.default_rng(5400 + n).random((n, 2))
+    g = PowerDiagram(p, np.zeros(n))
+    g.add_box_shape(np.zeros(2), np.ones(2))
+    rep = g.solve_weights(np.full(n, 1.0 / n), rel_mass_tol=1e-8)
+    assert rep["status"] == 0 and rep["pcg_levels"] > 0
+    assert np.abs(g.integrals() * n - 1).max() <= 1e-8
