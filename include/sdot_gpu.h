@@ -187,8 +187,8 @@ int sdot_get_image_of_cell_nums(sdot_ctx *ctx, const double *min_pt, const doubl
  * (the Hessian entry (0,0) doubled when there is no ball cut, .tcc:62-63),
  * solves H dw = m - target by preconditioned conjugate gradients on the
  * device and sets w -= tau dw.  The preconditioner is a multilevel V-cycle
- * over aggregates of 8 consecutive cells in Morton order (damped Jacobi
- * smoothing, exact coarsest solve) or plain Jacobi.
+ * over aggregates of 4, then 8, consecutive cells in Morton order (damped
+ * Jacobi smoothing, exact coarsest solve) or plain Jacobi.
  *   damping = 0: the reference rule: tau = 1; when a cell is empty the step
  *                is undone as w = 0.9 w_old + 0.1 w (.tcc:72-79).
  *   damping = 1: Kitagawa-Merigot-Thibert damping: tau halves until every

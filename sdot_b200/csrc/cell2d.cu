@@ -56,7 +56,7 @@ constexpr int WTIER_WARPS = 148 * 4;  // warps of the warp tier in global scratc
 // caller then skips the access.  Guards cover every index that comes from
 // data (tree nodes, leaf ranges, item offsets), so a corrupt input gives an
 // error status instead of a fault.
-SDOT_KFN void guard_fail(const Cell2DArgs &A, int code, long long s, long long value) {
+__device__ void guard_fail(const Cell2DArgs &A, int code, long long s, long long value) {
 #ifdef __CUDA_ARCH__
     const bool first = A.guard && atomicCAS(&A.guard[0], 0, code) == 0;
 #else

@@ -125,14 +125,6 @@ struct CaptureCount {
     CaptureCount &operator=(const CaptureCount &) = delete;
 };
 
-// Per-cell kernel bodies are device functions; a host build of them (for
-// CPU-side debugging of the kernels) is compiled with SDOT_HOST_KERNELS.
-#ifdef SDOT_HOST_KERNELS
-#define SDOT_KFN __host__ __device__
-#else
-#define SDOT_KFN __device__
-#endif
-
 // Sets bits of the sticky error word (atomically on the device).
 __host__ __device__ inline void flag_error(unsigned *word, unsigned bits) {
 #ifdef __CUDA_ARCH__
