@@ -23,10 +23,11 @@ _lib = None
 
 
 def build(force=False):
-    """Compile oracle/_ref/libsdot_ref.so when the reference tree is present."""
+    """Compile oracle/_ref/libsdot_ref.so when the reference tree is present (a
+    directory without the sources is not)."""
     if os.path.exists(REF_LIB) and not force:
         return REF_LIB
-    if not os.path.isdir(REF_TREE):
+    if not os.path.isdir(os.path.join(REF_TREE, "src", "sdot")):
         return None
     subprocess.run(["make", "-C", HERE, "ref", f"REF={REF_TREE}"], check=True, capture_output=True)
     return REF_LIB
