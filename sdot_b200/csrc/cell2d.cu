@@ -274,7 +274,8 @@ struct AreaSink {
 // The cell (n vertices; box [xmin, xmax] x [ymin, ymax], or what of it its disc
 // reaches) cut to a pixel, into `piece`; an edge keeps its vertex number in the
 // cell as its id, a pixel's edge gets PID_OWN.  Only the pixel's lines that
-// pass through the box cut.  Returns the number of vertices (n + 4 at most).
+// pass through the box cut.  Returns the number of vertices (piece.cap, at least
+// n + 4, at most).
 // The piece lies in memory of its own (shared in the fast tier) between short
 // loops; streamed through four nested clip stages and the disc's, each holding
 // its state in local memory, with 4 to 8 KB of spills a thread, 500,000 cells
@@ -292,7 +293,9 @@ __device__ __forceinline__ int clip_to_pixel(const PolyView<double> &piece, cons
     for (int side = 0; side < 4; ++side) {
         const bool y = side >= 2, hi = side & 1;
         const double c = y ? (hi ? y1 : y0) : (hi ? x1 : x0);
-        if (hi ? (y ? ymax : xmax) > c : (y ? ymin : xmin) < c) m = axis_cut(piece, m, y, c, hi ? -1.0 : 1.0, PID_OWN);
+        // (the other lines' room is kept)
+        if (hi ? (y ? ymax : xmax) > c : (y ? ymin : xmin) < c)
+            m = axis_cut(piece, m, y, c, hi ? -1.0 : 1.0, PID_OWN, piece.cap - 3 + side);
     }
     return m;
 }

@@ -61,21 +61,31 @@ struct CutFacts {
     }
 };
 
+SDOT_HD int popcount(unsigned v) {
+#ifdef __CUDA_ARCH__
+    return __popc(v);
+#else
+    return __builtin_popcount(v);
+#endif
+}
+// The place of the lowest bit set (-1: none).
+SDOT_HD int first_bit(unsigned v) {
+#ifdef __CUDA_ARCH__
+    return __ffs(int(v)) - 1;
+#else
+    return __builtin_ffs(int(v)) - 1;
+#endif
+}
+
 // The same facts from a bit mask of the outside vertices (bit k: vertex k;
 // polygons of at most 32 vertices).
 SDOT_HD CutFacts cut_facts(unsigned mask, int n) {
     CutFacts f;
     const unsigned valid = n >= 32 ? 0xffffffffu : ((1u << n) - 1u);
     const unsigned in = ~mask & valid;
-#ifdef __CUDA_ARCH__
-    f.nb_out = __popc(mask);
-    f.first_out = __ffs(int(mask)) - 1;
-    f.first_in = __ffs(int(in)) - 1;
-#else
-    f.nb_out = __builtin_popcount(mask);
-    f.first_out = __builtin_ffs(int(mask)) - 1;
-    f.first_in = __builtin_ffs(int(in)) - 1;
-#endif
+    f.nb_out = popcount(mask);
+    f.first_out = first_bit(mask);
+    f.first_in = first_bit(in);
     f.out1 = n > 1 && ((mask >> 1) & 1u);
     f.out_last = (mask >> (n - 1)) & 1u;
     return f;
@@ -341,47 +351,96 @@ SDOT_HD void bisector(T c0x, T c0y, T w0, T c1x, T c1y, T w1, T &ox, T &oy, T &n
     oy = c0y + x * ny;
 }
 
-#ifdef __CUDACC__
-// Cuts the polygon q (m vertices; room for m + 1) in place to the half-plane
-// s (coord - c) >= 0, coord = x if axis == 0 else y; the new edge along the line
-// gets the id `own`.  Returns the new count.  The vertex after the one being
-// looked at is held in registers: what is written does not pass it, as each
-// vertex written in addition leaves the half-plane before one that is dropped.
-// (Where rounding crosses the line more often than twice, no more is written
-// than fits.)
+// Cuts the polygon q (m vertices) in place to the half-plane s (coord - c) >= 0,
+// coord = x if axis == 0 else y; the new edge along the line gets the id `own`.
+// Returns the new count: m + 1 at most (there is room for it), or up to `room`
+// where that is more.
+// A run of vertices outside gives way to two on the line: A on the edge into the
+// run, B on the edge out of it.  The run of the farthest vertex goes first.  A
+// convex polygon has no other one but for rounding; where a side of the cell lies
+// on a pixel's line and its corners are several vertices at one place (a lattice
+// of Diracs over an image) there are some more, and each is cut in its turn, so
+// that the pixels on both sides of the line share out the side's length.  (Taken
+// edge by edge in one pass in place, the third crossing would be written over a
+// vertex not read yet.)  A vertex outside by rounding for which there is no room
+// stays.
+// The vertices keep their order; the polygon starts at its vertex 0 or, where
+// that one goes, at the B of its run.
 template <class P>
-__device__ __forceinline__ int axis_cut(const P &q, int m, int axis, double c, double s, int own) {
-    if (m == 0) return 0;
-    const double fx = q.X(0), fy = q.Y(0);
-    double ax = fx, ay = fy, va = s * ((axis == 0 ? ax : ay) - c);
-    int at = q.I(0), w = 0;
-    for (int k = 0; k < m; ++k) {
-        const bool more = k + 1 < m;
-        const double bx = more ? q.X(k + 1) : fx, by = more ? q.Y(k + 1) : fy;
-        const int bt = more ? q.I(k + 1) : 0;
-        const double vb = s * ((axis == 0 ? bx : by) - c);
-        const bool ina = va >= 0, inb = vb >= 0;
-        if (ina && w < q.cap) {
-            q.X(w) = ax;
-            q.Y(w) = ay;
-            q.I(w) = at;
-            ++w;
+SDOT_HD int axis_cut(const P &q, int m, int axis, double c, double s, int own, int room) {
+    auto val = [&](int k) { return s * ((axis == 0 ? q.X(k) : q.Y(k)) - c); };
+    for (bool first = true;; first = false) {
+        // the run: gone vertices from i1 on (cyclic) of the out outside
+        int i1 = -1, gone = 0, out = 0;
+        if (m <= 32) {
+            unsigned mask = 0;
+            for (int k = 0; k < m; ++k) mask |= unsigned(val(k) < 0) << k;
+            if (!mask) return m;
+            const unsigned starts = mask & ~(mask << 1 | mask >> (m - 1));
+            out = popcount(mask);
+            if (!starts) return 0;
+            if (!(starts & (starts - 1))) {
+                i1 = first_bit(starts);
+                gone = out;
+            }
         }
-        if (ina != inb && w < q.cap) {
-            const double t = va / (va - vb);
-            q.X(w) = axis == 0 ? c : ax + t * (bx - ax);
-            q.Y(w) = axis == 0 ? ay + t * (by - ay) : c;
-            q.I(w) = ina ? own : at;
-            ++w;
+        if (!gone) {
+            double low = 0;
+            out = 0;
+            for (int k = 0; k < m; ++k) {
+                const double v = val(k);
+                out += v < 0;
+                if (v < low) {
+                    low = v;
+                    i1 = k;
+                }
+            }
+            if (!out) return m;
+            if (out == m) return 0;
+            for (gone = 1; val(i1 == 0 ? m - 1 : i1 - 1) < 0; ++gone) i1 = i1 == 0 ? m - 1 : i1 - 1;
+            while (val((i1 + gone) % m) < 0) ++gone;
         }
-        ax = bx;
-        ay = by;
-        at = bt;
-        va = vb;
+        // i0 the vertex before the run, [i1, i2] the run, i3 the one after
+        const int i0 = i1 == 0 ? m - 1 : i1 - 1, i2 = i1 + gone - 1 < m ? i1 + gone - 1 : i1 + gone - 1 - m;
+        const int i3 = i2 + 1 == m ? 0 : i2 + 1;
+        const double v0 = val(i0), v1 = val(i1), v2 = val(i2), v3 = val(i3);
+        if (gone == 1 && !first && m >= room) return m;
+        auto on_line = [&](int k, double vk, int l, double vl, double &x, double &y) {
+            const double px = q.X(k), py = q.Y(k), t = vk / (vk - vl);
+            x = axis == 0 ? c : px + t * (q.X(l) - px);
+            y = axis == 0 ? py + t * (q.Y(l) - py) : c;
+        };
+        double ax, ay, bx, by;
+        on_line(i0, v0, i1, v1, ax, ay);
+        on_line(i2, v2, i3, v3, bx, by);
+        const int bt = q.I(i2);
+        int ia, ib;  // their places
+        if (i1 == 0 || i1 > i2) {  // vertex 0 goes: B, the kept run from i3 on, A
+            ib = 0;
+            ia = m - gone + 1;
+            if (i3 > 1)
+                for (int k = 1; k < ia; ++k) q.copy(k, i3 + k - 1);
+        } else {
+            ia = i1;
+            ib = i1 + 1;
+            if (gone == 1) {
+                for (int k = m; k > ib; --k) q.copy(k, k - 1);
+            } else if (gone > 2) {
+                for (int k = i2 + 1; k < m; ++k) q.copy(k + 2 - gone, k);
+            }
+        }
+        q.X(ia) = ax;
+        q.Y(ia) = ay;
+        q.I(ia) = own;
+        q.X(ib) = bx;
+        q.Y(ib) = by;
+        q.I(ib) = bt;
+        m += 2 - gone;
+        if (gone == out) return m;
     }
-    return w;
 }
 
+#ifdef __CUDACC__
 // Disc clipping restated from ConvexPolyhedron2::ball_cut
 // (ConvexPolyhedron2.tcc:534-666): the edge a -> b of a polygon emits 0, 1 or 2
 // vertices of the clipped one (x, y, and whether an arc leaves it; else its
