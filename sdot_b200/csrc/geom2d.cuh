@@ -498,12 +498,16 @@ __device__ __forceinline__ int disc_edge(double ax, double ay, double bx, double
 // disc (c, r), arcs tagged ID_ARC; with CLOSE the first one once more at the end
 // (closing).  One loop and one call of push, so that it is inlined once.
 // Returns the radius of the result as the reference stores it: r, 0 if void;
-// -1 without a disc.  A polygon that leaves no vertex stands for the full disc,
-// unless the centre lies outside one of its edges' half-planes.
+// -1 without a disc.  A polygon that leaves no vertex is apart from the circle: it
+// stands for the full disc where the centre lies inside it, which is where a ray
+// from the centre to greater x crosses an odd number of edges.  (Its side of
+// every edge says the same, but not of an edge between vertices at one place,
+// whose direction is rounding; such an edge lies far from the centre, and on one
+// side of it whatever its direction.)
 template <bool BALL, bool CLOSE, class P, class Tag, class S>
 __device__ __forceinline__ double stream_piece(const P &q, int m, const Tag &tag, double cx, double cy, double r, S &sink) {
     int nout = 0, ft = 0;
-    bool center_out = false;
+    bool inside = false;
     double fx = 0, fy = 0;
     double ax = m > 0 ? q.X(0) : 0, ay = m > 0 ? q.Y(0) : 0;
     const double qx = ax, qy = ay;
@@ -521,8 +525,8 @@ __device__ __forceinline__ double stream_piece(const P &q, int m, const Tag &tag
             const double bx = k + 1 < m ? q.X(k + 1) : qx, by = k + 1 < m ? q.Y(k + 1) : qy;
             t = tag(k);
             if (BALL) {
-                // outward normal of a counter-clockwise edge is (dy, -dx)
-                if ((cx - ax) * (by - ay) - (cy - ay) * (bx - ax) > 0) center_out = true;
+                if ((ay > cy) != (by > cy))
+                    inside ^= ((bx - ax) * (cy - ay) - (cx - ax) * (by - ay) > 0) == (by > ay);
                 cnt = disc_edge(ax, ay, bx, by, cx, cy, r, e);
             } else {
                 e.x[0] = ax;
@@ -547,7 +551,7 @@ __device__ __forceinline__ double stream_piece(const P &q, int m, const Tag &tag
         }
     }
     if (!BALL) return -1.0;
-    return m == 0 || (nout == 0 && center_out) ? 0.0 : r;
+    return m == 0 || (nout == 0 && !inside) ? 0.0 : r;
 }
 
 // The segment of the disc (c, r) between the chord p0 -> p1 and the arc (area,
