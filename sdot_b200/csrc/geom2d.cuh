@@ -558,6 +558,11 @@ __device__ __forceinline__ double stream_piece(const P &q, int m, const Tag &tag
 // moments about the origin, angle of the arc), restated from
 // ConvexPolyhedron2::_arc_area / _centroid_arc / _arc_length
 // (ConvexPolyhedron2.tcc:2296-2381), which each take the angles anew.
+// Ends that meet to rounding may come in the wrong order (the sides of a sliver,
+// an ulp apart, cut by the circle), and the arc would be all but a full turn: it
+// is none if the rest is less than 1000 ulp of the coordinates, as seen from the
+// centre.  (A chord that leaves an arc of all but a full turn spans 1e-8 at
+// least, where its line touches the circle to rounding.)
 struct Arc {
     double area, mx, my, angle;
 };
@@ -567,6 +572,7 @@ __device__ __forceinline__ Arc arc_segment(double p0x, double p0y, double p1x, d
     const double a0 = atan2(p0y, p0x);
     double a1 = atan2(p1y, p1x);
     if (a1 < a0) a1 += 2 * kPi;
+    if ((2 * kPi - (a1 - a0)) * r < 0x1p-42 * (fabs(cx) + fabs(cy) + r)) a1 = a0;
     const double ex = p0x - p1x, ey = p0y - p1y;
     const double d0 = sqrt(ex * ex + ey * ey) / 2;
     const double d1 = sqrt(fmax(0.0, r * r - d0 * d0));

@@ -1,5 +1,7 @@
 """Discs in the cells of regular lattices, whose corners are several vertices at
-one place: a disc inside its cell is whole, one around it leaves the cell.
+one place: a disc inside its cell is whole, one around it leaves the cell, and one
+that reaches past the sides leaves no arc of a full turn in the slivers that a
+pixel's line may cut off there.
 
 Areas of a disc and of a square; TOL as in test_gpu_lattice_pixels.py (a disc's
 own area, pi r^2, is exact to a few ulp)."""
@@ -26,7 +28,7 @@ def diagram(m, lo, hi, rho):
     return PowerDiagram(p, np.full(m * m, (rho * h) ** 2), radial_func="in_ball_w05"), h
 
 
-@pytest.mark.parametrize("rho", [0.4, 2.0])
+@pytest.mark.parametrize("rho", [0.4, 0.55, 0.6, 0.7, 2.0])
 @pytest.mark.parametrize("m,res", SIZES)
 def test_discs_over_pixels(gpu_lib, m, res, rho):
     d, h = diagram(m, 0.1, 0.8, rho)
@@ -34,7 +36,7 @@ def test_discs_over_pixels(gpu_lib, m, res, rho):
     assert np.abs(d.integrals() - share(rho) * h * h).max() <= TOL * h * h
 
 
-@pytest.mark.parametrize("rho", [0.4, 2.0])
+@pytest.mark.parametrize("rho", [0.4, 0.6, 2.0])
 @pytest.mark.parametrize("lo,hi", BOXES)
 @pytest.mark.parametrize("m", [10, 49, 64, 97, 130, 200])
 def test_discs_in_a_box(gpu_lib, m, lo, hi, rho):
