@@ -426,12 +426,22 @@ struct Ring {
     __device__ double X(int k) const { return c0x + ux(k); }
     __device__ double Y(int k) const { return c0y + uy(k); }
 
+    // The mask of a cut's farthest run, where rounding gives more than one.
+    __device__ __noinline__ unsigned one_run(int n, double nx, double ny, double b) const {
+        int i1, gone;
+        farthest_run(n, [&](int k) { return b - (ux(k) * nx + uy(k) * ny); }, i1, gone);
+        const unsigned run = (1u << gone) - 1u;
+        return (run << i1 | run >> (n - i1)) & ((1u << n) - 1u);
+    }
+
     // Cuts the polygon (n vertices) by nx ux + ny uy <= b; bit k of mask:
     // vertex k is outside.  Same new vertices at the same places as
     // plane_cut_apply: with i1 the first and i2 the last vertex removed, A on
     // the edge into i1 takes the cut's id, B on the edge out of i2 keeps that
     // edge's.  Returns the new count, or -1 past CAP.
     __device__ int cut(int n, unsigned mask, double nx, double ny, double b, int cut_id) {
+        const unsigned starts = mask & ~(mask << 1 | mask >> (n - 1));
+        if (starts & (starts - 1)) mask = one_run(n, nx, ny, b);
         const CutFacts f = cut_facts(mask, n);
         if (f.nb_out == n) return 0;
         const int nb_in = n - f.nb_out;

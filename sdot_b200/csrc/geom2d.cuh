@@ -91,6 +91,30 @@ SDOT_HD CutFacts cut_facts(unsigned mask, int n) {
     return f;
 }
 
+// The run [i1, i1 + gone) (cyclic) of vertices with d(k) < 0 that holds the
+// lowest, for a polygon with some such vertices and some others.  A convex
+// polygon has one run but for rounding: where several vertices lie at one place
+// (the corners of a lattice's cells), others may be outside by an ulp here and
+// there, and the run of the farthest is the one that a cut removes.
+template <class D>
+SDOT_HDI void farthest_run(int n, const D &d, int &i1, int &gone) {
+    double low = 0;
+    i1 = 0;
+    for (int k = 0; k < n; ++k) {
+        const double v = d(k);
+        if (v < low) {
+            low = v;
+            i1 = k;
+        }
+    }
+    gone = 1;
+    while (gone < n && d(i1 == 0 ? n - 1 : i1 - 1) < 0) {
+        i1 = i1 == 0 ? n - 1 : i1 - 1;
+        ++gone;
+    }
+    while (gone < n && d((i1 + gone) % n) < 0) ++gone;
+}
+
 template <class T>
 SDOT_HD int plane_cut_apply(const PolyView<T> &p, int n, int cap, T ox, T oy, T nx, T ny, int cut_id,
                             const CutFacts &f);
@@ -191,18 +215,17 @@ __device__ int plane_cut_warp(const PolyView<T> &p, int n, int cap, T ox, T oy, 
                               bool normalize) {
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    int nb_out = 0, first_out = -1, first_in = -1;
+    int nb_out = 0, first_out = -1, first_in = -1, runs = 0;
     bool out1 = false, out_last = false;
+    auto side = [&](int k) -> T { return (ox - p.X(k)) * nx + (oy - p.Y(k)) * ny; };
     for (int base = 0; base < n; base += 32) {
         const int k = base + lane;
         const bool valid = k < n;
-        bool o = false;
-        if (valid) {
-            const T d = (ox - p.X(k)) * nx + (oy - p.Y(k)) * ny;
-            o = d < T(0);
-        }
+        const bool o = valid && side(k) < T(0);
         const unsigned mo = __ballot_sync(FULL, o), mi = __ballot_sync(FULL, valid && !o);
         nb_out += __popc(mo);
+        runs += __popc(mo & ~(mo << 1 | unsigned(out_last)));  // out_last: of the vertices before
+        out_last = mo >> 31;
         if (first_out < 0 && mo) first_out = base + __ffs(mo) - 1;
         if (first_in < 0 && mi) first_in = base + __ffs(mi) - 1;
         if (base == 0 && n > 1) out1 = (mo >> 1) & 1u;
@@ -210,6 +233,17 @@ __device__ int plane_cut_warp(const PolyView<T> &p, int n, int cap, T ox, T oy, 
     }
     if (nb_out == 0) return n;
     if (nb_out == n) return 0;
+    if (runs - (out_last && first_out == 0) > 1) {
+        // (every lane alike; rare)
+        int a, g;
+        farthest_run(n, side, a, g);
+        nb_out = g;
+        const bool wrap = a + g > n;
+        first_out = wrap ? 0 : a;
+        first_in = wrap ? a + g - n : a == 0 ? g : 0;
+        out1 = wrap ? a + g - n > 1 || a == 1 : a <= 1 && a + g > 1;
+        out_last = a + g >= n;
+    }
     T inv = T(1);
     if (normalize) inv = T(1) / sqrt(nx * nx + ny * ny);
     auto dist = [&](int k) -> T { return ((ox - p.X(k)) * nx + (oy - p.Y(k)) * ny) * inv; };
@@ -385,20 +419,11 @@ SDOT_HD int axis_cut(const P &q, int m, int axis, double c, double s, int own, i
             }
         }
         if (!gone) {
-            double low = 0;
             out = 0;
-            for (int k = 0; k < m; ++k) {
-                const double v = val(k);
-                out += v < 0;
-                if (v < low) {
-                    low = v;
-                    i1 = k;
-                }
-            }
+            for (int k = 0; k < m; ++k) out += val(k) < 0;
             if (!out) return m;
             if (out == m) return 0;
-            for (gone = 1; val(i1 == 0 ? m - 1 : i1 - 1) < 0; ++gone) i1 = i1 == 0 ? m - 1 : i1 - 1;
-            while (val((i1 + gone) % m) < 0) ++gone;
+            farthest_run(m, val, i1, gone);
         }
         // i0 the vertex before the run, [i1, i2] the run, i3 the one after
         const int i0 = i1 == 0 ? m - 1 : i1 - 1, i2 = i1 + gone - 1 < m ? i1 + gone - 1 : i1 + gone - 1 - m;
