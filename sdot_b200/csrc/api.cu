@@ -300,8 +300,8 @@ struct sdot_ctx {
     long long nnz = 0, nb_total = 0;
     long long n_void = 0;
     int last_ovf = 0;
-    unsigned last_err = 0;
-    int last_guard[3] = {0, 0, 0};
+    unsigned last_err = 0, nb_err = 0;             // of the last evaluation or raster, of the neighbour lists
+    int last_guard[3] = {0, 0, 0}, nb_guard[3] = {0, 0, 0};
     cudaEvent_t ev[4] = {};
     float times[3] = {0, 0, 0};
 
@@ -740,40 +740,44 @@ struct sdot_ctx {
         if (r.side_val) dalloc(r.side_val, r.side_cap);
     }
 
-    int finish_status() {
-        if (last_err & DE_ITER) {
+    int finish_status() { return status_of(last_err, last_guard); }
+
+    // The status (and message) of a pass with these error bits and this guard.
+    int status_of(unsigned e, const int *g) {
+        if (e & DE_ITER) {
             last_error = "a tree traversal visited more nodes than the tree holds (inconsistent tree)";
             return SDOT_ITER_CAP;
         }
-        if (last_err & DE_CAPACITY) {
+        if (e & DE_CAPACITY) {
             last_error = dim == 3 ? "a cell exceeded the maximum polyhedron capacity (256 faces of 128 vertices)"
                                   : "a cell exceeded the maximum polygon capacity (1024 vertices)";
             return SDOT_CAPACITY;
         }
-        if (last_err & DE_SIDE) {
+        if (e & DE_SIDE) {
             last_error = "long Hessian rows or neighbour lists exceeded the side buffer after it was grown";
             return SDOT_CAPACITY;
         }
-        if (last_err & DE_DEGEN) {
+        if (e & DE_DEGEN) {
             last_error = "a 3D cut met degenerate geometry (the affected cells are NaN)";
             return SDOT_CAPACITY;
         }
-        if (last_err & DE_GUARD) {
-            last_error = "inconsistent input or tree (guard " + std::to_string(last_guard[0]) + " at cell " +
-                         std::to_string(last_guard[1]) + ", value " + std::to_string(last_guard[2]) + ")";
+        if (e & DE_GUARD) {
+            last_error = "inconsistent input or tree (guard " + std::to_string(g[0]) + " at cell " +
+                         std::to_string(g[1]) + ", value " + std::to_string(g[2]) + ")";
             return SDOT_BAD_ARG;
         }
-        if (last_err & DE_STACK) {
+        if (e & DE_STACK) {
             last_error = "traversal stack overflow";
             return SDOT_CAPACITY;
         }
         return SDOT_OK;
     }
 
-    void evaluate_neighbors() {
-        if (!nb_dirty) return;
+    // The neighbour lists, and the status of the walk that made them.
+    int evaluate_neighbors() {
+        if (!nb_dirty) return status_of(nb_err, nb_guard);
         // the walk alone: the lists need no integrals (an evaluation, when one
-        // is asked for too, is a pass of its own)
+        // is asked for too, is a pass of its own, with a status of its own)
         check_domain();
         reserve_eval();
         SDOT_CUDA(cudaMemsetAsync(dstat, 0, sizeof(DevStatus), stream));
@@ -803,10 +807,11 @@ struct sdot_ctx {
                 a.nb = nb;
                 cells2d_launch(a, scratch, stream);
             }
-            unsigned e = 0;
-            SDOT_CUDA(cudaMemcpyAsync(&e, err, sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
+            SDOT_CUDA(cudaMemcpyAsync(hstat, dstat, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
             SDOT_CUDA(cudaStreamSynchronize(stream));
-            if (!(e & DE_SIDE) || attempt >= 4) break;
+            nb_err = hstat->err;
+            for (int k = 0; k < 3; ++k) nb_guard[k] = hstat->guard[k];
+            if (!(nb_err & DE_SIDE) || attempt >= 4) break;
             grow_side(nb);  // long id lists outgrew the side buffer
         }
         nb_counts(nb, n, perm(), cnt_orig, stream);
@@ -814,6 +819,7 @@ struct sdot_ctx {
         SDOT_CUDA(cudaMemcpyAsync(&nb_total, nb_offsets + n, sizeof(long long), cudaMemcpyDeviceToHost, stream));
         SDOT_CUDA(cudaStreamSynchronize(stream));
         nb_dirty = false;
+        return status_of(nb_err, nb_guard);
     }
 
     // get_image_integrals / get_image_of_cell_nums (get_image_integrals.h:16-78,
@@ -1619,10 +1625,11 @@ int sdot_get_der_integrals_wrt_weights(sdot_ctx *ctx, int64_t *offsets, int64_t 
 int sdot_get_neighbors(sdot_ctx *ctx, int64_t *offsets, int64_t *ids, int64_t *count_inout, int mem_space) {
     return guarded(ctx, [&] {
         if (!count_inout) throw BadArg("null count");
-        ctx->evaluate_neighbors();
+        // a walk that failed leaves empty lists and its status
+        const int st = ctx->evaluate_neighbors();
         if (!ids) {
             *count_inout = ctx->nb_total;
-            return int(SDOT_OK);
+            return st;
         }
         if (*count_inout < ctx->nb_total) throw BadArg("ids buffer smaller than count");
         if (!offsets) throw BadArg("null offsets");
@@ -1638,7 +1645,7 @@ int sdot_get_neighbors(sdot_ctx *ctx, int64_t *offsets, int64_t *ids, int64_t *c
         ctx->copy_out(offsets, ctx->nb_offsets, size_t(n + 1) * sizeof(long long), mem_space);
         SDOT_CUDA(cudaStreamSynchronize(ctx->stream));
         *count_inout = tot;
-        return int(SDOT_OK);
+        return st;
     });
 }
 
@@ -1675,7 +1682,7 @@ int sdot_get_der_centroids_and_integrals_wrt_weight_and_positions(sdot_ctx *ctx,
         if (ctx->ball) throw Unsupported("position derivatives with the disc clip are not available in this build");
         if (ctx->mode != DM_SINGLE && ctx->mode != DM_PERIODIC)
             throw Unsupported("position derivatives are available for one-shape domains");
-        ctx->evaluate_neighbors();
+        const int st = ctx->evaluate_neighbors();
         const long long n = ctx->n;
         // block counts per Dirac, their scan, then the rows
         ctx->reserve_stage(std::max<long long>(n + 1, 1));
@@ -1696,7 +1703,7 @@ int sdot_get_der_centroids_and_integrals_wrt_weight_and_positions(sdot_ctx *ctx,
         const long long nnz = 9 * total;
         if (!columns) {
             *nnz_inout = nnz;
-            return ctx->finish_status();
+            return st;
         }
         if (*nnz_inout < nnz) throw BadArg("columns/values buffers smaller than nnz");
         if (!offsets || !values || !v_values) throw BadArg("null output");
@@ -1720,7 +1727,7 @@ int sdot_get_der_centroids_and_integrals_wrt_weight_and_positions(sdot_ctx *ctx,
         }
         SDOT_CUDA(cudaStreamSynchronize(ctx->stream));
         *nnz_inout = nnz;
-        return ctx->finish_status();
+        return st;
     });
 }
 
