@@ -705,7 +705,7 @@ struct sdot_ctx {
         // outputs in caller order; nnz and the empty cells to the status block,
         // which comes back (with error bits, overflow count, guard) in one copy
         unpermute(s_mass, o_mass, s_mass_c, o_mass_c, s_ctd, o_ctd, n, dim, perm(), offsets, &dstat->nnz, &dstat->n_void,
-                  stream);
+                  dim == 3 ? tree3.sync : tree2.sync, err, stream);
         SDOT_CUDA(cudaEventRecord(ev[3], stream));
         SDOT_CUDA(cudaMemcpyAsync(hstat, dstat, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
         SDOT_CUDA(cudaStreamSynchronize(stream));
@@ -727,7 +727,7 @@ struct sdot_ctx {
             side_retries = 0;
             return st;
         }
-        eval_dirty = false;
+        eval_dirty = tree_lost(last_err);
         return finish_status();
     }
 
@@ -740,10 +740,26 @@ struct sdot_ctx {
         if (r.side_val) dalloc(r.side_val, r.side_cap);
     }
 
+    // A wait of the tree's kernels was given up: the next call builds it again.
+    bool tree_lost(unsigned e) {
+        if (e & DE_TREE) pos_dirty = true;
+        return e & DE_TREE;
+    }
+    void tree_status() {
+        if (dim == 3)
+            tree3.status(err, stream);
+        else
+            tree2.status(err, stream);
+    }
+
     int finish_status() { return status_of(last_err, last_guard); }
 
     // The status (and message) of a pass with these error bits and this guard.
     int status_of(unsigned e, const int *g) {
+        if (e & DE_TREE) {
+            last_error = "a wait in the kernels of the tree was given up";
+            return SDOT_ITER_CAP;
+        }
         if (e & DE_ITER) {
             last_error = "a tree traversal visited more nodes than the tree holds (inconsistent tree)";
             return SDOT_ITER_CAP;
@@ -807,6 +823,7 @@ struct sdot_ctx {
                 a.nb = nb;
                 cells2d_launch(a, scratch, stream);
             }
+            tree_status();
             SDOT_CUDA(cudaMemcpyAsync(hstat, dstat, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
             SDOT_CUDA(cudaStreamSynchronize(stream));
             nb_err = hstat->err;
@@ -818,7 +835,7 @@ struct sdot_ctx {
         scan_exclusive_total<long long>(cnt_orig, nb_offsets, n, scan_tmp, stream);
         SDOT_CUDA(cudaMemcpyAsync(&nb_total, nb_offsets + n, sizeof(long long), cudaMemcpyDeviceToHost, stream));
         SDOT_CUDA(cudaStreamSynchronize(stream));
-        nb_dirty = false;
+        nb_dirty = tree_lost(nb_err);
         return status_of(nb_err, nb_guard);
     }
 
@@ -876,10 +893,12 @@ struct sdot_ctx {
             a.mode = DM_RASTER;
             cells2d_launch(a, scratch, stream);
         }
+        tree_status();
         SDOT_CUDA(cudaMemcpyAsync(hstat, dstat, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream));
         SDOT_CUDA(cudaStreamSynchronize(stream));
         last_err = hstat->err;
         for (int k = 0; k < 3; ++k) last_guard[k] = hstat->guard[k];
+        tree_lost(last_err);
     }
 
     void copy_out(void *dst, const void *src, size_t bytes, int mem_space) {

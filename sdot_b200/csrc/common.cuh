@@ -135,6 +135,10 @@ __host__ __device__ inline void flag_error(unsigned *word, unsigned bits) {
 }
 
 #ifdef __CUDACC__
+// Turns of a wait before it is given up (seconds).
+#ifndef SDOT_BARRIER_SPINS
+#define SDOT_BARRIER_SPINS (1u << 24)
+#endif
 // (Cooperative launches: every block is resident.  sync: two words, zeroed
 // before the launch: the arrivals, and a mark that a wait was given up.)
 // Waits for every block of the grid; false when the wait was given up (by any
@@ -148,7 +152,7 @@ __device__ inline bool grid_barrier(unsigned *sync, unsigned &target) {
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sync[0]) : "memory");
         ok = 0;
-        for (unsigned k = 0; k < (1u << 24); ++k) {
+        for (unsigned k = 0; k < SDOT_BARRIER_SPINS; ++k) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&sync[0]) : "memory");
             if (int(v - target) >= 0) {
@@ -180,6 +184,7 @@ enum DevErr : unsigned {
     DE_GUARD = 16u,        // an input failed a consistency guard (see the debug triple)
     DE_DEGEN = 32u,        // a 3D cut met degenerate geometry (a face cut twice, an open new face)
     DE_SIDE = 64u,         // a long row did not fit the side buffer (the host grows it and runs again)
+    DE_TREE = 128u,        // a wait in the kernels of the tree or of its sort was given up
 };
 
 }  // namespace sdot

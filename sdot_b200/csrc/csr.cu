@@ -304,10 +304,10 @@ __global__ void k_nb_write(Rows NB, long long n, const int *idx, const long long
 }
 
 // Masses and centroids to caller order, the number of empty cells added to
-// *n_void, and the last CSR offset to *nnz.
+// *n_void, the last CSR offset to *nnz, and the tree's status to *err.
 __global__ void k_unpermute(const double *m, double *om, const double *mc, double *omc, const double *c, double *oc,
                             long long n, int d, const int *idx, const long long *offsets, long long *nnz,
-                            unsigned long long *n_void) {
+                            unsigned long long *n_void, const unsigned *tree_sync, unsigned *err) {
     const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const bool in = s < n;
     const double ms = in ? m[s] : 1.0;
@@ -319,7 +319,10 @@ __global__ void k_unpermute(const double *m, double *om, const double *mc, doubl
     }
     const int z = __syncthreads_count(ms == 0.0);  // one atomic per block
     if (threadIdx.x == 0 && z) atomicAdd(n_void, (unsigned long long)z);
-    if (s == 0) *nnz = offsets[n];
+    if (s == 0) {
+        *nnz = offsets[n];
+        if (tree_sync[1] | tree_sync[3]) atomicOr(err, unsigned(DE_TREE));
+    }
 }
 
 // ---- domains of several shapes: one cell pass per shape, summed here
@@ -420,9 +423,10 @@ void nb_write(const Rows &NB, long long n, const int *idx, const long long *offs
     SDOT_CUDA(cudaGetLastError());
 }
 void unpermute(const double *m, double *om, const double *mc, double *omc, const double *c, double *oc, long long n, int d,
-               const int *idx, const long long *offsets, long long *nnz, unsigned long long *n_void, cudaStream_t st) {
+               const int *idx, const long long *offsets, long long *nnz, unsigned long long *n_void,
+               const unsigned *tree_sync, unsigned *err, cudaStream_t st) {
     if (n <= 0) return;
-    k_unpermute<<<ceil_div(n, TB), TB, 0, st>>>(m, om, mc, omc, c, oc, n, d, idx, offsets, nnz, n_void);
+    k_unpermute<<<ceil_div(n, TB), TB, 0, st>>>(m, om, mc, omc, c, oc, n, d, idx, offsets, nnz, n_void, tree_sync, err);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
 }

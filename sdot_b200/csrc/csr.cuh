@@ -29,8 +29,10 @@ void accum_pass(double *mass, double *mass_c, double *mom, const double *t_mass,
                 const double *t_ctd, long long n, int dim, cudaStream_t st);
 void centroids_final(double *ctd, const double *mom, const double *mass_c, long long n, int dim, cudaStream_t st);
 // Masses (m and mc) and centroids (c, d coordinates) to caller order; *n_void +=
-// the number of zeros in m (the empty cells); *nnz = offsets[n].
+// the number of zeros in m (the empty cells); *nnz = offsets[n]; and the status
+// of the tree (DeviceTree::status, with its sync words) to *err.
 void unpermute(const double *m, double *om, const double *mc, double *omc, const double *c, double *oc, long long n, int d,
-               const int *idx, const long long *offsets, long long *nnz, unsigned long long *n_void, cudaStream_t st);
+               const int *idx, const long long *offsets, long long *nnz, unsigned long long *n_void,
+               const unsigned *tree_sync, unsigned *err, cudaStream_t st);
 
 }  // namespace sdot

@@ -84,12 +84,14 @@ __global__ void k_morton(const double *pos, long long n, const unsigned long lon
     vals[i] = unsigned(i);
 }
 
+// (A sort that was given up has left no order: any permutation keeps the indexes
+// in range, and the level kernel marks the tree.)
 template <int D>
-__global__ void k_gather(const double *pos, const double *w, const unsigned *order, long long n, double *pos_s,
-                         double *w_s, int *idx, int *inv) {
+__global__ void k_gather(const double *pos, const double *w, const unsigned *order, const unsigned *lost, long long n,
+                         double *pos_s, double *w_s, int *idx, int *inv) {
     long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (s >= n) return;
-    unsigned i = order[s];
+    const unsigned i = *lost ? unsigned(s) : order[s];
     for (int d = 0; d < D; ++d) pos_s[D * s + d] = pos[D * (long long)i + d];
     w_s[s] = w[i];
     idx[s] = int(i);
@@ -145,6 +147,21 @@ __device__ __forceinline__ void warp_bounds(const unsigned *keys, int a, int b, 
     for (int c = 1; c < C; ++c) st[c] = lo[c];
 }
 
+// A tree that cannot be used: every walk that starts with a vertex opens the
+// root, and its guard ends it there.
+template <int D>
+__device__ void lose_tree(TreeNode<D> *nodes) {
+    nodes[0].a = -1;
+    nodes[0].b = 1;
+    for (int d = 0; d < D; ++d) nodes[0].lo[d] = nodes[0].hi[d] = 0;
+    nodes[0].maxw = 1.0 / 0.0;
+}
+
+// err |= DE_TREE where a wait of the tree's kernels was given up.
+__global__ void k_tree_status(const unsigned *sync, unsigned *err) {
+    if (sync[1] | sync[3]) atomicOr(err, unsigned(DE_TREE));
+}
+
 template <int D>
 struct TreeArgs {
     TreeNode<D> *nodes;
@@ -179,6 +196,10 @@ __global__ void __launch_bounds__(TREE_TB, 1) k_tree(const TreeArgs<D> A) {
     int *const start = A.counters + 1, *const added = A.counters + A.npass + 4;
     unsigned target = 0;
     int depth = 0;  // levels in use
+    if (BUILD && A.sync[3]) {  // the sort's wait was given up: its keys are in no order
+        if (thread == 0) lose_tree(A.nodes);
+        return;
+    }
     if (BUILD) {
         // nodes [beg, end) are the level's; added[p]: how many it gives the next
         int beg = 0, end = 1;
@@ -217,8 +238,7 @@ __global__ void __launch_bounds__(TREE_TB, 1) k_tree(const TreeArgs<D> A) {
                 }
             }
             if (!grid_barrier(A.sync, target)) {
-                A.nodes[0].a = -1;  // the walks' guard reports it
-                A.nodes[0].b = 1;
+                lose_tree(A.nodes);
                 return;
             }
             depth = p + 1;
@@ -232,8 +252,7 @@ __global__ void __launch_bounds__(TREE_TB, 1) k_tree(const TreeArgs<D> A) {
         while (depth < A.npass && start[depth] < start[depth + 1]) ++depth;
         for (long long s = thread; s < A.n; s += nthreads) A.w[s] = A.w_orig[A.idx[s]];
         if (!grid_barrier(A.sync, target)) {
-            A.nodes[0].a = -1;
-            A.nodes[0].b = 1;
+            lose_tree(A.nodes);
             return;
         }
     }
@@ -279,8 +298,7 @@ __global__ void __launch_bounds__(TREE_TB, 1) k_tree(const TreeArgs<D> A) {
     }
     for (int p = depth - 2; p >= 0; --p) {  // the last level holds leaves only
         if (!grid_barrier(A.sync, target)) {
-            A.nodes[0].a = -1;
-            A.nodes[0].b = 1;
+            lose_tree(A.nodes);
             return;
         }
         int end;
@@ -485,7 +503,7 @@ void DeviceTree<D>::build_launches(const double *pos_orig, const double *w_orig,
     note_launch();
     SDOT_CUDA(cudaGetLastError());
     radix_sort_pairs(keys, vals, keys2, vals2, keys3, vals3, n, D * key_bits, tmp, sync + 2, st);
-    k_gather<D><<<ceil_div(n, TB), TB, 0, st>>>(pos_orig, w_orig, vals2, n, pos, w, idx, inv);
+    k_gather<D><<<ceil_div(n, TB), TB, 0, st>>>(pos_orig, w_orig, vals2, sync + 3, n, pos, w, idx, inv);
     note_launch();
     SDOT_CUDA(cudaGetLastError());
     tree_launch<D, true>(TreeArgs<D>{nodes, node_level, counters, keys2, pos, w, nullptr, idx, n, key_bits, max_per_leaf,
@@ -517,6 +535,14 @@ void DeviceTree<D>::weights_launches(const double *w_orig, cudaStream_t st) {
     tree_launch<D, false>(TreeArgs<D>{nodes, node_level, counters, keys2, pos, w, w_orig, idx, n, key_bits, max_per_leaf,
                                       max_nodes, npass, sync},
                           st);
+}
+
+template <int D>
+void DeviceTree<D>::status(unsigned *err, cudaStream_t st) const {
+    if (n == 0) return;
+    k_tree_status<<<1, 1, 0, st>>>(sync, err);
+    note_launch();
+    SDOT_CUDA(cudaGetLastError());
 }
 
 template struct DeviceTree<2>;

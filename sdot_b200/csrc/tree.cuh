@@ -42,7 +42,9 @@ struct DeviceTree {
     // [0] node count, [1 + p] first node of level p (npass + 1 of them),
     // [npass + 4 + p] nodes that level p gave the next (builds)
     int *counters = nullptr;
-    unsigned *sync = nullptr;  // grid barriers: of the level kernel, of the sort
+    // grid barriers (two words each: arrivals, given up): of the level kernel, of
+    // the sort
+    unsigned *sync = nullptr;
     int npass = 0;
     // scratch
     unsigned *keys = nullptr, *keys2 = nullptr, *keys3 = nullptr;
@@ -69,6 +71,9 @@ struct DeviceTree {
     void build(const double *pos_orig, const double *w_orig, long long n, cudaStream_t st);
     // new weights (original order, device pointer): re-gather and refresh maxw
     void update_weights(const double *w_orig, cudaStream_t st);
+    // flags DE_TREE in *err if a wait of the last build or refresh was given up
+    // (the tree is then to be built again)
+    void status(unsigned *err, cudaStream_t st) const;
 };
 
 extern template struct DeviceTree<2>;
