@@ -259,8 +259,7 @@ struct sdot_ctx {
     int mode = DM_SINGLE;
     int start_n = 0;
     double coeff = 1;
-    double *d_start = nullptr, *d_img = nullptr, *d_item_xy = nullptr, *d_item_nrm = nullptr, *d_item_coeff = nullptr;
-    int *d_item_off = nullptr;
+    double *d_start = nullptr, *d_img = nullptr, *d_item_xy = nullptr;
 
     // evaluation buffers
     long long ecap = 0;
@@ -285,7 +284,6 @@ struct sdot_ctx {
     bool hint_valid = false;
     unsigned *err = nullptr;   // &dstat->err
     int *guard = nullptr;      // dstat->guard
-    long long item_nv = 0;
     // device staging of the CSR columns / values and neighbour ids that go to
     // host buffers (int64 + double per entry), grown with nnz
     long long *stage_i = nullptr;
@@ -310,7 +308,7 @@ struct sdot_ctx {
         tree2.release();
         tree3.release();
         dfree(d_pos); dfree(d_w);
-        dfree(d_start); dfree(d_img); dfree(d_item_xy); dfree(d_item_nrm); dfree(d_item_coeff); dfree(d_item_off);
+        dfree(d_start); dfree(d_img); dfree(d_item_xy);
         dfree(d_trans);
         dfree(d_planes3);
         free_eval();
@@ -382,7 +380,7 @@ struct sdot_ctx {
         guard = dstat->guard;
         if (!hstat) SDOT_CUDA(cudaMallocHost(reinterpret_cast<void **>(&hstat), sizeof(DevStatus)));
         dalloc(ovf_list2, ecap);
-        dalloc(ovf_cnt2, 3);  // the count, and the cursors of the 3D passes over the lists
+        dalloc(ovf_cnt2, 3);  // the count, and the cursors of the larger tiers over the lists
         if (dim == 3) {
             dalloc(hint3, ecap);
             hint_valid = false;
@@ -416,36 +414,27 @@ struct sdot_ctx {
             double mn[2] = {std::numeric_limits<double>::max(), std::numeric_limits<double>::max()};
             double mx[2] = {-std::numeric_limits<double>::max(), -std::numeric_limits<double>::max()};
             std::vector<int> off = {0};
-            std::vector<double> xy, nrm, co;
+            std::vector<double> xy;
             for (const Item2 &it : items) {
                 for (size_t k = 0; k < it.xy.size(); ++k) {
                     mn[k % 2] = std::min(mn[k % 2], it.xy[k]);
                     mx[k % 2] = std::max(mx[k % 2], it.xy[k]);
                 }
                 xy.insert(xy.end(), it.xy.begin(), it.xy.end());
-                nrm.insert(nrm.end(), it.nrm.begin(), it.nrm.end());
                 off.push_back(int(xy.size() / 2));
-                co.push_back(it.coeff);
             }
             double dx = mx[0] - mn[0], dy = mx[1] - mn[1];
             Item2 eb = box_item(mn[0] - dx, mn[1] - dy, mx[0] + dx, mx[1] + dy, 1.0);
             start_n = 4;
             dalloc(d_start, 8);
             SDOT_CUDA(cudaMemcpyAsync(d_start, eb.xy.data(), 8 * sizeof(double), cudaMemcpyHostToDevice, stream));
-            item_nv = off.back();
             item_off_h = off;
             for (size_t k = 0; k + 1 < off.size(); ++k)
                 if (off[k + 1] - off[k] > kMaxDomainVertices)
                     throw Unsupported("a domain shape has more than " + std::to_string(kMaxDomainVertices) +
                                       " vertices");
-            dalloc(d_item_off, off.size());
-            SDOT_CUDA(cudaMemcpyAsync(d_item_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
             dalloc(d_item_xy, xy.size());
             SDOT_CUDA(cudaMemcpyAsync(d_item_xy, xy.data(), xy.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
-            dalloc(d_item_nrm, nrm.size());
-            SDOT_CUDA(cudaMemcpyAsync(d_item_nrm, nrm.data(), nrm.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
-            dalloc(d_item_coeff, co.size());
-            SDOT_CUDA(cudaMemcpyAsync(d_item_coeff, co.data(), co.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
         } else {
             throw BadArg("no domain: call sdot_add_box_shape (or another add_..._shape) first");
         }
@@ -462,7 +451,6 @@ struct sdot_ctx {
         a.nodes = tree2.nodes;
         a.max_nodes = tree2.max_nodes;
         a.guard = guard;
-        a.item_nv = item_nv;
         a.start_n = start_n;
         a.start_xy = d_start;
         a.coeff = coeff;
@@ -473,11 +461,6 @@ struct sdot_ctx {
         a.img_nx = int(img_size[0]);
         a.img_ny = int(img_size[1]);
         a.img = d_img;
-        a.nitems = int(items.size());
-        a.item_off = d_item_off;
-        a.item_xy = d_item_xy;
-        a.item_nrm = d_item_nrm;
-        a.item_coeff = d_item_coeff;
         a.ovf_list = ovf_list;
         a.ovf_cnt = ovf_cnt;
         a.ovf_list2 = ovf_list2;
@@ -765,7 +748,7 @@ struct sdot_ctx {
             return SDOT_ITER_CAP;
         }
         if (e & DE_CAPACITY) {
-            last_error = dim == 3 ? "a cell exceeded the maximum polyhedron capacity (256 faces of 128 vertices)"
+            last_error = dim == 3 ? "a cell exceeded the maximum polyhedron capacity (640 vertices, 256 faces)"
                                   : "a cell exceeded the maximum polygon capacity (1024 vertices)";
             return SDOT_CAPACITY;
         }

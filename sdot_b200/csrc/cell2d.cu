@@ -4,8 +4,9 @@
 // a warp works on 32 neighbouring cells and walks nearly the same tree nodes.
 // The fast tier keeps the cell polygon in shared memory (one column per thread,
 // coordinates relative to the Dirac, the order of the vertices in a register);
-// cells that outgrow it are rebuilt by the warp tier, whose polygons live in
-// global scratch.  The traversal stack lives in local memory.
+// cells that outgrow it, and all those of a small diagram, are built by the warp
+// tier, a warp per cell, with polygons in shared memory or, past 64 vertices, in
+// global scratch.  The fast tier's traversal stack lives in local memory.
 //
 // Reference behaviour restated here:
 //  * traversal, eviction test and bisector cuts: SpZGrid::for_each_laguerre_cell
@@ -1057,7 +1058,7 @@ __device__ int build_cell_warp(const Cell2DArgs &A, long long s, const PolyView<
                         const int l = __ffs(int(cm)) - 1;
                         n = plane_cut_warp(cell, n, cap, __shfl_sync(FULL, ox, l), __shfl_sync(FULL, oy, l),
                                            __shfl_sync(FULL, nx, l), __shfl_sync(FULL, ny, l),
-                                           PER ? j0 + l + (sym + 1) * int(A.n) : j0 + l, false);
+                                           PER ? j0 + l + (sym + 1) * int(A.n) : j0 + l);
                         if (n <= 0) return n;
                     }
                 }

@@ -103,13 +103,6 @@ struct Cell2DArgs {
     double img_lo[2] = {0, 0}, img_hi[2] = {1, 1};
     int img_nx = 0, img_ny = 0;
     const double *img = nullptr;
-    // multi items: item k has vertices [item_off[k], item_off[k+1]) in item_xy
-    // (2 per vertex) with outward unit normals item_nrm, density item_coeff[k]
-    int nitems = 0;
-    const int *item_off = nullptr;
-    const double *item_xy = nullptr;
-    const double *item_nrm = nullptr;
-    const double *item_coeff = nullptr;
     // outputs (sorted order); null pointers skip that output
     double *mass = nullptr;       // get_integrals
     double *mass_c = nullptr;     // mass as get_centroids computes it
@@ -137,7 +130,6 @@ struct Cell2DArgs {
     const double *trans = nullptr;
     unsigned *err = nullptr;
     int *guard = nullptr;          // first failed guard: (code, sorted index, value)
-    long long item_nv = 0;         // number of item vertices (multi items)
 };
 
 size_t cells2d_scratch_bytes();

@@ -73,9 +73,9 @@ __host__ __device__ inline void check_fail(int code, int line, long long value) 
 
 inline int ceil_div(long long a, long long b) { return int((a + b - 1) / b); }
 
-// Per-device state of a kernel launcher (shared-memory attributes, tuned block
-// sizes): one slot per device ordinal, read and written under one mutex, so
-// that contexts on several devices, or several threads, can launch at once.
+// Per-device state of a kernel launcher (function attributes): one slot per
+// device ordinal under one mutex, so that contexts on several devices, or several
+// threads, can launch at once.
 constexpr int kDeviceSlots = 64;
 template <class T>
 struct PerDevice {
@@ -87,16 +87,6 @@ struct PerDevice {
         SDOT_CUDA(cudaGetDevice(&d));
         if (d < 0 || d >= kDeviceSlots) throw CudaError{cudaErrorInvalidDevice, "device ordinal beyond 64"};
         return d;
-    }
-    T get() {
-        const int d = device();
-        std::lock_guard<std::mutex> g(m);
-        return slot[d];
-    }
-    void set(const T &v) {
-        const int d = device();
-        std::lock_guard<std::mutex> g(m);
-        slot[d] = v;
     }
     // runs f() unless this device's slot is already set, then sets it (f runs
     // under the lock: concurrent first calls on one device wait for it)
@@ -180,7 +170,6 @@ enum DevErr : unsigned {
     DE_CAPACITY = 1u,      // cell polygon overflowed its capacity (re-run in the large path)
     DE_STACK = 2u,         // traversal stack overflow (should not happen: depth bounded)
     DE_ITER = 4u,          // an iteration cap was reached
-    DE_PIECE = 8u,         // a piece overflowed its capacity
     DE_GUARD = 16u,        // an input failed a consistency guard (see the debug triple)
     DE_DEGEN = 32u,        // a 3D cut met degenerate geometry (a face cut twice, an open new face)
     DE_SIDE = 64u,         // a long row did not fit the side buffer (the host grows it and runs again)

@@ -47,16 +47,15 @@ struct PolyView {
 // divides its distances by |nrm| for un-normalised normals (N<0>); the
 // interpolation ratios are the same without it.
 // Returns the new vertex count, or -1 if the result would exceed `cap`.
-// The facts the reference reads from its `outside` bitset: count, first set
-// bit, first clear bit, bits 1 and n - 1 (one pass over the vertices).
+// The facts read from the vertices' sides: how many are outside, the first one
+// outside, the first one inside, and the last one's side.
 struct CutFacts {
     int nb_out = 0, first_out = -1, first_in = -1;
-    bool out1 = false, out_last = false;
+    bool out_last = false;
     SDOT_HD void add(int k, int n, bool o) {
         nb_out += o;
         if (o && first_out < 0) first_out = k;
         if (!o && first_in < 0) first_in = k;
-        if (k == 1) out1 = o;
         if (k == n - 1) out_last = o;
     }
 };
@@ -86,7 +85,6 @@ SDOT_HD CutFacts cut_facts(unsigned mask, int n) {
     f.nb_out = popcount(mask);
     f.first_out = first_bit(mask);
     f.first_in = first_bit(in);
-    f.out1 = n > 1 && ((mask >> 1) & 1u);
     f.out_last = (mask >> (n - 1)) & 1u;
     return f;
 }
@@ -132,9 +130,9 @@ SDOT_HD int plane_cut(const PolyView<T> &p, int n, int cap, T ox, T oy, T nx, T 
 // The cut itself, given the classification of the vertices.  The new
 // vertices sit at the ratios s_a / (s_b - s_a) of the signed distances along
 // their edges; the ratios do not depend on the scale of the normal, so the
-// distances are left unnormalised, and in FP64 both ratios come from one
-// division (1 / (u v), u and v the two distance differences: products of
-// coordinates, far from underflow).
+// distances are left unnormalised, and both ratios come from one division
+// (1 / (u v), u and v the two distance differences: products of coordinates, far
+// from underflow).
 template <class T>
 SDOT_HD int plane_cut_apply(const PolyView<T> &p, int n, int cap, T ox, T oy, T nx, T ny, int cut_id,
                             const CutFacts &f) {
@@ -145,15 +143,9 @@ SDOT_HD int plane_cut_apply(const PolyView<T> &p, int n, int cap, T ox, T oy, T 
     auto dist = [&](int k) -> T { return (ox - p.X(k)) * nx + (oy - p.Y(k)) * ny; };
     // the two edge ratios a / (b - a), c / (d - c)
     auto ratios = [](T a, T b, T c, T d, T &m1, T &m2) {
-        const T u = b - a, v = d - c;
-        if constexpr (sizeof(T) == 8) {
-            const T r = T(1) / (u * v);
-            m1 = a * v * r;
-            m2 = c * u * r;
-        } else {  // FP32: u v of small cells can underflow
-            m1 = a / u;
-            m2 = c / v;
-        }
+        const T u = b - a, v = d - c, r = T(1) / (u * v);
+        m1 = a * v * r;
+        m2 = c * u * r;
     };
 
     // One layout for every case.  The removed run is [i1, i2] (cyclic), the
@@ -211,17 +203,16 @@ SDOT_HD int plane_cut_apply(const PolyView<T> &p, int n, int cap, T ox, T oy, T 
 // that keeps the scalar loop's result.  Same cases, same new vertices, same
 // vertex order as plane_cut.
 template <class T>
-__device__ int plane_cut_warp(const PolyView<T> &p, int n, int cap, T ox, T oy, T nx, T ny, int cut_id,
-                              bool normalize) {
+__device__ int plane_cut_warp(const PolyView<T> &p, int n, int cap, T ox, T oy, T nx, T ny, int cut_id) {
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     int nb_out = 0, first_out = -1, first_in = -1, runs = 0;
     bool out1 = false, out_last = false;
-    auto side = [&](int k) -> T { return (ox - p.X(k)) * nx + (oy - p.Y(k)) * ny; };
+    auto dist = [&](int k) -> T { return (ox - p.X(k)) * nx + (oy - p.Y(k)) * ny; };
     for (int base = 0; base < n; base += 32) {
         const int k = base + lane;
         const bool valid = k < n;
-        const bool o = valid && side(k) < T(0);
+        const bool o = valid && dist(k) < T(0);
         const unsigned mo = __ballot_sync(FULL, o), mi = __ballot_sync(FULL, valid && !o);
         nb_out += __popc(mo);
         runs += __popc(mo & ~(mo << 1 | unsigned(out_last)));  // out_last: of the vertices before
@@ -236,7 +227,7 @@ __device__ int plane_cut_warp(const PolyView<T> &p, int n, int cap, T ox, T oy, 
     if (runs - (out_last && first_out == 0) > 1) {
         // (every lane alike; rare)
         int a, g;
-        farthest_run(n, side, a, g);
+        farthest_run(n, dist, a, g);
         nb_out = g;
         const bool wrap = a + g > n;
         first_out = wrap ? 0 : a;
@@ -244,9 +235,6 @@ __device__ int plane_cut_warp(const PolyView<T> &p, int n, int cap, T ox, T oy, 
         out1 = wrap ? a + g - n > 1 || a == 1 : a <= 1 && a + g > 1;
         out_last = a + g >= n;
     }
-    T inv = T(1);
-    if (normalize) inv = T(1) / sqrt(nx * nx + ny * ny);
-    auto dist = [&](int k) -> T { return ((ox - p.X(k)) * nx + (oy - p.Y(k)) * ny) * inv; };
     int i1 = first_out;
     if (nb_out == 1) {
         if (n + 1 > cap) return -1;
