@@ -138,7 +138,9 @@ int sdot_get_der_integrals_wrt_weights(sdot_ctx *ctx, int64_t *offsets, int64_t 
                                        double *masses, int64_t *nnz_inout, int stop_if_void, int mem_space);
 /* Cut ids of each final cell boundary, in vertex order (the CP2 cut_ids the
  * traversal hands to its callback, SpZGrid.tcc:643): Dirac index, -1 for a
- * domain edge, -2 for a disc arc.  Two-phase like the Hessian.               */
+ * domain edge, -2 for a disc arc.  Two-phase like the Hessian.  A status other
+ * than SDOT_OK is that of the walk that made the lists (SDOT_CAPACITY: a cell
+ * outgrew the kernels and has an empty list); they are still written.         */
 int sdot_get_neighbors(sdot_ctx *ctx, int64_t *offsets, int64_t *ids, int64_t *count_inout, int mem_space);
 
 /* get_der_centroids_and_integrals_wrt_weight_and_positions( m_offsets,
